@@ -1,0 +1,68 @@
+"""The half-pair kernel whose jobs are cut by cost on the device (boxes above
+the all-pairs kernel's largest size, 14,336): accelerations and sums against
+the CPU oracle at the sizes and shapes where the job table can go wrong.
+
+Tolerances as in test_gpu_parity.py: both sides sum the same FP64 pair terms
+in another order; the terms are within a few ulp of the oracle's (1e-15) and
+a force is a sum of up to n of them with cancellation, which 1e-12 of the
+2-norm covers (n = 16,385: sqrt(n) roundings of terms up to the norm, 3e-14).
+"""
+import numpy as np
+import pytest
+
+from oracle.oracle import Oracle
+from yukawamd_b200 import abi, configs
+
+from test_gpu_parity import check_accel, workload
+
+pytestmark = pytest.mark.gpu
+
+PRECS = pytest.mark.parametrize("prec", [abi.YK_PREC_FP64, abi.YK_PREC_MIXED], ids=["fp64", "mixed"])
+
+
+@pytest.fixture(scope="module")
+def orc():
+    return Oracle("double", threads=8)
+
+
+@PRECS
+@pytest.mark.parametrize("kind", ["pure", "mix", "nn"])
+@pytest.mark.parametrize("n", [14336, 14337, 16385])
+def test_sizes_around_the_kernel_change(gpu, orc, kind, n, prec):
+    """The largest all-pairs box, the smallest cost-cut one (its last tile
+    holds one particle) and one more tile."""
+    w = workload(kind, n, 500 + n)
+    check_accel(orc, w, prec, True)
+    check_accel(orc, w, prec, False)
+
+
+def _clustered(kind, n, seed):
+    """Half the particles in one corner of the box, the rest spread out: rows
+    with everything and rows with nothing within reach."""
+    w = workload(kind, n, seed)
+    rng = np.random.default_rng(seed)
+    L = np.array(w.params["xl"])
+    x = rng.random((n, 3))
+    x[: n // 2] *= 0.15
+    w.x = np.ascontiguousarray((x * L).reshape(-1))
+    w.params["rccut"] = 0.1 * L[0] if kind != "nn" else w.params["rccut"]
+    return w
+
+
+@PRECS
+@pytest.mark.parametrize("sort", ["sorted", "unsorted"])
+def test_uneven_work(gpu, orc, sort, prec):
+    w = _clustered("mix", 15000, 3)
+    check_accel(orc, w, prec, True, tuning=dict(sort_every=4 if sort == "sorted" else -1))
+
+
+@pytest.mark.parametrize("n", [700, 14500])
+@pytest.mark.parametrize("rccut", [1.0e50, 1.0e200], ids=["1e50", "1e200"])
+def test_no_cutoff(gpu, orc, n, rccut):
+    """No cutoff (rccut at its 1e50 default, and one whose square overflows):
+    every pair counts, no image can be shared by a tile, and list pads and
+    empty target slots must still add nothing.  FP64 (the mixed form's FP32
+    energies of an uncut plasma are not held to 1e-6)."""
+    w = configs.pure_ion_ocp(11, n)
+    w.params["rccut"] = rccut
+    check_accel(orc, w, abi.YK_PREC_FP64, True)

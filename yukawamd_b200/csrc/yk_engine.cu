@@ -15,6 +15,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <limits>
 #include <mutex>
 #include <queue>
 #include <string>
@@ -27,6 +28,7 @@
 #include "yk_internal.h"
 #include "yk_pairs.cuh"
 #include "yk_pairs2.cuh"
+#include "yk_octets.cuh"
 #include "yk_gofr.cuh"
 #include "yk_near.cuh"
 #include "yk_sort.cuh"
@@ -171,6 +173,17 @@ struct yk_ctx {
     int* row_slots = nullptr;
     int* job_counter = nullptr;
     PairJobs pj{};
+    // octet kernel (yk_octets.cuh)
+    bool oct = false;                   // the half-pair kernel of this box is k_force_octets
+    bool oct_jobs_due = true;           // the slot order changed: cut the jobs anew
+    int sms = 0;
+    int oct_target = 0;                 // jobs aimed at (k_octet_rows)
+    double2* posq = nullptr;            // positions by tile: 128 (x, y), 128 (z, w)
+    float4* obox = nullptr;             // octet boxes
+    unsigned char* oct_cost = nullptr;  // per unit: the cost of its windows
+    int *row_cost = nullptr, *row_start = nullptr;
+    double* rsum = nullptr;             // per row: measuring sums
+    int oct_chunks = 0, oct_len = 0;    // k_force_octets_all: source chunks and their length (0: k_force_octets)
     // argument blocks and tunables
     ForceArgs fa{};
     StepArgs sa{};
@@ -250,7 +263,7 @@ static void setup_args(yk_ctx* c)
         const double hl = 0.5 * p.xl[k];
         std::memcpy(&f.hlb[k], &hl, sizeof hl);
     }
-    f.rc2 = p.rccut * p.rccut;
+    f.rc2 = std::min(p.rccut * p.rccut, std::numeric_limits<double>::max());
     f.rn2 = p.rncut * p.rncut;
     f.xmuc = p.xmuc;
     f.vc = p.vc;
@@ -544,7 +557,70 @@ static void free_pairs(yk_ctx* c)
     c->tbox = nullptr;
     cudaFree(c->Sjf);
     c->Sjf = nullptr;
+    cudaFree(c->posq);
+    cudaFree(c->obox);
+    cudaFree(c->oct_cost);
+    cudaFree(c->row_cost);
+    cudaFree(c->row_start);
+    cudaFree(c->rsum);
+    c->posq = nullptr;
+    c->obox = nullptr;
+    c->oct_cost = nullptr;
+    c->row_cost = c->row_start = nullptr;
+    c->rsum = nullptr;
+    c->oct = false;
     c->pj = PairJobs{};
+}
+
+// Whether the half-pair kernel of the context is k_force_octets: FP64 ions
+// with one target per thread (its lanes are 8 targets by 4 sources whatever
+// pair_seg and source_split say: the jobs are cut by cost).
+static bool octets_apply(const yk_ctx* c)
+{
+    return c->kernel_req != 3 && c->p.precision == YK_PREC_FP64 && pair_tt(c) == 1 &&
+           (c->p.sim_type == YK_SIM_PURE_ION || c->p.sim_type == YK_SIM_ION_MIXTURE);
+}
+
+// Scratch of the octet kernels.  Boxes of up to OCT_ALL_MAX_N particles take
+// every pair from both sides (k_force_octets_all): their half-pair units are
+// too few and too long to balance.  Measured (FP64 force call, B200): 500 ions
+// 67 us with k_force_pairs, 19 with k_force_octets_all and 44 with
+// k_force_octets; 2,000 ions 50 / 35 / 79; 4,096 ions 64 / 55 / 111; 12,345 ions
+// (r_c = 115 fm) 114 / 115 / 136; 16,384 ions 185 / 195 / 178; 55,296 ions
+// (r_c = 298 fm) 2,007 / 2,860 / 1,320; 131,072 ions (r_c = 149 fm) 2,215 / - /
+// 650.
+static int setup_octets(yk_ctx* c)
+{
+    const int M = (c->n + PB - 1) / PB;
+    const size_t units = (size_t)M * (M + 1) / 2;
+    c->pj.M = M;
+    c->pj_tt = 1;
+    c->oct = true;
+    CK(c, cudaMalloc((void**)&c->rsum, sizeof(double) * (size_t)M * NSCAL));
+    CK(c, cudaMalloc((void**)&c->tbox, 2 * sizeof(float4) * (size_t)M));
+    CK(c, cudaMalloc((void**)&c->obox, 2 * sizeof(float4) * (size_t)M * OCTETS));
+    CK(c, cudaMalloc((void**)&c->posq, 2 * sizeof(double2) * (size_t)M * PB));
+    c->oct_chunks = 0;
+    if (c->n <= OCT_ALL_MAX_N) {
+        c->oct_len = octet_all_len(c->n);
+        c->oct_chunks = (c->n + c->oct_len - 1) / c->oct_len;
+        const size_t jobs = (size_t)M * (PB / 32) * c->oct_chunks;
+        CK(c, cudaMalloc((void**)&c->Si, sizeof(double) * (size_t)c->oct_chunks * M * PB * 3));
+        CK(c, cudaMalloc((void**)&c->Sm, sizeof(double) * jobs * NSCAL));
+        return YK_OK;
+    }
+    c->oct_target = OCT_JOBS * OCT_WARPS * c->sms;
+    const size_t jobs = (size_t)octet_jobs_cap(M, c->oct_target);
+    CK(c, cudaMalloc(&c->Sj, sizeof(double) * units * PB * 3));
+    CK(c, cudaMalloc((void**)&c->Si, sizeof(double) * jobs * PB * 3));
+    CK(c, cudaMalloc((void**)&c->Sm, sizeof(double) * jobs * NSCAL));
+    CK(c, cudaMalloc((void**)&c->jobs, sizeof(int4) * jobs));
+    CK(c, cudaMalloc((void**)&c->row_start, sizeof(int) * ((size_t)M + 1)));
+    CK(c, cudaMalloc((void**)&c->row_cost, sizeof(int) * OCT_COST_CTAS * (size_t)M));
+    CK(c, cudaMalloc((void**)&c->oct_cost, OCT_WPT * units));
+    CK(c, cudaMalloc((void**)&c->Sjf, units));
+    c->oct_jobs_due = true;
+    return YK_OK;
 }
 
 // Build the job table of the half-pair kernel (build_pair_jobs) and its
@@ -554,6 +630,7 @@ static int setup_pairs(yk_ctx* c)
     free_pairs(c);
     const int M = (c->n + PB - 1) / PB;
     if (c->seg_auto) c->seg = auto_pair_seg(c);
+    if (octets_apply(c)) return setup_octets(c);
     std::vector<int4> jobs;
     std::vector<int> slots;
     // the near-list kernel reads whole tiles: no split for it
@@ -582,14 +659,43 @@ static int setup_pairs(yk_ctx* c)
     return YK_OK;
 }
 
+// Bytes of the scratch that the half-pair kernel of the context takes.
+static size_t half_pair_bytes(const yk_ctx* c)
+{
+    if (!octets_apply(c)) return pair_scratch_bytes(c->n, c->seg, c->dev, c->p.precision);
+    const size_t M = (size_t)(c->n + PB - 1) / PB, row = sizeof(double) * PB * 3;
+    const size_t boxes = M * (2 * sizeof(double2) * PB + 2 * sizeof(float4) * (OCTETS + 1) + sizeof(double) * NSCAL);
+    if (c->n <= OCT_ALL_MAX_N) {
+        const size_t chunks = ((size_t)c->n + octet_all_len(c->n) - 1) / octet_all_len(c->n);
+        return boxes + chunks * M * (row + sizeof(double) * NSCAL * (PB / 32));
+    }
+    const size_t units = M * (M + 1) / 2;
+    const size_t jobs = (size_t)octet_jobs_cap((int)M, OCT_JOBS * OCT_WARPS * c->sms);
+    return boxes + units * (row + OCT_WPT + 1) + jobs * (row + sizeof(double) * NSCAL + sizeof(int4)) +
+           sizeof(int) * M * (OCT_COST_CTAS + 1);
+}
+
+// setup_pairs; if its scratch cannot be had, the context falls back to the row
+// kernel, which needs none, and stays usable.
+static int setup_or_rows(yk_ctx* c)
+{
+    const int rc = setup_pairs(c);
+    if (rc) {
+        cudaGetLastError();
+        free_pairs(c);
+        c->kernel = 1;
+    }
+    return rc;
+}
+
 // A new box can change whether k_force_pairs2 applies (fa.img_k, fa.lo):
 // rebuild the job table when it does.
 static int refresh_pair_tt(yk_ctx* c)
 {
-    if (c->kernel == 2 && pair_tt(c) != c->pj_tt) {
+    if (c->kernel == 2 && (pair_tt(c) != c->pj_tt || octets_apply(c) != c->oct)) {
         CK(c, cudaSetDevice(c->dev));
         CK(c, cudaStreamSynchronize(c->stream));
-        return setup_pairs(c);
+        return setup_or_rows(c);
     }
     return YK_OK;
 }
@@ -602,9 +708,9 @@ static int resolve_kernel(yk_ctx* c)
     // autotuner candidate: with nucleons in species-major slot order it is
     // 1.35x slower than kernel 2 on the 51,200-nucleon box, and on the
     // 55,296-ion mixture 1.5x slower.)
-    if (k == 0) k = (pair_scratch_bytes(c->n, c->seg, c->dev, c->p.precision) <= PAIR_SCRATCH_BUDGET) ? 2 : 1;
+    if (k == 0) k = half_pair_bytes(c) <= PAIR_SCRATCH_BUDGET ? 2 : 1;
     if (k == 2 || k == 3) {
-        int rc = setup_pairs(c);
+        int rc = setup_or_rows(c);
         if (rc) return rc;
     } else {
         free_pairs(c);
@@ -646,6 +752,7 @@ static int enqueue_order(yk_ctx* c, bool sort)
         }
         ++k;
         c->need_sort = false;
+        c->oct_jobs_due = true;
     }
     k_apply_perm<<<nb, VBLOCK, 0, st>>>(c->perm, c->iperm, c->x, c->zii, c->pos, c->posf, n,
                                         c->sa.pack_w);
@@ -683,9 +790,55 @@ static int persistent_grid(int dev)
     return g;
 }
 
+// The octet kernel's force call: slot-ordered tiles and boxes, the job table
+// when the slot order is new, the kernel and its combine.
+template <int SIM, bool MEAS>
+static int launch_octets(yk_ctx* c)
+{
+    cudaStream_t st = c->stream;
+    const int M = c->pj.M;
+    float4* tbox = reinterpret_cast<float4*>(c->tbox);
+    k_octet_pack<<<M, PB, 0, st>>>(c->pos, c->n, c->fa, c->posq, c->obox, tbox);
+    int k = 3;
+    if (c->oct_chunks) {
+        const OctetBox bx{c->posq, c->obox, tbox, nullptr, nullptr, nullptr, c->Sm, nullptr, nullptr, c->n, M};
+        const int grid = M * (PB / 32) * c->oct_chunks;
+        if (c->fa.exp_ok)
+            k_force_octets_all<SIM, MEAS, false><<<grid, 32, 0, st>>>(bx, c->oct_chunks, c->oct_len, c->Si, c->fa,
+                                                                      c->err);
+        else
+            k_force_octets_all<SIM, MEAS, true><<<grid, 32, 0, st>>>(bx, c->oct_chunks, c->oct_len, c->Si, c->fa,
+                                                                     c->err);
+        k_octet_all_combine<SIM, MEAS><<<M, COMB_THREADS, 0, st>>>(c->Si, c->Sm, c->oct_chunks, M, c->perm, c->zii,
+                                                                   c->aii, c->fa, c->a, c->rsum);
+        return k;
+    }
+    cudaMemsetAsync(c->job_counter, 0, sizeof(int), st);
+    if (c->oct_jobs_due) {
+        k_octet_cost<<<dim3(M, OCT_COST_CTAS), 256, 0, st>>>(c->obox, tbox, M, c->fa, c->oct_cost, c->row_cost);
+        k_octet_rows<<<1, 1024, 0, st>>>(c->row_cost, M, c->oct_target, c->row_start);
+        k_octet_jobs<<<M, 1024, 0, st>>>(c->oct_cost, c->row_cost, M, c->row_start, c->jobs);
+        c->oct_jobs_due = false;
+        k += 3;
+    }
+    const OctetBox bx{c->posq, c->obox, tbox, c->Si, static_cast<double*>(c->Sj), c->Sjf, c->Sm, c->jobs,
+                      c->row_start, c->n, M};
+    const int grid = OCT_WARPS * c->sms;
+    if (c->fa.exp_ok) k_force_octets<SIM, MEAS, false><<<grid, 32, 0, st>>>(bx, c->job_counter, c->fa, c->err);
+    else k_force_octets<SIM, MEAS, true><<<grid, 32, 0, st>>>(bx, c->job_counter, c->fa, c->err);
+    const size_t smem = comb_smem_bytes(M);
+    if (smem > (size_t)40 << 10)
+        cudaFuncSetAttribute(k_octet_combine<SIM, MEAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_octet_combine<SIM, MEAS><<<M, COMB_THREADS, smem, st>>>(bx, c->perm, c->zii, c->aii, c->fa, c->a, c->rsum);
+    return k;
+}
+
 template <int SIM, int PREC, bool MEAS>
 static int launch_force_t(yk_ctx* c)
 {
+    if constexpr (SIM != SIM_NUCLEON && PREC == PREC_FP64) {
+        if (c->kernel == 2 && c->oct) return launch_octets<SIM, MEAS>(c);
+    }
     if (c->kernel == 1) {
         k_force_rows<SIM, PREC, MEAS><<<c->nfb, FBLOCK, FORCE_SMEM, c->stream>>>(
             c->pos, c->posf, c->perm, c->aii, c->fa, c->a, c->fpart, c->err);
@@ -730,13 +883,8 @@ static int launch_force_t(yk_ctx* c)
                 k_force_pairs<SIM, PREC, MEAS, true><<<std::min(grid, njobs), PB, 0, c->stream>>>(
                     c->pos, c->posf, pj, c->job_counter, c->fa, c->Si, Sj, c->Sm, c->err);
             }
-        } else if (SIM != SIM_NUCLEON && c->fa.img_k && c->fa.exp_ok) {
-            if constexpr (SIM != SIM_NUCLEON) {
-                const int grid = persistent_grid<k_force_pairs<SIM, PREC, MEAS, false, true>>(c->dev);
-                k_force_pairs<SIM, PREC, MEAS, false, true><<<std::min(grid, njobs), PB, 0, c->stream>>>(
-                    c->pos, c->posf, pj, c->job_counter, c->fa, c->Si, Sj, c->Sm, c->err);
-            }
-        } else {
+        } else if constexpr (SIM == SIM_NUCLEON || PREC == PREC_MIXED) {
+            // (FP64 ions take k_force_octets)
             const int grid = persistent_grid<k_force_pairs<SIM, PREC, MEAS>>(c->dev);
             k_force_pairs<SIM, PREC, MEAS><<<std::min(grid, njobs), PB, 0, c->stream>>>(
                 c->pos, c->posf, pj, c->job_counter, c->fa, c->Si, Sj, c->Sm, c->err);
@@ -791,15 +939,15 @@ static int enqueue_finish(yk_ctx* c, bool meas, int kin_mode, bool series)
     z.force_mode = has_force ? 1 : 0;
     z.do_meas = meas ? 1 : 0;
     if (c->kernel >= 2) {
-        z.nfp = (has_force && meas) ? c->pj.njobs : 0;
-        z.half = 1.0;                   // each unique pair counted once
+        z.nfp = (has_force && meas) ? (c->oct ? c->pj.M : c->pj.njobs) : 0;
+        z.half = (c->oct && c->oct_chunks) ? 0.5 : 1.0;   // each unique pair counted once, or from both sides
     } else {
         z.nfp = (has_force && meas) ? c->nfb : 0;
         z.half = 0.5;                   // each pair counted from both sides
     }
     z.kin_mode = kin_mode;
     z.nkp = (kin_mode == 2) ? c->nvb : 0;
-    k_finish<<<1, 256, 0, c->stream>>>(c->kernel >= 2 ? c->Sm : c->fpart, c->kpart, z, c->a, c->ds,
+    k_finish<<<1, 256, 0, c->stream>>>(c->kernel >= 2 ? (c->oct ? c->rsum : c->Sm) : c->fpart, c->kpart, z, c->a, c->ds,
                                        series ? c->series : nullptr, c->series_idx);
     return 1;
 }
@@ -1125,6 +1273,10 @@ int yk_create(const yk_params* p, int n, const double* x, const double* v, const
         delete c;
         return fail(nullptr, YK_ERR_CUDA, "cudaSetDevice(%d) failed", p->device);
     }
+    if (cudaDeviceGetAttribute(&c->sms, cudaDevAttrMultiProcessorCount, c->dev) != cudaSuccess || c->sms < 1) {
+        delete c;
+        return fail(nullptr, YK_ERR_CUDA, "cudaDeviceGetAttribute failed");
+    }
     setup_args(c);
     c->seg = auto_pair_seg(c);
 
@@ -1135,7 +1287,7 @@ int yk_create(const yk_params* p, int n, const double* x, const double* v, const
     size_t bytes = sizeof(double) * (3 * (size_t)n * 3 + 3 * (size_t)(n + 3) + 2 * (size_t)n) +
                    (sizeof(double4) + sizeof(float) * SHADOW_FLOATS / SHADOW_TILE) * ((size_t)n + SHADOW_TILE) + sizeof(int) * 5 * (size_t)n + cub_bytes +
                    sizeof(double) * (size_t)(8 * c->nfb + NKIN * c->nvb) + 4096;
-    const size_t pair_bytes = pair_scratch_bytes(n, c->seg, c->dev, p->precision);
+    const size_t pair_bytes = half_pair_bytes(c);
     const bool pairs_fit = pair_bytes <= PAIR_SCRATCH_BUDGET;
     if (pairs_fit) bytes += pair_bytes;
     size_t free_b = 0, total_b = 0;
@@ -1828,12 +1980,17 @@ __global__ void k_noalloc_prepare(int* perm, int n, int4* jobs, int* row_slots, 
 struct NoallocLayout {
     size_t pos, posf, perm, iperm, Si, Sj, Sm, jobs, row_slots, ds, counter, err, total;
     int M, nseg, njobs;
+    // octets (FP64 ions): k_force_octets_all in place of the job table
+    size_t posq, obox, tbox, rsum;
+    bool oct;
+    int chunks, len;
 };
 
-static NoallocLayout noalloc_layout(int n)
+static NoallocLayout noalloc_layout(int n, bool oct)
 {
     NoallocLayout L{};
     L.M = (n + PB - 1) / PB;
+    L.oct = oct;
     L.nseg = (L.M + NOALLOC_SEG - 1) / NOALLOC_SEG;
     L.njobs = 0;
     for (int R = 0; R < L.M; ++R) L.njobs += (L.M - R + NOALLOC_SEG - 1) / NOALLOC_SEG;
@@ -1847,6 +2004,27 @@ static NoallocLayout noalloc_layout(int n)
     L.posf = take(sizeof(float) * SHADOW_FLOATS * (size_t)L.M);
     L.perm = take(sizeof(int) * (size_t)n);
     L.iperm = take(sizeof(int) * (size_t)n);
+    if (oct) {
+        L.posq = take(2 * sizeof(double2) * PB * (size_t)L.M);
+        L.obox = take(2 * sizeof(float4) * OCTETS * (size_t)L.M);
+        L.tbox = take(2 * sizeof(float4) * (size_t)L.M);
+        L.rsum = take(sizeof(double) * NSCAL * (size_t)L.M);
+        L.ds = take(sizeof(DevScalars));
+        L.counter = take(sizeof(int));
+        L.err = take(sizeof(unsigned));
+        // the longest chunks' partial sums take what is left
+        for (L.len = octet_all_len(n);; L.len *= 2) {
+            L.chunks = (n + L.len - 1) / L.len;
+            const size_t part = sizeof(double) * 3 * PB * (size_t)L.M * L.chunks;
+            const size_t sm = sizeof(double) * NSCAL * (PB / 32) * (size_t)L.M * L.chunks;
+            if (off + part + sm + 512 > NOALLOC_BYTES && L.chunks > 1) continue;
+            L.Si = take(part);
+            L.Sm = take(sm);
+            break;
+        }
+        L.total = off;
+        return L;
+    }
     L.Si = take(sizeof(double) * 3 * PB * (size_t)L.M * L.nseg);
     L.Sj = take(sizeof(double) * 3 * PB * ((size_t)L.M * (L.M + 1) / 2));
     L.Sm = take(sizeof(double) * NSCAL * (size_t)L.njobs);
@@ -1857,6 +2035,26 @@ static NoallocLayout noalloc_layout(int n)
     L.err = take(sizeof(unsigned));
     L.total = off;
     return L;
+}
+
+// FP64 ions: k_force_octets_all (every pair from both sides).
+template <int SIM, bool MEAS>
+static void noalloc_octets(cudaStream_t st, const NoallocLayout& L, unsigned char* b, const double4* pos,
+                           const ForceArgs& fa, unsigned* err, const int* perm, const double* zii, const double* aii,
+                           double* a)
+{
+    double2* posq = reinterpret_cast<double2*>(b + L.posq);
+    float4* obox = reinterpret_cast<float4*>(b + L.obox);
+    float4* tbox = reinterpret_cast<float4*>(b + L.tbox);
+    double* part = reinterpret_cast<double*>(b + L.Si);
+    double* Sm = reinterpret_cast<double*>(b + L.Sm);
+    k_octet_pack<<<L.M, PB, 0, st>>>(pos, fa.n, fa, posq, obox, tbox);
+    const OctetBox bx{posq, obox, tbox, nullptr, nullptr, nullptr, Sm, nullptr, nullptr, fa.n, L.M};
+    const int grid = L.M * (PB / 32) * L.chunks;
+    if (fa.exp_ok) k_force_octets_all<SIM, MEAS, false><<<grid, 32, 0, st>>>(bx, L.chunks, L.len, part, fa, err);
+    else k_force_octets_all<SIM, MEAS, true><<<grid, 32, 0, st>>>(bx, L.chunks, L.len, part, fa, err);
+    k_octet_all_combine<SIM, MEAS><<<L.M, COMB_THREADS, 0, st>>>(part, Sm, L.chunks, L.M, perm, zii, aii, fa, a,
+                                                                reinterpret_cast<double*>(b + L.rsum));
 }
 
 template <int SIM, int PREC, bool MEAS>
@@ -1888,7 +2086,7 @@ static void noalloc_force_s(bool mixed, bool meas, int dev, cudaStream_t st, con
     if (mixed) {
         if (meas) noalloc_force<SIM, PREC_MIXED, true>(dev, st, pos, posf, pj, counter, fa, Si, Sj, Sm, err, perm, zii, aii, a);
         else noalloc_force<SIM, PREC_MIXED, false>(dev, st, pos, posf, pj, counter, fa, Si, Sj, Sm, err, perm, zii, aii, a);
-    } else {
+    } else if constexpr (SIM == SIM_NUCLEON) {
         if (meas) noalloc_force<SIM, PREC_FP64, true>(dev, st, pos, posf, pj, counter, fa, Si, Sj, Sm, err, perm, zii, aii, a);
         else noalloc_force<SIM, PREC_FP64, false>(dev, st, pos, posf, pj, counter, fa, Si, Sj, Sm, err, perm, zii, aii, a);
     }
@@ -1910,7 +2108,9 @@ extern "C" int yk_accel_noalloc(const yk_params* p, int n, const double* x_dev, 
         return fail(nullptr, YK_ERR_ARG, "this sim_type needs zii");
     if (p->sim_type == YK_SIM_ION_MIXTURE && !aii_dev)
         return fail(nullptr, YK_ERR_ARG, "ion-mixture runs need aii");
-    const NoallocLayout L = noalloc_layout(n);
+    const bool oct = p->precision == YK_PREC_FP64 &&
+                     (p->sim_type == YK_SIM_PURE_ION || p->sim_type == YK_SIM_ION_MIXTURE);
+    const NoallocLayout L = noalloc_layout(n, oct);
     if (L.total > NOALLOC_BYTES)
         return fail(nullptr, YK_ERR_ARG, "n = %d needs %zu scratch bytes, more than the %zu available", n,
                     L.total, NOALLOC_BYTES);
@@ -1959,7 +2159,7 @@ extern "C" int yk_accel_noalloc(const yk_params* p, int n, const double* x_dev, 
     CK(nullptr, cudaMemsetAsync(ds, 0, sizeof(DevScalars), st));
     CK(nullptr, cudaMemsetAsync(counter, 0, sizeof(int), st));
     CK(nullptr, cudaMemsetAsync(err, 0, sizeof(unsigned), st));
-    k_noalloc_prepare<<<(n + 255) / 256, 256, 0, st>>>(perm, n, jobs, row_slots, L.M, NOALLOC_SEG);
+    k_noalloc_prepare<<<(n + 255) / 256, 256, 0, st>>>(perm, n, jobs, row_slots, oct ? 0 : L.M, NOALLOC_SEG);
     k_apply_perm<<<(n + VBLOCK - 1) / VBLOCK, VBLOCK, 0, st>>>(perm, iperm, x_dev, zii_dev, pos, posf, n,
                                                               tmp.sa.pack_w);
     int k = 2;
@@ -1970,6 +2170,14 @@ extern "C" int yk_accel_noalloc(const yk_params* p, int n, const double* x_dev, 
     pj.row_slots = row_slots;
     pj.nseg_max = L.nseg;
     const bool mixed = p->precision == YK_PREC_MIXED;
+    if (oct) {
+        const bool pure = p->sim_type == YK_SIM_PURE_ION;
+        if (pure && meas) noalloc_octets<SIM_PURE, true>(st, L, b, pos, fa, err, perm, zii_dev, aii_dev, a_dev);
+        else if (pure) noalloc_octets<SIM_PURE, false>(st, L, b, pos, fa, err, perm, zii_dev, aii_dev, a_dev);
+        else if (meas) noalloc_octets<SIM_MIX, true>(st, L, b, pos, fa, err, perm, zii_dev, aii_dev, a_dev);
+        else noalloc_octets<SIM_MIX, false>(st, L, b, pos, fa, err, perm, zii_dev, aii_dev, a_dev);
+        k += 3;
+    } else
     switch (p->sim_type) {
     case YK_SIM_PURE_ION:
         noalloc_force_s<SIM_PURE>(mixed, meas, dev, st, pos, posf, pj, counter, fa, Si, Sj, Sm, err, perm, zii_dev,
@@ -1994,11 +2202,11 @@ extern "C" int yk_accel_noalloc(const yk_params* p, int n, const double* x_dev, 
     const bool has_force = p->sim_type != YK_SIM_BFIELD;
     z.force_mode = has_force ? 1 : 0;
     z.do_meas = meas ? 1 : 0;
-    z.nfp = (has_force && meas) ? L.njobs : 0;
-    z.half = 1.0;
+    z.nfp = (has_force && meas) ? (oct ? L.M : L.njobs) : 0;
+    z.half = oct ? 0.5 : 1.0;
     z.kin_mode = 0;
     z.nkp = 0;
-    k_finish<<<1, 256, 0, st>>>(Sm, nullptr, z, a_dev, ds, nullptr, nullptr);
+    k_finish<<<1, 256, 0, st>>>(oct ? reinterpret_cast<double*>(b + L.rsum) : Sm, nullptr, z, a_dev, ds, nullptr, nullptr);
     ++k;
     g_launches += k;
 
