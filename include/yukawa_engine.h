@@ -306,8 +306,10 @@ typedef struct yk_tuning {
     int pair_seg;         /* longest job of the half-pair kernels, in source
                              tiles (jobs shrink towards the end of the job
                              list); 0 = automatic (8 FP64, 4 mixed).  No
-                             effect on FP64 ion boxes with one target per
-                             thread, whose jobs are cut by cost on the device */
+                             effect on ion boxes that take the octet kernel
+                             (one target per thread; FP64, or mixed up to
+                             6,144 and from 24,576 particles), whose jobs are
+                             cut by cost on the device                      */
     int sort_every;       /* steps between Hilbert re-orderings (-1 = never,
                              0 = automatic: 4)                              */
     int graph_steps;      /* steps per CUDA graph of yk_run: the graphs take
@@ -319,8 +321,8 @@ typedef struct yk_tuning {
                              taking a contiguous 1/split of every source tile,
                              so split x more CTAs (threads per target) work on
                              a small box: 1, 2 or 4 (jobs of one tile then);
-                             0 = 1; ignored by kernels 1 and 3 and by FP64 ion
-                             boxes (as pair_seg).  Batches: 0/1              */
+                             0 = 1; ignored by kernels 1 and 3 and by the octet
+                             kernel (as pair_seg).  Batches: 0/1             */
     int targets_per_thread; /* targets each thread of the half-pair kernel
                              holds: 1, or 2 (blocks of 256 targets, every
                              source read and reaction reduction shared by two

@@ -1,11 +1,13 @@
-"""The half-pair kernel whose jobs are cut by cost on the device (boxes above
-the all-pairs kernel's largest size, 14,336): accelerations and sums against
-the CPU oracle at the sizes and shapes where the job table can go wrong.
+"""The octet kernels: accelerations and sums against the CPU oracle at the sizes
+where the engine changes kernel (FP64: every pair from both sides up to 9,216
+particles, half pairs in jobs cut by cost above; mixed: up to 6,144 and from
+24,576) and at the shapes where the job table can go wrong.
 
 Tolerances as in test_gpu_parity.py: both sides sum the same FP64 pair terms
 in another order; the terms are within a few ulp of the oracle's (1e-15) and
 a force is a sum of up to n of them with cancellation, which 1e-12 of the
-2-norm covers (n = 16,385: sqrt(n) roundings of terms up to the norm, 3e-14).
+2-norm covers (n = 24,577: sqrt(n) roundings of terms up to the norm, 4e-14).
+Mixed: 1e-6, the form's bound.
 """
 import numpy as np
 import pytest
@@ -25,12 +27,14 @@ def orc():
     return Oracle("double", threads=8)
 
 
-@PRECS
 @pytest.mark.parametrize("kind", ["pure", "mix", "nn"])
-@pytest.mark.parametrize("n", [14336, 14337, 16385])
+@pytest.mark.parametrize("n,prec", [(9216, abi.YK_PREC_FP64), (9217, abi.YK_PREC_FP64), (10369, abi.YK_PREC_FP64),
+                                    (6143, abi.YK_PREC_MIXED), (6145, abi.YK_PREC_MIXED),
+                                    (24575, abi.YK_PREC_MIXED), (24577, abi.YK_PREC_MIXED)])
 def test_sizes_around_the_kernel_change(gpu, orc, kind, n, prec):
     """The largest all-pairs box, the smallest cost-cut one (its last tile
-    holds one particle) and one more tile."""
+    holds one particle), one more tile; the mixed form's changes, with last
+    tiles that end on half a source pair."""
     w = workload(kind, n, 500 + n)
     check_accel(orc, w, prec, True)
     check_accel(orc, w, prec, False)
@@ -56,7 +60,7 @@ def test_uneven_work(gpu, orc, sort, prec):
     check_accel(orc, w, prec, True, tuning=dict(sort_every=4 if sort == "sorted" else -1))
 
 
-@pytest.mark.parametrize("n", [700, 14500])
+@pytest.mark.parametrize("n", [700, 9500])
 @pytest.mark.parametrize("rccut", [1.0e50, 1.0e200], ids=["1e50", "1e200"])
 def test_no_cutoff(gpu, orc, n, rccut):
     """No cutoff (rccut at its 1e50 default, and one whose square overflows):

@@ -29,6 +29,7 @@
 #include "yk_pairs.cuh"
 #include "yk_pairs2.cuh"
 #include "yk_octets.cuh"
+#include "yk_octets32.cuh"
 #include "yk_gofr.cuh"
 #include "yk_near.cuh"
 #include "yk_sort.cuh"
@@ -178,7 +179,7 @@ struct yk_ctx {
     bool oct_jobs_due = true;           // the slot order changed: cut the jobs anew
     int sms = 0;
     int oct_target = 0;                 // jobs aimed at (k_octet_rows)
-    double2* posq = nullptr;            // positions by tile: 128 (x, y), 128 (z, w)
+    float4* posq = nullptr;             // positions by tile, in the form's layout (Form64, Form32)
     float4* obox = nullptr;             // octet boxes
     unsigned char* oct_cost = nullptr;  // per unit: the cost of its windows
     int *row_cost = nullptr, *row_start = nullptr;
@@ -481,16 +482,17 @@ static void build_pair_jobs2(int M, int smax, int P, std::vector<int4>& jobs, st
 // Targets per thread of the half-pair kernel for the context as it stands:
 // 2 (k_force_pairs2) for ion boxes on the paths that kernel has (FP64 with
 // exact screen images, mixed with the hi/lo displacement) when requested,
-// else 1.  Automatic (0): 2 for mixed-form ion boxes of TPT2_AUTO_MIN_N
-// particles or more.  Measured on a B200 (force call, CUDA events): the
-// 55,296-ion mixture mixed 1.050 -> 1.004 ms with two targets (jobs of up
-// to 8 tiles), FP64 2.21 -> 2.46 ms (four CTAs per SM instead of five, and
-// the larger warp boxes evaluate more masked pairs); the 4,096-ion OCP mixed
-// 0.046 -> 0.048 ms (too few jobs); the 51,200-nucleon box mixed 1.15 ->
-// 1.40 ms (its one-target kernel runs 7 CTAs per SM, and 64-nucleon warp
-// boxes are large against the 11.5 fm nuclear cutoff), so nucleons take two
-// targets only when asked (the tuner tries it).
+// else 1.  Automatic (0): 2 for mixed-form ion boxes from TPT2_AUTO_MIN_N up to
+// the size where the octet kernel takes over (octets_apply).  Measured on a
+// B200 (force call, CUDA events): the 55,296-ion mixture mixed 1.050 -> 1.004
+// ms with two targets (jobs of up to 8 tiles), FP64 2.21 -> 2.46 ms (four CTAs
+// per SM instead of five, and the larger warp boxes evaluate more masked
+// pairs); the 4,096-ion OCP mixed 0.046 -> 0.048 ms (too few jobs); the
+// 51,200-nucleon box mixed 1.15 -> 1.40 ms (its one-target kernel runs 7 CTAs
+// per SM, and 64-nucleon warp boxes are large against the 11.5 fm nuclear
+// cutoff), so nucleons take two targets only when asked (the tuner tries it).
 constexpr int TPT2_AUTO_MIN_N = 16384;
+constexpr int OCT_MIXED_MIN_N = 24576;
 constexpr int DEFAULT_SEG_MIXED_TT2 = 8;
 
 static int pair_tt(const yk_ctx* c)
@@ -502,7 +504,8 @@ static int pair_tt(const yk_ctx* c)
         return (c->tpt_req == 2 && mixed && c->fa.hilo) ? 2 : 1;
     }
     if (c->p.sim_type != YK_SIM_PURE_ION && c->p.sim_type != YK_SIM_ION_MIXTURE) return 1;
-    const int want = c->tpt_req != 0 ? c->tpt_req : ((mixed && c->n >= TPT2_AUTO_MIN_N) ? 2 : 1);
+    const int want = c->tpt_req != 0 ? c->tpt_req
+                                     : ((mixed && c->n >= TPT2_AUTO_MIN_N && c->n < OCT_MIXED_MIN_N) ? 2 : 1);
     if (want != 2) return 1;
     return (mixed ? c->fa.lo : (c->fa.img_k && c->fa.exp_ok)) ? 2 : 1;
 }
@@ -572,23 +575,35 @@ static void free_pairs(yk_ctx* c)
     c->pj = PairJobs{};
 }
 
-// Whether the half-pair kernel of the context is k_force_octets: FP64 ions
-// with one target per thread (its lanes are 8 targets by 4 sources whatever
-// pair_seg and source_split say: the jobs are cut by cost).
+// Whether the half-pair kernel of the context is an octet kernel: ions with
+// one target per thread (the octet kernel's lanes are 8 targets by 4 sources
+// whatever pair_seg and source_split say: its jobs are cut by cost), FP64 at
+// every size and the mixed form, where it takes the hi/lo displacement, outside
+// the sizes in between that the tiles of k_force_pairs and k_force_pairs2
+// serve better.  Measured (step, B200; before / octets): FP64 5,000 ions (r_c =
+// 149 fm) 100 / 89 us, 10,000 155 / 145, 20,000 (298 fm) 753 / 589, 55,296
+// (298 fm) 2,054 / 1,390, 131,072 (149 fm) 2,268 / 700; mixed 5,000 75 / 67 us,
+// 10,000 (149 fm) 100 / 108, 16,384 (249 fm) 233 / 254, 28,000 (298 fm) 508 /
+// 487 and (75 fm) 141 / 121, 55,296 (298 fm) 920 / 800, 131,072 (149 fm) 950 /
+// 510.
 static bool octets_apply(const yk_ctx* c)
 {
-    return c->kernel_req != 3 && c->p.precision == YK_PREC_FP64 && pair_tt(c) == 1 &&
-           (c->p.sim_type == YK_SIM_PURE_ION || c->p.sim_type == YK_SIM_ION_MIXTURE);
+    if (c->kernel_req == 3 || pair_tt(c) != 1) return false;
+    if (c->p.sim_type != YK_SIM_PURE_ION && c->p.sim_type != YK_SIM_ION_MIXTURE) return false;
+    if (c->p.precision == YK_PREC_FP64) return true;
+    return c->fa.lo && (c->n <= OCT_ALL_MAX_N32 || c->n >= OCT_MIXED_MIN_N);
 }
 
-// Scratch of the octet kernels.  Boxes of up to OCT_ALL_MAX_N particles take
-// every pair from both sides (k_force_octets_all): their half-pair units are
-// too few and too long to balance.  Measured (FP64 force call, B200): 500 ions
-// 67 us with k_force_pairs, 19 with k_force_octets_all and 44 with
-// k_force_octets; 2,000 ions 50 / 35 / 79; 4,096 ions 64 / 55 / 111; 12,345 ions
-// (r_c = 115 fm) 114 / 115 / 136; 16,384 ions 185 / 195 / 178; 55,296 ions
-// (r_c = 298 fm) 2,007 / 2,860 / 1,320; 131,072 ions (r_c = 149 fm) 2,215 / - /
-// 650.
+// Whether that is k_force_octets_all, every pair from both sides: half-pair
+// units of a small box are too few and too long to balance (FP64 step, before
+// / all pairs / half pairs: 500 ions 95 / 46 / 64 us; 3,000 61 / 42 / 75; 5,000
+// 100 / 89 / 109; 8,000 134 / 121 / 142; 10,000 155 / 150 / 145).
+static bool octets_all(const yk_ctx* c)
+{
+    return c->n <= (c->p.precision == YK_PREC_FP64 ? OCT_ALL_MAX_N64 : OCT_ALL_MAX_N32);
+}
+
+// Scratch of the octet kernels.
 static int setup_octets(yk_ctx* c)
 {
     const int M = (c->n + PB - 1) / PB;
@@ -599,9 +614,9 @@ static int setup_octets(yk_ctx* c)
     CK(c, cudaMalloc((void**)&c->rsum, sizeof(double) * (size_t)M * NSCAL));
     CK(c, cudaMalloc((void**)&c->tbox, 2 * sizeof(float4) * (size_t)M));
     CK(c, cudaMalloc((void**)&c->obox, 2 * sizeof(float4) * (size_t)M * OCTETS));
-    CK(c, cudaMalloc((void**)&c->posq, 2 * sizeof(double2) * (size_t)M * PB));
+    CK(c, cudaMalloc((void**)&c->posq, sizeof(float4) * OCT_UNITS * (size_t)M));
     c->oct_chunks = 0;
-    if (c->n <= OCT_ALL_MAX_N) {
+    if (octets_all(c)) {
         c->oct_len = octet_all_len(c->n);
         c->oct_chunks = (c->n + c->oct_len - 1) / c->oct_len;
         const size_t jobs = (size_t)M * (PB / 32) * c->oct_chunks;
@@ -611,7 +626,7 @@ static int setup_octets(yk_ctx* c)
     }
     c->oct_target = OCT_JOBS * OCT_WARPS * c->sms;
     const size_t jobs = (size_t)octet_jobs_cap(M, c->oct_target);
-    CK(c, cudaMalloc(&c->Sj, sizeof(double) * units * PB * 3));
+    CK(c, cudaMalloc(&c->Sj, sj_elem_bytes(c->p.precision) * units * PB * 3));
     CK(c, cudaMalloc((void**)&c->Si, sizeof(double) * jobs * PB * 3));
     CK(c, cudaMalloc((void**)&c->Sm, sizeof(double) * jobs * NSCAL));
     CK(c, cudaMalloc((void**)&c->jobs, sizeof(int4) * jobs));
@@ -664,14 +679,14 @@ static size_t half_pair_bytes(const yk_ctx* c)
 {
     if (!octets_apply(c)) return pair_scratch_bytes(c->n, c->seg, c->dev, c->p.precision);
     const size_t M = (size_t)(c->n + PB - 1) / PB, row = sizeof(double) * PB * 3;
-    const size_t boxes = M * (2 * sizeof(double2) * PB + 2 * sizeof(float4) * (OCTETS + 1) + sizeof(double) * NSCAL);
-    if (c->n <= OCT_ALL_MAX_N) {
+    const size_t boxes = M * (sizeof(float4) * OCT_UNITS + 2 * sizeof(float4) * (OCTETS + 1) + sizeof(double) * NSCAL);
+    if (octets_all(c)) {
         const size_t chunks = ((size_t)c->n + octet_all_len(c->n) - 1) / octet_all_len(c->n);
         return boxes + chunks * M * (row + sizeof(double) * NSCAL * (PB / 32));
     }
     const size_t units = M * (M + 1) / 2;
     const size_t jobs = (size_t)octet_jobs_cap((int)M, OCT_JOBS * OCT_WARPS * c->sms);
-    return boxes + units * (row + OCT_WPT + 1) + jobs * (row + sizeof(double) * NSCAL + sizeof(int4)) +
+    return boxes + units * (sj_elem_bytes(c->p.precision) * PB * 3 + OCT_WPT + 1) + jobs * (row + sizeof(double) * NSCAL + sizeof(int4)) +
            sizeof(int) * M * (OCT_COST_CTAS + 1);
 }
 
@@ -792,23 +807,26 @@ static int persistent_grid(int dev)
 
 // The octet kernel's force call: slot-ordered tiles and boxes, the job table
 // when the slot order is new, the kernel and its combine.
-template <int SIM, bool MEAS>
+template <class F, int SIM, bool MEAS>
 static int launch_octets(yk_ctx* c)
 {
     cudaStream_t st = c->stream;
     const int M = c->pj.M;
     float4* tbox = reinterpret_cast<float4*>(c->tbox);
-    k_octet_pack<<<M, PB, 0, st>>>(c->pos, c->n, c->fa, c->posq, c->obox, tbox);
+    // exponents past 700 (FP64 only; the mixed form's hardware exponential
+    // flushes to 0)
+    const bool range = F::PREC == PREC_FP64 && !c->fa.exp_ok;
+    k_octet_pack<F><<<M, PB, 0, st>>>(c->pos, c->n, c->fa, c->posq, c->obox, tbox);
     int k = 3;
     if (c->oct_chunks) {
         const OctetBox bx{c->posq, c->obox, tbox, nullptr, nullptr, nullptr, c->Sm, nullptr, nullptr, c->n, M};
         const int grid = M * (PB / 32) * c->oct_chunks;
-        if (c->fa.exp_ok)
-            k_force_octets_all<SIM, MEAS, false><<<grid, 32, 0, st>>>(bx, c->oct_chunks, c->oct_len, c->Si, c->fa,
-                                                                      c->err);
+        if (range)
+            k_force_octets_all<F, SIM, MEAS, F::PREC == PREC_FP64><<<grid, 32, 0, st>>>(bx, c->oct_chunks, c->oct_len,
+                                                                                       c->Si, c->fa, c->err);
         else
-            k_force_octets_all<SIM, MEAS, true><<<grid, 32, 0, st>>>(bx, c->oct_chunks, c->oct_len, c->Si, c->fa,
-                                                                     c->err);
+            k_force_octets_all<F, SIM, MEAS, false><<<grid, 32, 0, st>>>(bx, c->oct_chunks, c->oct_len, c->Si, c->fa,
+                                                                         c->err);
         k_octet_all_combine<SIM, MEAS><<<M, COMB_THREADS, 0, st>>>(c->Si, c->Sm, c->oct_chunks, M, c->perm, c->zii,
                                                                    c->aii, c->fa, c->a, c->rsum);
         return k;
@@ -821,23 +839,25 @@ static int launch_octets(yk_ctx* c)
         c->oct_jobs_due = false;
         k += 3;
     }
-    const OctetBox bx{c->posq, c->obox, tbox, c->Si, static_cast<double*>(c->Sj), c->Sjf, c->Sm, c->jobs,
-                      c->row_start, c->n, M};
+    const OctetBox bx{c->posq, c->obox, tbox, c->Si, c->Sj, c->Sjf, c->Sm, c->jobs, c->row_start, c->n, M};
     const int grid = OCT_WARPS * c->sms;
-    if (c->fa.exp_ok) k_force_octets<SIM, MEAS, false><<<grid, 32, 0, st>>>(bx, c->job_counter, c->fa, c->err);
-    else k_force_octets<SIM, MEAS, true><<<grid, 32, 0, st>>>(bx, c->job_counter, c->fa, c->err);
+    if (range) k_force_octets<F, SIM, MEAS, F::PREC == PREC_FP64><<<grid, 32, 0, st>>>(bx, c->job_counter, c->fa, c->err);
+    else k_force_octets<F, SIM, MEAS, false><<<grid, 32, 0, st>>>(bx, c->job_counter, c->fa, c->err);
     const size_t smem = comb_smem_bytes(M);
     if (smem > (size_t)40 << 10)
-        cudaFuncSetAttribute(k_octet_combine<SIM, MEAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_octet_combine<SIM, MEAS><<<M, COMB_THREADS, smem, st>>>(bx, c->perm, c->zii, c->aii, c->fa, c->a, c->rsum);
+        cudaFuncSetAttribute(k_octet_combine<SIM, F::PREC, MEAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)smem);
+    k_octet_combine<SIM, F::PREC, MEAS><<<M, COMB_THREADS, smem, st>>>(bx, c->perm, c->zii, c->aii, c->fa, c->a,
+                                                                       c->rsum);
     return k;
 }
 
 template <int SIM, int PREC, bool MEAS>
 static int launch_force_t(yk_ctx* c)
 {
-    if constexpr (SIM != SIM_NUCLEON && PREC == PREC_FP64) {
-        if (c->kernel == 2 && c->oct) return launch_octets<SIM, MEAS>(c);
+    if constexpr (SIM != SIM_NUCLEON) {
+        using F = std::conditional_t<PREC == PREC_FP64, Form64, Form32>;
+        if (c->kernel == 2 && c->oct) return launch_octets<F, SIM, MEAS>(c);
     }
     if (c->kernel == 1) {
         k_force_rows<SIM, PREC, MEAS><<<c->nfb, FBLOCK, FORCE_SMEM, c->stream>>>(
@@ -2005,7 +2025,7 @@ static NoallocLayout noalloc_layout(int n, bool oct)
     L.perm = take(sizeof(int) * (size_t)n);
     L.iperm = take(sizeof(int) * (size_t)n);
     if (oct) {
-        L.posq = take(2 * sizeof(double2) * PB * (size_t)L.M);
+        L.posq = take(sizeof(float4) * OCT_UNITS * (size_t)L.M);
         L.obox = take(2 * sizeof(float4) * OCTETS * (size_t)L.M);
         L.tbox = take(2 * sizeof(float4) * (size_t)L.M);
         L.rsum = take(sizeof(double) * NSCAL * (size_t)L.M);
@@ -2043,16 +2063,16 @@ static void noalloc_octets(cudaStream_t st, const NoallocLayout& L, unsigned cha
                            const ForceArgs& fa, unsigned* err, const int* perm, const double* zii, const double* aii,
                            double* a)
 {
-    double2* posq = reinterpret_cast<double2*>(b + L.posq);
+    float4* posq = reinterpret_cast<float4*>(b + L.posq);
     float4* obox = reinterpret_cast<float4*>(b + L.obox);
     float4* tbox = reinterpret_cast<float4*>(b + L.tbox);
     double* part = reinterpret_cast<double*>(b + L.Si);
     double* Sm = reinterpret_cast<double*>(b + L.Sm);
-    k_octet_pack<<<L.M, PB, 0, st>>>(pos, fa.n, fa, posq, obox, tbox);
+    k_octet_pack<Form64><<<L.M, PB, 0, st>>>(pos, fa.n, fa, posq, obox, tbox);
     const OctetBox bx{posq, obox, tbox, nullptr, nullptr, nullptr, Sm, nullptr, nullptr, fa.n, L.M};
     const int grid = L.M * (PB / 32) * L.chunks;
-    if (fa.exp_ok) k_force_octets_all<SIM, MEAS, false><<<grid, 32, 0, st>>>(bx, L.chunks, L.len, part, fa, err);
-    else k_force_octets_all<SIM, MEAS, true><<<grid, 32, 0, st>>>(bx, L.chunks, L.len, part, fa, err);
+    if (fa.exp_ok) k_force_octets_all<Form64, SIM, MEAS, false><<<grid, 32, 0, st>>>(bx, L.chunks, L.len, part, fa, err);
+    else k_force_octets_all<Form64, SIM, MEAS, true><<<grid, 32, 0, st>>>(bx, L.chunks, L.len, part, fa, err);
     k_octet_all_combine<SIM, MEAS><<<L.M, COMB_THREADS, 0, st>>>(part, Sm, L.chunks, L.M, perm, zii, aii, fa, a,
                                                                 reinterpret_cast<double*>(b + L.rsum));
 }

@@ -32,8 +32,10 @@
 namespace yk {
 
 constexpr int OCTETS = PB / 8;            // octets of a target block
+constexpr int OCT_UNITS = 2 * PB;         // 16-byte units of a tile in global memory
 constexpr int OCT_PAD = PB;               // list index of the pad source
-constexpr int OCT_ZW = PB + 4;            // offset of a source's (z, w) from its (x, y) in shared memory
+constexpr int OCT_GAP = 4;                // 16-byte units between a tile's sections in shared memory (the pad's)
+constexpr int OCT_ZW = PB + OCT_GAP;      // FP64 form: offset of a source's (z, w) from its (x, y) in shared memory
 constexpr int OCT_WIN = 8;                // sources of a window, the unit that jobs are cut in
 constexpr int OCT_WPT = PB / OCT_WIN;     // windows per tile
 constexpr double OCT_FAR = 1e160;         // its coordinates: r^2 overflows, no cutoff reaches it
@@ -257,23 +259,13 @@ __device__ __forceinline__ void octet_batch(const ForceArgs& fa, const double4& 
     }
 }
 
-// Shared memory of one warp.  One tile stage: the warps of an SM hide each
-// other's copies (a reached tile is tens of batches), and the room of a second
-// stage lets a fourth warp live on each SM sub-partition.
-struct OctetSmem {
-    double2 tile[2 * OCT_ZW];             // source tile (TMA) and the pad source: x, y and z, w
-    double row[(PB + 1) * 3 + 1];         // reactions on the tile's sources (and the pad's)
-    double acc[PB * 3];                   // target sums of the job
-    float xs[3][PB];                      // the tile's coordinates in FP32, for the lists
-    float4 box[OCTETS][2];                // the block's octet boxes
-    alignas(16) unsigned char list[PB];   // the octet's source list
-    uint64_t bar;
-};
-
 // The octet's source list on a tile: lane l tests sources l, l + 32, ... against
 // the octet's box (centre oc, half-width oh).  UNI: oc already carries the one
 // image of the whole tile; otherwise each source takes its own minimum image,
-// and kcode receives the common image code of the listed sources, or -1.
+// and kcode receives the common image code of the listed sources, or -1.  (A
+// bounding sphere in place of the box saves 6 of the 13 instructions of a
+// test but lists about 5 % more sources: 55,296 ions FP64 1,314 -> 1,361 us,
+// mixed 720 -> 742 us.)
 template <bool UNI>
 __device__ __forceinline__ int octet_list(const ForceArgs& fa, const float (&oc)[3], const float (&oh)[3],
                                           const float (*__restrict__ xs)[PB], int jlim, int jmin,
@@ -303,7 +295,7 @@ __device__ __forceinline__ int octet_list(const ForceArgs& fa, const float (&oc)
             const float m = fmaxf(fabsf(v) - oh[c], 0.f);
             dist2 = fmaf(m, m, dist2);
         }
-        const bool near = j >= jmin && j < jlim && dist2 <= fa.scr_c2;
+        const bool near = (unsigned)(j - jmin) < (unsigned)(jlim - jmin) && dist2 <= fa.scr_c2;
         if constexpr (!UNI) {
             if (near) {
                 c_and &= code;
@@ -356,11 +348,11 @@ __device__ __forceinline__ void octet_eval(const ForceArgs& fa, double4 pt, int 
 // boxes of the octets and tiles (centre, -, half-width with the rounding
 // margin, -).  Written by k_octet_pack.
 struct OctetBox {
-    const double2* posq;
+    const float4* posq;                   // tiles of OCT_UNITS 16-byte units
     const float4* obox;
     const float4* tbox;
     double* Si;                           // per job: target sums of its block, [PB][3]
-    double* Sj;                           // per unit tri(C, R): reactions on tile C, [PB][3]
+    void* Sj;                             // per unit tri(C, R): reactions on tile C, [PB][3]
     unsigned char* Sjf;                   // per unit: 1 if its Sj row was written, 0 if it is zero
     double* Sm;                           // per job: NSCAL measuring sums
     const int4* jobs;                     // (R, s0, s1, -), row by row
@@ -369,8 +361,9 @@ struct OctetBox {
 };
 
 // One CTA of PB threads per tile.
+template <class F>
 static __global__ void __launch_bounds__(PB)
-k_octet_pack(const double4* __restrict__ pos, int n, ForceArgs fa, double2* __restrict__ posq,
+k_octet_pack(const double4* __restrict__ pos, int n, ForceArgs fa, float4* __restrict__ posq,
              float4* __restrict__ obox, float4* __restrict__ tbox)
 {
     __shared__ float red[PWARPS][6];
@@ -378,8 +371,7 @@ k_octet_pack(const double4* __restrict__ pos, int n, ForceArgs fa, double2* __re
     const int i = C * PB + j;
     const bool on = i < n;
     const double4 p = on ? pos[i] : make_double4(OCT_FAR, OCT_FAR, OCT_FAR, 0.0);
-    posq[2 * (size_t)C * PB + j] = make_double2(p.x, p.y);
-    posq[2 * (size_t)C * PB + PB + j] = make_double2(p.z, p.w);
+    F::pack(posq + (size_t)C * OCT_UNITS, j, p, on);
     const float inf = __int_as_float(0x7f800000);
     const float v[3] = {__double2float_rn(p.x), __double2float_rn(p.y), __double2float_rn(p.z)};
     float lo[3], hi[3], cc[3], hh[3], mu[3];
@@ -474,32 +466,6 @@ __device__ __forceinline__ bool octet_reach(const ForceArgs& fa, const float4& o
     return dist2 <= fa.scr_c2;
 }
 
-// The octet's list on a tile (octet_list) in the image that octet_reach found,
-// if it did; timg: every listed source has image kcode in every pair that
-// counts.
-__device__ __forceinline__ int octet_list_any(const ForceArgs& fa, bool uni, const float4 (&box)[2],
-                                              const float (*__restrict__ xs)[PB], int jlim, int jmin,
-                                              unsigned char* __restrict__ list, int& kcode, bool& timg)
-{
-    float oc[3] = {box[0].x, box[0].y, box[0].z};
-    const float oh[3] = {box[1].x, box[1].y, box[1].z};
-    timg = uni;
-    if (uni) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) oc[c] = fmaf(img_of(kcode, c), fa.Lf[c], oc[c]);
-        return octet_list<true>(fa, oc, oh, xs, jlim, jmin, list, kcode);
-    }
-    const int cnt = octet_list<false>(fa, oc, oh, xs, jlim, jmin, list, kcode);
-    // the listed sources' one image, where no pair inside r_c has another
-    timg = kcode >= 0;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        const float e = 0.5f * fa.Lf[c] - oh[c] - 1.0f;
-        timg = timg && e > 0.f && e * e > fa.scr_c2;
-    }
-    return cnt;
-}
-
 // FP32 copies of the tile's coordinates (its unfilled slots are never listed).
 __device__ __forceinline__ void octet_tile_f32(const double2* __restrict__ tl, float (*__restrict__ xs)[PB], int jmin,
                                                int jlim)
@@ -516,18 +482,171 @@ __device__ __forceinline__ void octet_tile_f32(const double2* __restrict__ tl, f
     __syncwarp();
 }
 
+// The FP64 form: what the job loops below need of it.  The tile is two sections
+// of 128 units, (x, y) and (z, w).
+struct Form64 {
+    static constexpr int PREC = PREC_FP64, SECTIONS = 2, SEC = PB, ROW = (PB + 1) * 3 + 1;
+    struct Extra {
+        float xs[3][PB];                  // the tile's coordinates in FP32, for the lists
+    };
+    using Target = double4;
+
+    static __device__ __forceinline__ void pack(float4* __restrict__ tile, int j, const double4& p, bool)
+    {
+        double2* t = reinterpret_cast<double2*>(tile);
+        t[j] = make_double2(p.x, p.y);
+        t[PB + j] = make_double2(p.z, p.w);
+    }
+
+    static __device__ __forceinline__ void pad(float4* __restrict__ tile)
+    {
+        double2* t = reinterpret_cast<double2*>(tile);
+        t[OCT_PAD] = make_double2(OCT_FAR, OCT_FAR);
+        t[OCT_ZW + OCT_PAD] = make_double2(OCT_FAR, 0.0);
+    }
+
+    static __device__ __forceinline__ void tile_ready(const float4* __restrict__ tile, Extra& x, int jmin, int jlim)
+    {
+        octet_tile_f32(reinterpret_cast<const double2*>(tile), x.xs, jmin, jlim);
+    }
+
+    static __device__ __forceinline__ Target target(const float4* __restrict__ posq, int R, int s, bool on)
+    {
+        const double2* t = reinterpret_cast<const double2*>(posq) + 2 * (size_t)R * PB + s;
+        const double2 xy = t[0], zw = t[PB];
+        return make_double4(on ? xy.x : -OCT_FAR, xy.y, zw.x, zw.y);      // no target: no pair
+    }
+
+    static __device__ __forceinline__ double weight(const Target& t) { return t.w; }
+
+    template <bool UNI>
+    static __device__ __forceinline__ int list(const ForceArgs& fa, const float (&oc)[3], const float (&oh)[3],
+                                               const float4* __restrict__, const Extra& x, int jlim, int jmin,
+                                               unsigned char* __restrict__ l, int& kcode)
+    {
+        return octet_list<UNI>(fa, oc, oh, x.xs, jlim, jmin, l, kcode);
+    }
+
+    template <int SIM, bool MEAS, bool RANGE, bool TIMG, bool REACT>
+    static __device__ __forceinline__ void eval(const ForceArgs& fa, const Target& t, int lim, int kcode, int cnt,
+                                                const float4* __restrict__ tile, const unsigned char* __restrict__ l,
+                                                double tab, OctetSum<MEAS>& sum, double* __restrict__ row)
+    {
+        octet_eval<SIM, MEAS, RANGE, TIMG, REACT>(fa, t, lim, kcode, cnt, reinterpret_cast<const double2*>(tile), l,
+                                                  tab, sum, row);
+    }
+};
+
+// Shared memory of one warp (F: Form64 or Form32).  One tile stage: the warps of
+// an SM hide each other's copies (a reached tile is tens of batches), and the
+// room of a second stage lets a fourth warp live on each SM sub-partition.
+template <class F>
+struct OctetSmem {
+    float4 tile[F::SECTIONS * (F::SEC + OCT_GAP)];   // source tile (TMA) and the pad source, by section
+    double row[F::ROW];                   // reactions on the tile's sources (and the pad's)
+    double acc[PB * 3];                   // target sums of the job
+    typename F::Extra x;
+    float4 box[OCTETS][2];                // the block's octet boxes
+    alignas(16) unsigned char list[PB];   // the octet's source list
+    uint64_t bar;
+};
+
+// The octet's list on a tile in the image that octet_reach found, if it did;
+// timg: every listed source has image kcode in every pair that counts.
+template <class F>
+__device__ __forceinline__ int octet_list_any(const ForceArgs& fa, bool uni, const float4 (&box)[2],
+                                              const float4* __restrict__ tile, const typename F::Extra& x, int jlim,
+                                              int jmin, unsigned char* __restrict__ list, int& kcode, bool& timg)
+{
+    if (jlim <= jmin) return 0;
+    float oc[3] = {box[0].x, box[0].y, box[0].z};
+    const float oh[3] = {box[1].x, box[1].y, box[1].z};
+    timg = uni;
+    if (uni) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) oc[c] = fmaf(img_of(kcode, c), fa.Lf[c], oc[c]);
+        return F::template list<true>(fa, oc, oh, tile, x, jlim, jmin, list, kcode);
+    }
+    const int cnt = F::template list<false>(fa, oc, oh, tile, x, jlim, jmin, list, kcode);
+    // the listed sources' one image, where no pair inside r_c has another
+    timg = kcode >= 0;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const float e = 0.5f * fa.Lf[c] - oh[c] - 1.0f;
+        timg = timg && e > 0.f && e * e > fa.scr_c2;
+    }
+    return cnt;
+}
+
+// Asks for units [w0, w1) (slots) of the tile at src.
+template <class F>
+__device__ __forceinline__ void octet_issue(float4* __restrict__ tile, const float4* __restrict__ src, int w0, int w1,
+                                            uint64_t* bar)
+{
+    constexpr int SLOTS = PB / F::SEC;                 // slots per unit
+    const unsigned bytes = (unsigned)((w1 - w0) / SLOTS) * (unsigned)sizeof(float4);
+    mbar_arrive_expect_tx(bar, F::SECTIONS * bytes);
+#pragma unroll
+    for (int k = 0; k < F::SECTIONS; ++k)
+        bulk_g2s(tile + k * (F::SEC + OCT_GAP) + w0 / SLOTS, src + k * F::SEC + w0 / SLOTS, bytes, bar);
+}
+
+// One octet on the tile at hand (sources jmin <= j < jlim, image as octet_reach
+// says): its list, the pairs, the target sums into acc (this lane's target) and
+// S, with REACT the reactions into row (zeroed when the first octet of the
+// tile has pairs: used).
+template <class F, int SIM, bool MEAS, bool RANGE, bool REACT>
+__device__ __forceinline__ void octet_visit(const ForceArgs& fa, const float4* __restrict__ posq, int n, int R, int s,
+                                            const float4 (&box)[2], const float4* __restrict__ tile,
+                                            const typename F::Extra& x, unsigned char* __restrict__ list, bool diag,
+                                            int jmin, int jlim, bool uni, int kcode, double tab,
+                                            double* __restrict__ acc, double (&S)[MEAS ? NSCAL : 1],
+                                            double* __restrict__ row, bool& used)
+{
+    const int lane = threadIdx.x & 31;
+    const typename F::Target t = F::target(posq, R, s, R * PB + s < n);
+    bool timg;
+    const int cnt = octet_list_any<F>(fa, uni, box, tile, x, jlim, jmin, list, kcode, timg);
+    if (cnt == 0) return;
+    if (REACT && !used) {
+        used = true;
+#pragma unroll
+        for (int k = lane; k < PB * 3; k += 32) row[k] = 0.0;
+        __syncwarp();
+    }
+    OctetSum<MEAS> sum;
+    sum.zero();
+    if (timg && !diag) F::template eval<SIM, MEAS, RANGE, true, REACT>(fa, t, -1, kcode, cnt, tile, list, tab, sum, row);
+    else F::template eval<SIM, MEAS, RANGE, false, REACT>(fa, t, diag ? s : -1, kcode, cnt, tile, list, tab, sum, row);
+    // the target sums over the four source lanes
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        sum.f[c] += __shfl_xor_sync(0xffffffffu, sum.f[c], 8);
+        sum.f[c] += __shfl_xor_sync(0xffffffffu, sum.f[c], 16);
+    }
+    if (lane < 8) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) acc[c] += sum.f[c];
+    }
+    if constexpr (MEAS) {
+#pragma unroll
+        for (int k = 0; k < NSCAL; ++k) S[k] += SIM == SIM_MIX ? sum.s[k] * F::weight(t) : sum.s[k];
+    }
+    __syncwarp();                        // the list is free; the next octet adds to the same row
+}
+
 // Job (R, s0, s1) of box bx, one warp: target block R against the sources of
 // windows s0 <= s < s1 (OCT_WIN slots each), writing the target sums to si.
 // Tiles whose box is out of reach of the block's are neither loaded nor looked
 // at.  A tile shared by two jobs has its row written in parts, by both.  q
 // counts the tiles this warp has loaded (stage and mbarrier parity).  Returns
 // false if a copy timed out.
-template <int SIM, bool MEAS, bool RANGE>
-__device__ __forceinline__ bool octets_job(OctetSmem& sm, const ForceArgs& fa, const OctetBox& bx, int R, int s0,
+template <class F, int SIM, bool MEAS, bool RANGE>
+__device__ __forceinline__ bool octets_job(OctetSmem<F>& sm, const ForceArgs& fa, const OctetBox& bx, int R, int s0,
                                            int s1, double* __restrict__ si, double* __restrict__ sm_row,
                                            unsigned* __restrict__ err, unsigned& q, double tab)
 {
-    const int lane = threadIdx.x & 31, a = lane & 7, b = lane >> 3;
+    const int lane = threadIdx.x & 31, a = lane & 7;
     const int n = bx.n;
     const int C0 = s0 / OCT_WPT, C1 = (s1 + OCT_WPT - 1) / OCT_WPT;
 
@@ -553,12 +672,7 @@ __device__ __forceinline__ bool octets_job(OctetSmem& sm, const ForceArgs& fa, c
 #pragma unroll 1
         for (; tiles; tiles &= tiles - 1, ++q) {
             const int C = Cb + __ffs(tiles) - 1;
-            if (lane == 0) {
-                const double2* src = bx.posq + 2 * (size_t)C * PB;
-                mbar_arrive_expect_tx(&sm.bar, 2u * PB * (unsigned)sizeof(double2));
-                bulk_g2s(&sm.tile[0], src, PB * (unsigned)sizeof(double2), &sm.bar);
-                bulk_g2s(&sm.tile[OCT_ZW], src + PB, PB * (unsigned)sizeof(double2), &sm.bar);
-            }
+            if (lane == 0) octet_issue<F>(sm.tile, bx.posq + (size_t)C * OCT_UNITS, 0, PB, &sm.bar);
             // lane o < 16: octet o against the tile's box
             bool uni;
             int kc;
@@ -570,57 +684,24 @@ __device__ __forceinline__ bool octets_job(OctetSmem& sm, const ForceArgs& fa, c
             const bool diag = C == R;
             const int w0 = max(0, (s0 - C * OCT_WPT) * OCT_WIN), w1 = min(PB, (s1 - C * OCT_WPT) * OCT_WIN);
             const int jlim = min(n - C * PB, w1);
-            octet_tile_f32(sm.tile, sm.xs, w0, jlim);
+            F::tile_ready(sm.tile, sm.x, w0, jlim);
             bool used = false;
 #pragma unroll 1
             for (; om; om &= om - 1) {
                 const int o = __ffs(om) - 1;
                 const int s = 8 * o + a;                              // target slot in the block
-                const double2 txy = bx.posq[2 * (size_t)R * PB + s], tzw = bx.posq[2 * (size_t)R * PB + PB + s];
-                double4 pt = make_double4(txy.x, txy.y, tzw.x, tzw.y);
-                if (R * PB + s >= n) pt.x = -OCT_FAR;                 // no target: no pair
-                const int jmin = max(diag ? 8 * o + 1 : 0, w0);
-                int kcode = __shfl_sync(0xffffffffu, kc, o);
-                bool timg;
-                const int cnt = octet_list_any(fa, ((um >> o) & 1u) != 0, sm.box[o], sm.xs, jlim, jmin, sm.list, kcode,
-                                               timg);
-                if (cnt == 0) continue;
-                if (!used) {
-                    used = true;
-#pragma unroll
-                    for (int k = lane; k < PB * 3; k += 32) sm.row[k] = 0.0;
-                    __syncwarp();
-                }
-                OctetSum<MEAS> sum;
-                sum.zero();
-                if (timg && !diag)
-                    octet_eval<SIM, MEAS, RANGE, true, true>(fa, pt, 0, kcode, cnt, sm.tile, sm.list, tab, sum, sm.row);
-                else
-                    octet_eval<SIM, MEAS, RANGE, false, true>(fa, pt, diag ? s : -1, kcode, cnt, sm.tile, sm.list, tab,
-                                                              sum, sm.row);
-                // the target sums over the four source lanes
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    sum.f[c] += __shfl_xor_sync(0xffffffffu, sum.f[c], 8);
-                    sum.f[c] += __shfl_xor_sync(0xffffffffu, sum.f[c], 16);
-                }
-                if (b == 0) {
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) sm.acc[3 * s + c] += sum.f[c];
-                }
-                if constexpr (MEAS) {
-#pragma unroll
-                    for (int k = 0; k < NSCAL; ++k) S[k] += SIM == SIM_MIX ? sum.s[k] * pt.w : sum.s[k];
-                }
-                __syncwarp();                        // the next octet adds to the same row
+                octet_visit<F, SIM, MEAS, RANGE, true>(fa, bx.posq, n, R, s, sm.box[o], sm.tile, sm.x, sm.list, diag,
+                                                       max(diag ? 8 * o + 1 : 0, w0), jlim, ((um >> o) & 1u) != 0,
+                                                       __shfl_sync(0xffffffffu, kc, o), tab, sm.acc + 3 * s, S, sm.row,
+                                                       used);
             }
             const long long u = tri_index(C, R);
             if (!used && w0 == 0 && w1 == PB) {
                 if (lane == 0) bx.Sjf[u] = 0;
             } else {
-                double* dj = bx.Sj + (size_t)u * PB * 3;
+                row_t<F::PREC>* dj = static_cast<row_t<F::PREC>*>(bx.Sj) + (size_t)u * PB * 3;
 #pragma unroll 4
-                for (int k = 3 * w0 + lane; k < 3 * w1; k += 32) dj[k] = used ? sm.row[k] : 0.0;
+                for (int k = 3 * w0 + lane; k < 3 * w1; k += 32) dj[k] = (row_t<F::PREC>)(used ? sm.row[k] : 0.0);
                 if (lane == 0) bx.Sjf[u] = 1;
             }
             __syncwarp();                            // the tile is free
@@ -643,15 +724,14 @@ __device__ __forceinline__ bool octets_job(OctetSmem& sm, const ForceArgs& fa, c
 // fa.exp_ok is 0).
 constexpr int OCT_WARPS = 16;                 // resident warps per SM
 
-template <int SIM, bool MEAS, bool RANGE>
+template <class F, int SIM, bool MEAS, bool RANGE>
 __global__ void __launch_bounds__(32, OCT_WARPS)
 k_force_octets(OctetBox bx, int* __restrict__ job_counter, ForceArgs fa, unsigned* __restrict__ err)
 {
-    __shared__ __align__(128) OctetSmem sm;
+    __shared__ __align__(128) OctetSmem<F> sm;
     const int lane = threadIdx.x;
     if (lane == 0) {
-        sm.tile[OCT_PAD] = make_double2(OCT_FAR, OCT_FAR);
-        sm.tile[OCT_ZW + OCT_PAD] = make_double2(OCT_FAR, 0.0);
+        F::pad(sm.tile);
         mbar_init(&sm.bar, 1);
         fence_mbar_init();
     }
@@ -665,7 +745,7 @@ k_force_octets(OctetBox bx, int* __restrict__ job_counter, ForceArgs fa, unsigne
         if (job >= njobs) break;
         const int4 js = bx.jobs[job];
         if (lane == 0) next = atomicAdd(job_counter, 1);
-        if (!octets_job<SIM, MEAS, RANGE>(sm, fa, bx, js.x, js.y, js.z, bx.Si + (size_t)job * PB * 3,
+        if (!octets_job<F, SIM, MEAS, RANGE>(sm, fa, bx, js.x, js.y, js.z, bx.Si + (size_t)job * PB * 3,
                                           bx.Sm + (size_t)job * NSCAL, err, q, tab))
             return;
     }
@@ -682,8 +762,13 @@ k_force_octets(OctetBox bx, int* __restrict__ job_counter, ForceArgs fa, unsigne
 // that, the last 8 % a twelfth.  (Scheduling the listed costs of 55,296 ions
 // over 1,776 warps: 3 % above the mean against 6 to 37 % for row lengths that
 // ignore the cost; 131,072 ions with r_c = 149 fm 4 % against 37 to 65 %.)
+// No job is cut below OCT_MIN_COST, a quarter of a full unit: shorter ones cost
+// more in their own overhead and sums than they balance (FP64 force kernel and
+// combine, 20,000 ions with r_c = 149 fm: 174 us without the limit, 147 with it,
+// 149 at twice and 212 at four times it).
 // The slots of the scratch rows follow from the table, so which warp runs a
 // job does not matter to the result.
+constexpr int OCT_MIN_COST = 128;
 constexpr int OCT_COST_CTAS = 8;
 constexpr int OCT_JOBS = 3;                   // jobs per resident warp before the cuts get shorter
 
@@ -778,7 +863,7 @@ k_octet_rows(const int* __restrict__ row_cost, int M, int target, int* __restric
         const int f = u < 0.75 ? 1 : (u < 0.92 ? 4 : 12);
         const long long nj =
             R < M ? min(1 + (long long)((double)c * (double)f * (double)target / (double)total),
-                        (long long)OCT_WPT * (M - R)) : 0;
+                        min(1 + c / OCT_MIN_COST, (long long)OCT_WPT * (M - R))) : 0;
         const long long end = jobs + block_scan(nj, red, tot);
         jobs += tot;
         if (R < M) row_start[R + 1] = (int)end;
@@ -855,7 +940,7 @@ k_octet_jobs(const unsigned char* __restrict__ cost, const int* __restrict__ row
 // Sj rows) in a fixed order, the reference's scaling and the store to the
 // caller's order, as k_combine; measuring, also the row's sums of Sm into
 // rsum[R][NSCAL].
-template <int SIM, bool MEAS>
+template <int SIM, int PREC, bool MEAS>
 __global__ void __launch_bounds__(COMB_THREADS)
 k_octet_combine(OctetBox bx, const int* __restrict__ perm, const double* __restrict__ zii,
                 const double* __restrict__ aii, ForceArgs fa, double* __restrict__ a_out, double* __restrict__ rsum)
@@ -894,9 +979,9 @@ k_octet_combine(OctetBox bx, const int* __restrict__ perm, const double* __restr
         }
         __syncthreads();
         const int cnt = nz_count;
-        const double* sj = bx.Sj + (size_t)tri_index(R, 0) * ROW + t;
+        const row_t<PREC>* sj = static_cast<const row_t<PREC>*>(bx.Sj) + (size_t)tri_index(R, 0) * ROW + t;
 #pragma unroll 8
-        for (int q = g; q < cnt; q += COMB_GROUPS) F += sj[(size_t)nzl[q] * ROW];
+        for (int q = g; q < cnt; q += COMB_GROUPS) F += (double)sj[(size_t)nzl[q] * ROW];
     }
     part[g][t] = F;
     __syncthreads();
@@ -935,10 +1020,11 @@ k_octet_combine(OctetBox bx, const int* __restrict__ perm, const double* __restr
 // no reactions to add up (31 FP64 instructions per pair instead of 41, 2
 // shuffles instead of 9), no source-side rows, and chunks as short as the box
 // needs.  One warp per CTA and one CTA per job: the hardware hands them out.
+template <class F>
 struct OctetAllSmem {
-    double2 tile[2][2 * OCT_ZW];
+    float4 tile[2][F::SECTIONS * (F::SEC + OCT_GAP)];
     double acc[32 * 3];
-    float xs[3][PB];
+    typename F::Extra x;
     float4 box[4][2];
     alignas(16) unsigned char list[PB];
     uint64_t bar[2];
@@ -959,17 +1045,18 @@ inline int octet_all_len(int n, int n0 = 16)
     return len;
 }
 
-// Largest box that takes k_force_octets_all (see the engine's setup_octets).
-constexpr int OCT_ALL_MAX_N = 14336;
+// Largest box that takes k_force_octets_all, by form (see the engine's
+// octets_apply).
+constexpr int OCT_ALL_MAX_N64 = 9216, OCT_ALL_MAX_N32 = 6144;
 
 // posq etc. as OctetBox; part: target sums [chunk][slot][3], np slots; Sm: per job.
-template <int SIM, bool MEAS, bool RANGE>
+template <class F, int SIM, bool MEAS, bool RANGE>
 __global__ void __launch_bounds__(32, OCT_ALL_WARPS)
 k_force_octets_all(OctetBox bx, int chunks, int len, double* __restrict__ part, ForceArgs fa,
                    unsigned* __restrict__ err)
 {
-    __shared__ __align__(128) OctetAllSmem sm;
-    const int lane = threadIdx.x, a = lane & 7, b = lane >> 3;
+    __shared__ __align__(128) OctetAllSmem<F> sm;
+    const int lane = threadIdx.x, a = lane & 7;
     const int n = bx.n;
     const int g = blockIdx.x / chunks, ch = blockIdx.x % chunks;   // target group, source chunk
     const int j0 = ch * len, j1 = min(n, j0 + len);                // sources
@@ -981,24 +1068,16 @@ k_force_octets_all(OctetBox bx, int chunks, int len, double* __restrict__ part, 
         fence_mbar_init();
     }
     __syncwarp();
-    // the slots of tile C that the chunk covers, in pieces of 8 (16-byte copies)
+    // the slots of tile C that the chunk covers, in pieces of 8
     auto issue = [&](int C, unsigned qq) {
-        const int w0 = max(0, j0 - C * PB), w1 = min(PB, ((j1 - C * PB) + 7) & ~7);
-        const unsigned bytes = (unsigned)(w1 - w0) * (unsigned)sizeof(double2);
-        const double2* src = bx.posq + 2 * (size_t)C * PB + w0;
-        uint64_t* br = &sm.bar[qq & 1];
-        mbar_arrive_expect_tx(br, 2u * bytes);
-        bulk_g2s(&sm.tile[qq & 1][w0], src, bytes, br);
-        bulk_g2s(&sm.tile[qq & 1][OCT_ZW + w0], src + PB, bytes, br);
+        octet_issue<F>(sm.tile[qq & 1], bx.posq + (size_t)C * OCT_UNITS, max(0, j0 - C * PB),
+                       min(PB, ((j1 - C * PB) + 7) & ~7), &sm.bar[qq & 1]);
     };
     // a chunk inside one tile asks for it at once
     const bool single = C1 - C0 == 1;
     if (single && lane == 0) issue(C0, 0u);
     if (lane < 8) sm.box[lane >> 1][lane & 1] = bx.obox[8 * g + lane];
-    if (lane < 2) {
-        sm.tile[lane][OCT_PAD] = make_double2(OCT_FAR, OCT_FAR);
-        sm.tile[lane][OCT_ZW + OCT_PAD] = make_double2(OCT_FAR, 0.0);
-    }
+    if (lane < 2) F::pad(sm.tile[lane]);
     const double tab = exp2_32_lane();
 #pragma unroll
     for (int k = lane; k < 32 * 3; k += 32) sm.acc[k] = 0.0;
@@ -1039,41 +1118,15 @@ k_force_octets_all(OctetBox bx, int chunks, int len, double* __restrict__ part, 
             }
             const bool diag = C == R;
             const int jmin = max(0, j0 - C * PB), jlim = min(PB, j1 - C * PB);
-            const double2* tl = sm.tile[st];
-            octet_tile_f32(tl, sm.xs, jmin, jlim);
+            F::tile_ready(sm.tile[st], sm.x, jmin, jlim);
+            bool used = false;
 #pragma unroll 1
             for (; om; om &= om - 1) {
                 const int o = __ffs(om) - 1;
-                const int s = 32 * (g % (PB / 32)) + 8 * o + a;        // target slot in the block
-                const double2 txy = bx.posq[2 * (size_t)R * PB + s], tzw = bx.posq[2 * (size_t)R * PB + PB + s];
-                double4 pt = make_double4(txy.x, txy.y, tzw.x, tzw.y);
-                if (R * PB + s >= n) pt.x = -OCT_FAR;                  // no target: no pair
-                int kcode = __shfl_sync(0xffffffffu, kc, o);
-                bool timg;
-                const int cnt = octet_list_any(fa, ((um >> o) & 1u) != 0, sm.box[o], sm.xs, jlim, jmin, sm.list, kcode,
-                                               timg);
-                if (cnt == 0) continue;
-                OctetSum<MEAS> sum;
-                sum.zero();
-                if (timg && !diag)
-                    octet_eval<SIM, MEAS, RANGE, true, false>(fa, pt, 0, kcode, cnt, tl, sm.list, tab, sum, nullptr);
-                else
-                    octet_eval<SIM, MEAS, RANGE, false, false>(fa, pt, diag ? s : -1, kcode, cnt, tl, sm.list, tab, sum,
-                                                               nullptr);
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    sum.f[c] += __shfl_xor_sync(0xffffffffu, sum.f[c], 8);
-                    sum.f[c] += __shfl_xor_sync(0xffffffffu, sum.f[c], 16);
-                }
-                if (b == 0) {
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) sm.acc[3 * (8 * o + a) + c] += sum.f[c];
-                }
-                if constexpr (MEAS) {
-#pragma unroll
-                    for (int k = 0; k < NSCAL; ++k) S[k] += SIM == SIM_MIX ? sum.s[k] * pt.w : sum.s[k];
-                }
-                __syncwarp();                        // the list is free
+                octet_visit<F, SIM, MEAS, RANGE, false>(fa, bx.posq, n, R, 32 * (g % (PB / 32)) + 8 * o + a, sm.box[o],
+                                                        sm.tile[st], sm.x, sm.list, diag, jmin, jlim,
+                                                        ((um >> o) & 1u) != 0, __shfl_sync(0xffffffffu, kc, o), tab,
+                                                        sm.acc + 3 * (8 * o + a), S, nullptr, used);
             }
             if (ahead) {
                 if (lane == 0) issue(Cb + __ffs(ahead) - 1, asked);
