@@ -1,0 +1,43 @@
+"""yk_gofr_counts places pairs in FP32 and takes the exact arithmetic next to a
+bin edge: the counts must equal the oracle's bin for bin (integers, no
+tolerance) where that could go wrong -- pairs exactly on edges, coincident
+particles, coordinates on and outside the faces, unequal edges, bins below the
+FP32 resolution."""
+import numpy as np
+import pytest
+
+from oracle.oracle import Oracle
+from yukawamd_b200 import configs
+from yukawamd_b200.engine import Engine
+
+pytestmark = pytest.mark.gpu
+
+
+def _points(kind, n, xl, rng):
+    L = np.array(xl)
+    if kind == "lattice":              # distances that sit on bin edges, many exactly equal
+        m = int(np.ceil(n ** (1 / 3)))
+        c = rng.permutation(m ** 3)[:n]
+        return np.stack([c // (m * m), c // m % m, c % m], axis=1) / m * L
+    x = rng.random((n, 3)) * L
+    if kind == "faces":                # on and around both faces, some coincident
+        x[::3] = np.where(rng.random(x[::3].shape) < 0.5, 0.0, L)
+        x[1::7] = x[0]
+    if kind == "outside":              # beyond the range that the FP32 place covers
+        x[::5] += (rng.random(x[::5].shape) - 0.5) * L
+    return x
+
+
+@pytest.mark.parametrize("nbin", [1, 100, 8192])
+@pytest.mark.parametrize("kind,xl", [("lattice", (64.0, 64.0, 64.0)), ("faces", (71.3, 71.3, 71.3)),
+                                     ("faces", (40.0, 71.3, 250.0)), ("outside", (71.3, 50.0, 90.0)),
+                                     ("uniform", (1.7e4, 1.7e4, 1.7e4)), ("uniform", (1e-3, 2e-3, 1e-3))])
+def test_counts_equal_oracle(gpu, kind, xl, nbin):
+    n = 1153                           # nine tiles and one particle
+    w = configs.pure_ion_ocp(3, n)
+    w.x = np.ascontiguousarray(_points(kind, n, xl, np.random.default_rng(nbin)).reshape(-1))
+    w.params["xl"] = list(xl)
+    w.params["rccut"] = 0.3 * min(xl)
+    p = w.yk_params()
+    with Engine(p, w.x, w.v, w.zii, w.aii) as e:
+        assert np.array_equal(e.gofr_counts(nbin), Oracle("double").gofr_counts(p, w.x, nbin))

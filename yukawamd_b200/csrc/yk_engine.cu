@@ -1506,11 +1506,12 @@ int yk_gofr_counts(yk_ctx* c, int nbin, double* counts)
     g.nbin = nbin;
     g.n = c->n;
     g.M = (c->n + GOFR_BLOCK - 1) / GOFR_BLOCK;
+    gofr_place(g);
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->dev);
     const long long units = (long long)g.M * (g.M + 1) / 2;
     const int grid = (int)std::min<long long>(units, 8LL * sms);
-    const size_t smem = GOFR_BLOCK * sizeof(double4) + sizeof(unsigned) * (size_t)nbin;
+    const size_t smem = 3 * GOFR_BLOCK * sizeof(float) + sizeof(unsigned) * (size_t)nbin;
     CK(c, cudaFuncSetAttribute(k_gofr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     CK(c, cudaMemsetAsync(c->gofr, 0, sizeof(unsigned long long) * (size_t)nbin, c->stream));
     k_gofr<<<grid, GOFR_BLOCK, smem, c->stream>>>(c->pos, g, c->gofr);
