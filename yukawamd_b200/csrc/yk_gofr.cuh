@@ -21,9 +21,9 @@
 // coordinates is within GofrArgs::eps of the reference's fac2 rr, so a place
 // that far or farther from both edges of its bin is the reference's.  The rest
 // (1 in 1,000 on 500 bins) take the exact arithmetic.  27,000 ions, 500 bins:
-// 1,015 -> 340 us; what is left is the FP32 arithmetic and the shared-memory
-// atomics.  (min(|d|, L - |d|) is continuous in d, and |d - L rint(d / L)| is
-// the same value, so no pair's image matters to the bound.)
+// 1,037 -> 489 us a call, bound by instruction issue.  (min(|d|, L - |d|) is
+// continuous in d, and |d - L rint(d / L)| is the same value, so no pair's
+// image matters to the bound.)
 #pragma once
 
 #include <algorithm>
@@ -86,6 +86,64 @@ __device__ __forceinline__ int gofr_bin(const GofrArgs& g, const double4& pi, co
     return min(g.nbin, __double2int_rz(__dadd_rn(__dmul_rn(g.fac2, rr), 1.0))) - 1;
 }
 
+// The unit loop's constants, held in registers: opaque moves, because the
+// compiler otherwise loads each one from the constant bank in every pass.
+struct GofrRegs {
+    float il[3], nl[3], f2;
+};
+
+__device__ __forceinline__ float gofr_keep(float v)
+{
+    float r;
+    asm volatile("mov.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+__device__ __forceinline__ float2 gofr_dup(float v) { return make_float2(v, v); }
+
+// One target against the tile's sources jstart <= jj < cnt (EDGE: not all of
+// them count; those that do not go to the counter past the last bin).  The
+// lanes of a warp start at different sources, so that their counters differ.
+template <bool EDGE>
+__device__ __forceinline__ void gofr_unit(const GofrArgs& g, const GofrRegs& k, const float2* __restrict__ tx,
+                                          unsigned hs, const double4& pi, const float (&xi)[3],
+                                          const double4* __restrict__ src, int jstart, int cnt)
+{
+#pragma unroll 2
+    for (int q = 0; q < GOFR_BLOCK / 2; ++q) {
+        const int p = (q + threadIdx.x) & (GOFR_BLOCK / 2 - 1);
+        float2 r2 = gofr_dup(0.f);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const float2 d = __fadd2_rn(tx[c * (GOFR_BLOCK / 2) + p], gofr_dup(-xi[c]));
+            const float2 m = __fadd2_rn(__ffma2_rn(d, gofr_dup(k.il[c]), gofr_dup(12582912.0f)),
+                                        gofr_dup(-12582912.0f));
+            const float2 y = __ffma2_rn(gofr_dup(k.nl[c]), m, d);
+            r2 = __ffma2_rn(y, y, r2);
+        }
+        float2 r;
+        asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(r2.x));
+        asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(r2.y));
+        // w: the place from the middle of bin 0; b: its bin, as the low bits of
+        // the magic sum; f: the place from the middle of that bin
+        const float2 w = __ffma2_rn(gofr_dup(k.f2), r, gofr_dup(-0.5f));
+        const float2 b = __fadd2_rn(w, gofr_dup(12582912.0f));
+        const float2 f = sub2(w, __fadd2_rn(b, gofr_dup(-12582912.0f)));
+        int b0 = min(__float_as_int(b.x) - 0x4B400000, g.nbin - 1);
+        int b1 = min(__float_as_int(b.y) - 0x4B400000, g.nbin - 1);
+        if (fmaxf(fabsf(f.x), fabsf(f.y)) > g.in_bin) {
+            if (fabsf(f.x) > g.in_bin && (!EDGE || 2 * p < cnt)) b0 = gofr_bin(g, pi, src[2 * p]);
+            if (fabsf(f.y) > g.in_bin && (!EDGE || 2 * p + 1 < cnt)) b1 = gofr_bin(g, pi, src[2 * p + 1]);
+        }
+        if constexpr (EDGE) {
+            if (2 * p < jstart || 2 * p >= cnt) b0 = g.nbin;
+            if (2 * p + 1 < jstart || 2 * p + 1 >= cnt) b1 = g.nbin;
+        }
+        asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(hs + 4u * (unsigned)b0) : "memory");
+        asm volatile("red.shared.add.u32 [%0], 1;" ::"r"(hs + 4u * (unsigned)b1) : "memory");
+    }
+}
+
 static __global__ void __launch_bounds__(GOFR_BLOCK)
 k_gofr(const double4* __restrict__ pos, GofrArgs g, unsigned long long* __restrict__ hist)
 {
@@ -94,6 +152,14 @@ k_gofr(const double4* __restrict__ pos, GofrArgs g, unsigned long long* __restri
     unsigned* h = reinterpret_cast<unsigned*>(gsm + 3 * GOFR_BLOCK * sizeof(float));
     const int tid = threadIdx.x;
     for (int b = tid; b < g.nbin; b += GOFR_BLOCK) h[b] = 0u;
+    const unsigned hs = smem_u32(h);
+    GofrRegs k;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        k.il[c] = gofr_keep(g.ixlf[c]);
+        k.nl[c] = gofr_keep(-g.xlf[c]);
+    }
+    k.f2 = gofr_keep(g.fac2f);
     const long long units = (long long)g.M * (g.M + 1) / 2;
     for (long long u = blockIdx.x; u < units; u += gridDim.x) {
         // u = C (C + 1) / 2 + R with 0 <= R <= C
@@ -111,52 +177,23 @@ k_gofr(const double4* __restrict__ pos, GofrArgs g, unsigned long long* __restri
         const float xj[3] = {__double2float_rn(pj.x), __double2float_rn(pj.y), __double2float_rn(pj.z)};
         bool in = g.in_bin >= 0.0f;
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            const float mid = 0.5f * g.xlf[k], reach = 0.624f * g.xlf[k];
-            in = in && fabsf(xi[k] - mid) <= reach && fabsf(xj[k] - mid) <= reach;
+        for (int c = 0; c < 3; ++c) {
+            const float mid = 0.5f * g.xlf[c], reach = 0.624f * g.xlf[c];
+            in = in && fabsf(xi[c] - mid) <= reach && fabsf(xj[c] - mid) <= reach;
         }
         __syncthreads();                     // the previous unit's tile is no longer read
 #pragma unroll
-        for (int k = 0; k < 3; ++k) reinterpret_cast<float*>(tx)[k * GOFR_BLOCK + tid] = xj[k];
+        for (int c = 0; c < 3; ++c) reinterpret_cast<float*>(tx)[c * GOFR_BLOCK + tid] = xj[c];
         const bool place = __syncthreads_and(in);
         const int jstart = on ? ((C == R) ? tid + 1 : 0) : cnt;
         if (!place) {
             for (int jj = jstart; jj < cnt; ++jj) atomicAdd(&h[gofr_bin(g, pi, pos[j0 + jj])], 1u);
             continue;
         }
-        // the lanes of a warp start at different sources, so that their
-        // counters differ
-        const float2 nx[3] = {make_float2(-xi[0], -xi[0]), make_float2(-xi[1], -xi[1]), make_float2(-xi[2], -xi[2])};
-#pragma unroll 2
-        for (int q = 0; q < GOFR_BLOCK / 2; ++q) {
-            const int p = (q + tid) & (GOFR_BLOCK / 2 - 1);
-            float2 r2 = make_float2(0.f, 0.f);
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const float2 d = __fadd2_rn(tx[k * (GOFR_BLOCK / 2) + p], nx[k]);
-                const float2 m = __fadd2_rn(__ffma2_rn(d, make_float2(g.ixlf[k], g.ixlf[k]),
-                                                       make_float2(12582912.0f, 12582912.0f)),
-                                            make_float2(-12582912.0f, -12582912.0f));
-                const float2 y = __ffma2_rn(make_float2(-g.xlf[k], -g.xlf[k]), m, d);
-                r2 = __ffma2_rn(y, y, r2);
-            }
-            float2 r;
-            asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r.x) : "f"(r2.x));
-            asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r.y) : "f"(r2.y));
-            // c: the place from the middle of bin 0; b: its bin, as the low
-            // bits of the magic sum; f: the place from the middle of that bin
-            const float2 c = __ffma2_rn(make_float2(g.fac2f, g.fac2f), r, make_float2(-0.5f, -0.5f));
-            const float2 b = __fadd2_rn(c, make_float2(12582912.0f, 12582912.0f));
-            const float2 f = sub2(c, __fadd2_rn(b, make_float2(-12582912.0f, -12582912.0f)));
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-                const int jj = 2 * p + e;
-                if (jj < jstart || jj >= cnt) continue;
-                int bin = min(__float_as_int(e ? b.y : b.x) - 0x4B400000, g.nbin - 1);
-                if (fabsf(e ? f.y : f.x) > g.in_bin) bin = gofr_bin(g, pi, pos[j0 + jj]);
-                atomicAdd(&h[bin], 1u);
-            }
-        }
+        if (C != R && cnt == GOFR_BLOCK && (R + 1) * GOFR_BLOCK <= g.n)
+            gofr_unit<false>(g, k, tx, hs, pi, xi, pos + j0, 0, GOFR_BLOCK);
+        else
+            gofr_unit<true>(g, k, tx, hs, pi, xi, pos + j0, jstart, cnt);
     }
     __syncthreads();
     for (int b = tid; b < g.nbin; b += GOFR_BLOCK)
