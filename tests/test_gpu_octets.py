@@ -70,3 +70,18 @@ def test_no_cutoff(gpu, orc, n, rccut):
     w = configs.pure_ion_ocp(11, n)
     w.params["rccut"] = rccut
     check_accel(orc, w, abi.YK_PREC_FP64, True)
+
+
+@PRECS
+@pytest.mark.parametrize("n", [700, 24577])
+def test_power_of_two_edges(gpu, orc, n, prec):
+    """Box edges of 2^8 fm: an image shift of a far-away value by whole edges
+    is exact, so a pad of a source list that is told by its distance alone
+    must stay far away under any shift."""
+    w = workload("pure", n, 77 + n)
+    L = np.array(w.params["xl"])
+    w.x = np.ascontiguousarray((w.x.reshape(-1, 3) / L * 256.0).reshape(-1))
+    w.params["xl"] = [256.0, 256.0, 256.0]
+    w.params["rccut"] = 76.8
+    check_accel(orc, w, prec, True)
+    check_accel(orc, w, prec, False)

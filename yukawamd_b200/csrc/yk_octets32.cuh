@@ -23,6 +23,11 @@
 
 namespace yk {
 
+// Lo part of what is beyond every cutoff: list pads, empty slots, targets that
+// are none.  In the hi part it would go through the image shift, which takes
+// it to exactly 0 in a box whose edge is a power of two.
+constexpr float OCT_FAR32 = 1e18f;
+
 __device__ __forceinline__ float2 oct_dup(float v) { return make_float2(v, v); }
 
 __device__ __forceinline__ float rsqrt_ftz(float x)
@@ -166,10 +171,10 @@ struct Form32 {
         float h[3], l[3];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            // an empty slot is beyond every cutoff
-            const double hd = on ? shadow_hi(x[c]) : 1e18;
+            // an empty slot is beyond every cutoff (OCT_FAR32, in the lo part)
+            const double hd = on ? shadow_hi(x[c]) : 0.0;
             h[c] = __double2float_rn(hd);
-            l[c] = on ? __double2float_rn(__dsub_rn(x[c], hd)) : 0.f;
+            l[c] = on ? __double2float_rn(__dsub_rn(x[c], hd)) : OCT_FAR32;
         }
         t[0] = h[0];
         t[2] = h[1];
@@ -183,10 +188,10 @@ struct Form32 {
 
     static __device__ __forceinline__ void pad(float4* __restrict__ tile)
     {
-        tile[SEC] = make_float4(1e18f, 1e18f, 1e18f, 1e18f);
-        tile[SEC + SMEM_SEC] = make_float4(1e18f, 1e18f, 0.f, 0.f);
-        tile[SEC + 2 * SMEM_SEC] = make_float4(0.f, 0.f, 0.f, 0.f);
-        tile[SEC + 3 * SMEM_SEC] = make_float4(0.f, 0.f, 0.f, 0.f);
+        tile[SEC] = make_float4(0.f, 0.f, 0.f, 0.f);
+        tile[SEC + SMEM_SEC] = make_float4(0.f, 0.f, 0.f, 0.f);
+        tile[SEC + 2 * SMEM_SEC] = make_float4(OCT_FAR32, OCT_FAR32, OCT_FAR32, OCT_FAR32);
+        tile[SEC + 3 * SMEM_SEC] = make_float4(OCT_FAR32, OCT_FAR32, 0.f, 0.f);
     }
 
     static __device__ __forceinline__ void tile_ready(const float4*, Extra&, int, int) {}
@@ -195,11 +200,11 @@ struct Form32 {
     {
         const float* t = reinterpret_cast<const float*>(posq + (size_t)R * OCT_UNITS) + 4 * (s >> 1) + (s & 1);
         Target r;
-        r.h[0] = on ? -t[0] : 1e18f;      // no target: far from every source, the empty slots' too
+        r.h[0] = -t[0];
         r.h[1] = -t[2];
         r.h[2] = -t[4 * SEC];
         r.w = t[4 * SEC + 2];
-        r.l[0] = -t[8 * SEC];
+        r.l[0] = on ? -t[8 * SEC] : OCT_FAR32;      // no target: far from every source, the empty slots' too
         r.l[1] = -t[8 * SEC + 2];
         r.l[2] = -t[12 * SEC];
         return r;
