@@ -85,3 +85,28 @@ def test_power_of_two_edges(gpu, orc, n, prec):
     w.params["rccut"] = 76.8
     check_accel(orc, w, prec, True)
     check_accel(orc, w, prec, False)
+
+
+@pytest.mark.parametrize("n,prec", [(100, abi.YK_PREC_FP64), (4096, abi.YK_PREC_FP64), (4097, abi.YK_PREC_FP64),
+                                    (101, abi.YK_PREC_MIXED), (2047, abi.YK_PREC_MIXED), (2049, abi.YK_PREC_MIXED)])
+@pytest.mark.parametrize("terms", ["both", "nuclear", "coulomb", "cut", "edges"])
+def test_small_nucleon_boxes(gpu, orc, n, prec, terms):
+    """Nucleons up to and past the sizes that take every pair from both sides:
+    each term alone, a Coulomb cutoff inside the box, and box edges of a power
+    of two with protons exactly half an edge apart (the image's boundary)."""
+    w = workload("nn", n, 900 + n)
+    if terms == "nuclear":
+        w.params["coulomb_on"] = 0
+    elif terms == "coulomb":
+        w.params["nuclear_on"] = 0
+    elif terms == "cut":
+        w.params["rccut"] = 0.4 * w.params["xl"][0]
+    elif terms == "edges":
+        edge = 2.0 ** np.ceil(np.log2(w.params["xl"][0]))
+        x = w.x.reshape(-1, 3) / np.array(w.params["xl"]) * edge
+        protons = np.flatnonzero(np.asarray(w.zii)[:n] == 1.0)
+        x[protons[1]] = (x[protons[0]] + [0.5 * edge, 1.0, 2.0]) % edge
+        w.x = np.ascontiguousarray(x.reshape(-1))
+        w.params["xl"] = [edge] * 3
+    check_accel(orc, w, prec, True)
+    check_accel(orc, w, prec, False)

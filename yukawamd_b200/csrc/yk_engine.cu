@@ -265,7 +265,7 @@ static void setup_args(yk_ctx* c)
         std::memcpy(&f.hlb[k], &hl, sizeof hl);
     }
     f.rc2 = std::min(p.rccut * p.rccut, std::numeric_limits<double>::max());
-    f.rn2 = p.rncut * p.rncut;
+    f.rn2 = std::min(p.rncut * p.rncut, std::numeric_limits<double>::max());
     f.xmuc = p.xmuc;
     f.vc = p.vc;
     f.evcut = (p.sim_type == YK_SIM_NUCLEON) ? ev_cut(p, p.vc) : ev_cut(p, 1.0);
@@ -493,6 +493,15 @@ static void build_pair_jobs2(int M, int smax, int P, std::vector<int4>& jobs, st
 // cutoff), so nucleons take two targets only when asked (the tuner tries it).
 constexpr int TPT2_AUTO_MIN_N = 16384;
 constexpr int OCT_MIXED_MIN_N = 24576;
+// Small nucleon boxes take the all-pairs octets (octets_apply).  Their uncut p-p
+// Coulomb term leaves the lists little to skip, so the form only pays where
+// the half-pair units are too few (step, k_force_pairs / octets; FP64 500
+// nucleons 94 / 48 us, 2,000 100 / 64, 4,000 111 / 90, 5,000 130 / 120 but
+// measuring 152 / 153, 12,000 231 / 311; mixed 500 67 / 50 us, 2,000 70 / 63,
+// 5,000 94 / 110.  Half pairs on octets, 51,200 nucleons: FP64 1,702 / 1,619
+// us, mixed 832 / 1,431.)
+constexpr int OCT_NN_MAX_N64 = 4096;
+constexpr int OCT_NN_MAX_N32 = 2048;
 constexpr int DEFAULT_SEG_MIXED_TT2 = 8;
 
 static int pair_tt(const yk_ctx* c)
@@ -589,7 +598,8 @@ static void free_pairs(yk_ctx* c)
 static bool octets_apply(const yk_ctx* c)
 {
     if (c->kernel_req == 3 || pair_tt(c) != 1) return false;
-    if (c->p.sim_type != YK_SIM_PURE_ION && c->p.sim_type != YK_SIM_ION_MIXTURE) return false;
+    if (c->p.sim_type == YK_SIM_NUCLEON)
+        return c->p.precision == YK_PREC_FP64 ? c->n <= OCT_NN_MAX_N64 : c->n <= OCT_NN_MAX_N32 && c->fa.hilo;
     if (c->p.precision == YK_PREC_FP64) return true;
     return c->fa.lo && (c->n <= OCT_ALL_MAX_N32 || c->n >= OCT_MIXED_MIN_N);
 }
@@ -600,7 +610,7 @@ static bool octets_apply(const yk_ctx* c)
 // 100 / 89 / 109; 8,000 134 / 121 / 142; 10,000 155 / 150 / 145).
 static bool octets_all(const yk_ctx* c)
 {
-    return c->n <= (c->p.precision == YK_PREC_FP64 ? OCT_ALL_MAX_N64 : OCT_ALL_MAX_N32);
+    return c->n <= (c->p.precision == YK_PREC_FP64 ? OCT_ALL_MAX_N64 : OCT_ALL_MAX_N32);   // (all nucleon octets)
 }
 
 // Scratch of the octet kernels.
@@ -815,14 +825,16 @@ static int launch_octets(yk_ctx* c)
     float4* tbox = reinterpret_cast<float4*>(c->tbox);
     // exponents past 700 (FP64 only; the mixed form's hardware exponential
     // flushes to 0)
-    const bool range = F::PREC == PREC_FP64 && !c->fa.exp_ok;
+    // (nucleons: always, inside octet_batch_nn)
+    constexpr bool RANGE = F::PREC == PREC_FP64 && SIM != SIM_NUCLEON;
+    const bool range = RANGE && !c->fa.exp_ok;
     k_octet_pack<F><<<M, PB, 0, st>>>(c->pos, c->n, c->fa, c->posq, c->obox, tbox);
     int k = 3;
     if (c->oct_chunks) {
-        const OctetBox bx{c->posq, c->obox, tbox, nullptr, nullptr, nullptr, c->Sm, nullptr, nullptr, c->n, M};
+        const OctetBox bx{c->pos, c->posq, c->obox, tbox, nullptr, nullptr, nullptr, c->Sm, nullptr, nullptr, c->n, M};
         const int grid = M * (PB / 32) * c->oct_chunks;
         if (range)
-            k_force_octets_all<F, SIM, MEAS, F::PREC == PREC_FP64><<<grid, 32, 0, st>>>(bx, c->oct_chunks, c->oct_len,
+            k_force_octets_all<F, SIM, MEAS, RANGE><<<grid, 32, 0, st>>>(bx, c->oct_chunks, c->oct_len,
                                                                                        c->Si, c->fa, c->err);
         else
             k_force_octets_all<F, SIM, MEAS, false><<<grid, 32, 0, st>>>(bx, c->oct_chunks, c->oct_len, c->Si, c->fa,
@@ -831,34 +843,34 @@ static int launch_octets(yk_ctx* c)
                                                                    c->aii, c->fa, c->a, c->rsum);
         return k;
     }
-    cudaMemsetAsync(c->job_counter, 0, sizeof(int), st);
-    if (c->oct_jobs_due) {
-        k_octet_cost<<<dim3(M, OCT_COST_CTAS), 256, 0, st>>>(c->obox, tbox, M, c->fa, c->oct_cost, c->row_cost);
-        k_octet_rows<<<1, 1024, 0, st>>>(c->row_cost, M, c->oct_target, c->row_start);
-        k_octet_jobs<<<M, 1024, 0, st>>>(c->oct_cost, c->row_cost, M, c->row_start, c->jobs);
-        c->oct_jobs_due = false;
-        k += 3;
+    if constexpr (SIM != SIM_NUCLEON) {
+        cudaMemsetAsync(c->job_counter, 0, sizeof(int), st);
+        if (c->oct_jobs_due) {
+            k_octet_cost<<<dim3(M, OCT_COST_CTAS), 256, 0, st>>>(c->obox, tbox, M, c->fa, c->oct_cost, c->row_cost);
+            k_octet_rows<<<1, 1024, 0, st>>>(c->row_cost, M, c->oct_target, c->row_start);
+            k_octet_jobs<<<M, 1024, 0, st>>>(c->oct_cost, c->row_cost, M, c->row_start, c->jobs);
+            c->oct_jobs_due = false;
+            k += 3;
+        }
+        const OctetBox bx{c->pos, c->posq, c->obox, tbox, c->Si, c->Sj, c->Sjf, c->Sm, c->jobs, c->row_start, c->n, M};
+        const int grid = OCT_WARPS * c->sms;
+        if (range) k_force_octets<F, SIM, MEAS, RANGE><<<grid, 32, 0, st>>>(bx, c->job_counter, c->fa, c->err);
+        else k_force_octets<F, SIM, MEAS, false><<<grid, 32, 0, st>>>(bx, c->job_counter, c->fa, c->err);
+        const size_t smem = comb_smem_bytes(M);
+        if (smem > (size_t)40 << 10)
+            cudaFuncSetAttribute(k_octet_combine<SIM, F::PREC, MEAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)smem);
+        k_octet_combine<SIM, F::PREC, MEAS><<<M, COMB_THREADS, smem, st>>>(bx, c->perm, c->zii, c->aii, c->fa, c->a,
+                                                                           c->rsum);
     }
-    const OctetBox bx{c->posq, c->obox, tbox, c->Si, c->Sj, c->Sjf, c->Sm, c->jobs, c->row_start, c->n, M};
-    const int grid = OCT_WARPS * c->sms;
-    if (range) k_force_octets<F, SIM, MEAS, F::PREC == PREC_FP64><<<grid, 32, 0, st>>>(bx, c->job_counter, c->fa, c->err);
-    else k_force_octets<F, SIM, MEAS, false><<<grid, 32, 0, st>>>(bx, c->job_counter, c->fa, c->err);
-    const size_t smem = comb_smem_bytes(M);
-    if (smem > (size_t)40 << 10)
-        cudaFuncSetAttribute(k_octet_combine<SIM, F::PREC, MEAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
-    k_octet_combine<SIM, F::PREC, MEAS><<<M, COMB_THREADS, smem, st>>>(bx, c->perm, c->zii, c->aii, c->fa, c->a,
-                                                                       c->rsum);
     return k;
 }
 
 template <int SIM, int PREC, bool MEAS>
 static int launch_force_t(yk_ctx* c)
 {
-    if constexpr (SIM != SIM_NUCLEON) {
-        using F = std::conditional_t<PREC == PREC_FP64, Form64, Form32>;
-        if (c->kernel == 2 && c->oct) return launch_octets<F, SIM, MEAS>(c);
-    }
+    using F = std::conditional_t<PREC == PREC_FP64, Form64, Form32>;
+    if (c->kernel == 2 && c->oct) return launch_octets<F, SIM, MEAS>(c);
     if (c->kernel == 1) {
         k_force_rows<SIM, PREC, MEAS><<<c->nfb, FBLOCK, FORCE_SMEM, c->stream>>>(
             c->pos, c->posf, c->perm, c->aii, c->fa, c->a, c->fpart, c->err);
@@ -2072,7 +2084,7 @@ static void noalloc_octets(cudaStream_t st, const NoallocLayout& L, unsigned cha
     double* part = reinterpret_cast<double*>(b + L.Si);
     double* Sm = reinterpret_cast<double*>(b + L.Sm);
     k_octet_pack<Form64><<<L.M, PB, 0, st>>>(pos, fa.n, fa, posq, obox, tbox);
-    const OctetBox bx{posq, obox, tbox, nullptr, nullptr, nullptr, Sm, nullptr, nullptr, fa.n, L.M};
+    const OctetBox bx{pos, posq, obox, tbox, nullptr, nullptr, nullptr, Sm, nullptr, nullptr, fa.n, L.M};
     const int grid = L.M * (PB / 32) * L.chunks;
     if (fa.exp_ok) k_force_octets_all<Form64, SIM, MEAS, false><<<grid, 32, 0, st>>>(bx, L.chunks, L.len, part, fa, err);
     else k_force_octets_all<Form64, SIM, MEAS, true><<<grid, 32, 0, st>>>(bx, L.chunks, L.len, part, fa, err);

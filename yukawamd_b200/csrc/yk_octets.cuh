@@ -25,6 +25,8 @@
 // of 9), and no per-pair FP32 screen is needed.
 #pragma once
 
+#include <type_traits>
+
 #include <algorithm>
 
 #include "yk_pairs.cuh"
@@ -259,6 +261,109 @@ __device__ __forceinline__ void octet_batch(const ForceArgs& fa, const double4& 
     }
 }
 
+// octet_batch for nucleons (int_nn.f:208-229): the HPP terms inside rncut, taken
+// only if a lane of the warp has such a pair, and, with COUL (the octet and the
+// tile hold protons), the p-p Coulomb terms of proton pairs inside rccut.
+// Every pair from both sides: no reactions.
+template <bool MEAS, bool COUL, bool TIMG, int NQ>
+__device__ __forceinline__ void octet_batch_nn(const ForceArgs& fa, const double4& pt, unsigned w, int sw, int lim,
+                                               const double2* __restrict__ tl, double tab, OctetSum<MEAS>& sum)
+{
+    double d[NQ][3], r2[NQ], fs[NQ], u[NQ], wj[NQ];
+    bool ok[NQ], hn[NQ], any = false;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        const int jl = (int)__byte_perm(w, 0, 0x4440u | (unsigned)(q ^ sw));
+        const double2 xy = tl[jl], zw = tl[jl + OCT_ZW];
+        d[q][0] = __dsub_rn(pt.x, xy.x);
+        d[q][1] = __dsub_rn(pt.y, xy.y);
+        d[q][2] = __dsub_rn(pt.z, zw.x);
+        wj[q] = zw.y;
+        ok[q] = TIMG || jl != lim;
+    }
+    if constexpr (!TIMG) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) d[q][c] = min_image_abs(d[q][c], fa.xl[c]);
+    }
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) r2[q] = __dmul_rn(d[q][2], d[q][2]);
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) r2[q] = __fma_rn(d[q][1], d[q][1], r2[q]);
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        r2[q] = __fma_rn(d[q][0], d[q][0], r2[q]);
+        hn[q] = fa.nuclear_on && r2[q] <= fa.rn2 && ok[q];
+        any = any || hn[q];
+        fs[q] = 0.0;
+        u[q] = 0.0;
+    }
+    any = __any_sync(0xffffffffu, any);
+    if (!COUL && !any) return;
+    double sc[NQ], v[NQ];
+    if constexpr (COUL) {
+        double x[NQ], y[NQ], mr[NQ];
+        bool hc[NQ];
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            hc[q] = r2[q] <= fa.rc2 && ok[q] && pt.w == 1.0 && wj[q] == 1.0;
+            x[q] = __hiloint2double(hc[q] ? __double2hiint(r2[q]) : 0x3ff00000, __double2loint(r2[q]));
+            asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y[q]) : "d"(x[q]));
+        }
+        rsqrt_h64_step<NQ>(x, y);
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) mr[q] = __dmul_rn(x[q], y[q]);
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) mr[q] = __dmul_rn(mr[q], fa.xmuc);
+        exp_neg_f64_warp<true, NQ>(mr, tab, sc, v);
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) v[q] = __dmul_rn(__dmul_rn(v[q], fa.vc), y[q]);   // vc e^{-mu r}/r
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            if constexpr (MEAS) u[q] = hc[q] ? v[q] - fa.evcut : 0.0;
+            const double g = __dmul_rn(v[q], __dmul_rn(y[q], y[q]));
+            fs[q] = hc[q] ? __fma_rn(mr[q], g, g) : 0.0;
+        }
+    }
+    if (any) {
+        double t[NQ];
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) t[q] = hn[q] ? __dmul_rn(r2[q], fa.xp2i) : 0.0;
+        exp_neg_f64_warp<true, NQ>(t, tab, sc, v);
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            const double B = pt.w == wj[q] ? fa.bpc : fa.bmc;
+            const double fn = __dmul_rn(__dmul_rn(fa.xpi, __fma_rn(fa.aa2, v[q], B)), v[q]);
+            if (hn[q]) {
+                fs[q] = __dadd_rn(fs[q], fn);
+                if constexpr (MEAS) u[q] += (fa.aa * v[q] + B) * v[q];
+            }
+        }
+    }
+    // fs = 0 unless the pair interacts; d and r^2 of a pad or an empty target
+    // are as large as OCT_FAR, and only fs d and (MEAS) fs r^2 would see it
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        double f[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            f[c] = __dmul_rn(fs[q], d[q][c]);
+            sum.f[c] = __dadd_rn(sum.f[c], f[c]);
+        }
+        if constexpr (MEAS) {
+            sum.s[0] += u[q];
+            sum.s[1] += fs[q] * (fs[q] != 0.0 ? r2[q] : 0.0);
+            sum.s[2] += d[q][0] * f[0];
+            sum.s[3] += d[q][0] * f[1];
+            sum.s[4] += d[q][0] * f[2];
+            sum.s[5] += d[q][1] * f[1];
+            sum.s[6] += d[q][1] * f[2];
+            sum.s[7] += d[q][2] * f[2];
+        }
+    }
+}
+
 // The octet's source list on a tile: lane l tests sources l, l + 32, ... against
 // the octet's box (centre oc, half-width oh).  UNI: oc already carries the one
 // image of the whole tile; otherwise each source takes its own minimum image,
@@ -266,8 +371,11 @@ __device__ __forceinline__ void octet_batch(const ForceArgs& fa, const double4& 
 // bounding sphere in place of the box saves 6 of the 13 instructions of a
 // test but lists about 5 % more sources: 55,296 ions FP64 1,314 -> 1,361 us,
 // mixed 720 -> 742 us.)
-template <bool UNI>
-__device__ __forceinline__ int octet_list(const ForceArgs& fa, const float (&oc)[3], const float (&oh)[3],
+// limp, lim: squared radius for a proton and for any other source (ions: the
+// same).
+template <bool UNI, bool NUC>
+__device__ __forceinline__ int octet_list(const ForceArgs& fa, const float (&oc)[3], const float (&oh)[3], float limp,
+                                          float lim, const double2* __restrict__ tl,
                                           const float (*__restrict__ xs)[PB], int jlim, int jmin,
                                           unsigned char* __restrict__ list, int& kcode)
 {
@@ -295,7 +403,9 @@ __device__ __forceinline__ int octet_list(const ForceArgs& fa, const float (&oc)
             const float m = fmaxf(fabsf(v) - oh[c], 0.f);
             dist2 = fmaf(m, m, dist2);
         }
-        const bool near = (unsigned)(j - jmin) < (unsigned)(jlim - jmin) && dist2 <= fa.scr_c2;
+        bool near = dist2 <= lim;
+        if constexpr (NUC) near = near || (dist2 <= limp && tl[j + OCT_ZW].y == 1.0);
+        near = near && (unsigned)(j - jmin) < (unsigned)(jlim - jmin);
         if constexpr (!UNI) {
             if (near) {
                 c_and &= code;
@@ -316,7 +426,7 @@ __device__ __forceinline__ int octet_list(const ForceArgs& fa, const float (&oc)
 }
 
 // One octet (target pt, diagonal rule lim) on its list of cnt sources.
-template <int SIM, bool MEAS, bool RANGE, bool TIMG, bool REACT>
+template <int SIM, bool MEAS, bool RANGE, bool TIMG, bool REACT, bool COUL>
 __device__ __forceinline__ void octet_eval(const ForceArgs& fa, double4 pt, int lim, int kcode, int cnt,
                                            const double2* __restrict__ tl, const unsigned char* __restrict__ list,
                                            double tab, OctetSum<MEAS>& sum, double* __restrict__ row)
@@ -333,11 +443,17 @@ __device__ __forceinline__ void octet_eval(const ForceArgs& fa, double4 pt, int 
 #pragma unroll 1
     for (; cnt - k > 8; k += 16) {
         const unsigned w = *reinterpret_cast<const unsigned*>(&list[k + 4 * b]);
-        octet_batch<SIM, MEAS, RANGE, TIMG, REACT, 4>(fa, pt, w, sw4, lim, dup, tl, tab, sum, row);
+        if constexpr (SIM == SIM_NUCLEON)
+            octet_batch_nn<MEAS, COUL, TIMG, 4>(fa, pt, w, sw4, lim, tl, tab, sum);
+        else
+            octet_batch<SIM, MEAS, RANGE, TIMG, REACT, 4>(fa, pt, w, sw4, lim, dup, tl, tab, sum, row);
     }
     if (k < cnt) {
         const unsigned w = *reinterpret_cast<const unsigned short*>(&list[k + 2 * b]);
-        octet_batch<SIM, MEAS, RANGE, TIMG, REACT, 2>(fa, pt, w, sw2, lim, dup, tl, tab, sum, row);
+        if constexpr (SIM == SIM_NUCLEON)
+            octet_batch_nn<MEAS, COUL, TIMG, 2>(fa, pt, w, sw2, lim, tl, tab, sum);
+        else
+            octet_batch<SIM, MEAS, RANGE, TIMG, REACT, 2>(fa, pt, w, sw2, lim, dup, tl, tab, sum, row);
     }
 }
 
@@ -345,9 +461,11 @@ __device__ __forceinline__ void octet_eval(const ForceArgs& fa, double4 pt, int 
 // (x, y) then 128 (z, w), so that the 16 sources of a batch are read from
 // shared memory without bank conflicts (interleaved as double4 they took 8
 // cycles of the shared-memory pipe per pair instead of 4), and the bounding
-// boxes of the octets and tiles (centre, -, half-width with the rounding
-// margin, -).  Written by k_octet_pack.
+// boxes of the octets and tiles (centre, half-width with the rounding margin;
+// the centre's w says whether the box holds a proton).  Written by
+// k_octet_pack.
 struct OctetBox {
+    const double4* pos;                   // slot-ordered FP64 positions (mixed nucleon pairs next to |d| = L/2)
     const float4* posq;                   // tiles of OCT_UNITS 16-byte units
     const float4* obox;
     const float4* tbox;
@@ -393,9 +511,11 @@ k_octet_pack(const double4* __restrict__ pos, int n, ForceArgs fa, float4* __res
             }
         }
     }
+    const unsigned pm = __ballot_sync(0xffffffffu, on && p.w == 1.0);
+    const int protons = __syncthreads_or(pm != 0);
     if ((j & 7) == 0) {
         float4* o = obox + 2 * ((size_t)C * OCTETS + (j >> 3));
-        o[0] = make_float4(cc[0], cc[1], cc[2], 0.f);
+        o[0] = make_float4(cc[0], cc[1], cc[2], (pm >> lane & 0xffu) ? 1.f : 0.f);
         o[1] = make_float4(hh[0], hh[1], hh[2], 0.f);
     }
     if (lane == 0)
@@ -412,7 +532,8 @@ k_octet_pack(const double4* __restrict__ pos, int n, ForceArgs fa, float4* __res
             a[c] = fminf(fminf(red[0][c], red[1][c]), fminf(red[2][c], red[3][c]));
             b[c] = fmaxf(fmaxf(red[0][3 + c], red[1][3 + c]), fmaxf(red[2][3 + c], red[3][3 + c]));
         }
-        tbox[2 * C] = make_float4(0.5f * (a[0] + b[0]), 0.5f * (a[1] + b[1]), 0.5f * (a[2] + b[2]), 0.f);
+        tbox[2 * C] = make_float4(0.5f * (a[0] + b[0]), 0.5f * (a[1] + b[1]), 0.5f * (a[2] + b[2]),
+                                  protons ? 1.f : 0.f);
         tbox[2 * C + 1] = make_float4(fmaf(0.5f, b[0] - a[0], mu[0]), fmaf(0.5f, b[1] - a[1], mu[1]),
                                       fmaf(0.5f, b[2] - a[2], mu[2]), 0.f);
     }
@@ -436,14 +557,26 @@ __device__ __forceinline__ float box_dist2(const ForceArgs& fa, const float4& c1
     return dist2;
 }
 
+// Squared radius that counts between two boxes (their centres' words): ions the
+// cutoff, nucleons the nuclear range, or the Coulomb cutoff if both hold a
+// proton and it is larger.
+template <int SIM>
+__device__ __forceinline__ float octet_lim(const ForceArgs& fa, float p1, float p2)
+{
+    if constexpr (SIM != SIM_NUCLEON) return fa.scr_c2;
+    return (fa.coulomb_on && p1 != 0.f && p2 != 0.f) ? fmaxf(fa.scr_c2, fa.scr_n2) : fa.scr_n2;
+}
+
 // Whether an octet (box oc, oh) reaches a tile (box tc, th).  uni: seen from the
 // octet's centre every source of the tile has the image kc (packed code), and
 // that is the minimum image of every pair that counts: either no pair is as
 // far as L/2 on any axis, or none within the cutoff is (warp_box_of's
 // argument).
+template <int SIM>
 __device__ __forceinline__ bool octet_reach(const ForceArgs& fa, const float4& oc, const float4& oh, const float4& tc,
                                             const float4& th, bool& uni, int& kc)
 {
+    const float lim = octet_lim<SIM>(fa, oc.w, tc.w);
     const float MAGIC = 12582912.0f;
     const float td[3] = {tc.x - oc.x, tc.y - oc.y, tc.z - oc.z};
     const float thv[3] = {th.x, th.y, th.z}, ohv[3] = {oh.x, oh.y, oh.z};
@@ -460,10 +593,10 @@ __device__ __forceinline__ bool octet_reach(const ForceArgs& fa, const float4& o
         const float half = 0.5f * fa.Lf[c] - 1.0f;
         one = one && dm + thv[c] < half;
         const float s = half - ohv[c];
-        cut = cut && (dm + thv[c] + ohv[c] < half || (s > 0.f && s * s > fa.scr_c2));
+        cut = cut && (dm + thv[c] + ohv[c] < half || (s > 0.f && s * s > lim));
     }
     uni = one && cut;
-    return dist2 <= fa.scr_c2;
+    return dist2 <= lim;
 }
 
 // FP32 copies of the tile's coordinates (its unfilled slots are never listed).
@@ -519,21 +652,23 @@ struct Form64 {
 
     static __device__ __forceinline__ double weight(const Target& t) { return t.w; }
 
-    template <bool UNI>
+    template <bool UNI, bool NUC>
     static __device__ __forceinline__ int list(const ForceArgs& fa, const float (&oc)[3], const float (&oh)[3],
-                                               const float4* __restrict__, const Extra& x, int jlim, int jmin,
-                                               unsigned char* __restrict__ l, int& kcode)
+                                               float limp, float lim, const float4* __restrict__ tile, const Extra& x,
+                                               int jlim, int jmin, unsigned char* __restrict__ l, int& kcode)
     {
-        return octet_list<UNI>(fa, oc, oh, x.xs, jlim, jmin, l, kcode);
+        return octet_list<UNI, NUC>(fa, oc, oh, limp, lim, reinterpret_cast<const double2*>(tile), x.xs, jlim, jmin, l,
+                               kcode);
     }
 
-    template <int SIM, bool MEAS, bool RANGE, bool TIMG, bool REACT>
+    template <int SIM, bool MEAS, bool RANGE, bool TIMG, bool REACT, bool COUL>
     static __device__ __forceinline__ void eval(const ForceArgs& fa, const Target& t, int lim, int kcode, int cnt,
                                                 const float4* __restrict__ tile, const unsigned char* __restrict__ l,
-                                                double tab, OctetSum<MEAS>& sum, double* __restrict__ row)
+                                                double tab, OctetSum<MEAS>& sum, double* __restrict__ row,
+                                                const double4* __restrict__, const double4* __restrict__)
     {
-        octet_eval<SIM, MEAS, RANGE, TIMG, REACT>(fa, t, lim, kcode, cnt, reinterpret_cast<const double2*>(tile), l,
-                                                  tab, sum, row);
+        octet_eval<SIM, MEAS, RANGE, TIMG, REACT, COUL>(fa, t, lim, kcode, cnt, reinterpret_cast<const double2*>(tile),
+                                                        l, tab, sum, row);
     }
 };
 
@@ -553,10 +688,11 @@ struct OctetSmem {
 
 // The octet's list on a tile in the image that octet_reach found, if it did;
 // timg: every listed source has image kcode in every pair that counts.
-template <class F>
-__device__ __forceinline__ int octet_list_any(const ForceArgs& fa, bool uni, const float4 (&box)[2],
-                                              const float4* __restrict__ tile, const typename F::Extra& x, int jlim,
-                                              int jmin, unsigned char* __restrict__ list, int& kcode, bool& timg)
+template <class F, bool NUC>
+__device__ __forceinline__ int octet_list_any(const ForceArgs& fa, bool uni, const float4 (&box)[2], float limp,
+                                              float lim, const float4* __restrict__ tile,
+                                              const typename F::Extra& x, int jlim, int jmin,
+                                              unsigned char* __restrict__ list, int& kcode, bool& timg)
 {
     if (jlim <= jmin) return 0;
     float oc[3] = {box[0].x, box[0].y, box[0].z};
@@ -565,15 +701,15 @@ __device__ __forceinline__ int octet_list_any(const ForceArgs& fa, bool uni, con
     if (uni) {
 #pragma unroll
         for (int c = 0; c < 3; ++c) oc[c] = fmaf(img_of(kcode, c), fa.Lf[c], oc[c]);
-        return F::template list<true>(fa, oc, oh, tile, x, jlim, jmin, list, kcode);
+        return F::template list<true, NUC>(fa, oc, oh, limp, lim, tile, x, jlim, jmin, list, kcode);
     }
-    const int cnt = F::template list<false>(fa, oc, oh, tile, x, jlim, jmin, list, kcode);
+    const int cnt = F::template list<false, NUC>(fa, oc, oh, limp, lim, tile, x, jlim, jmin, list, kcode);
     // the listed sources' one image, where no pair inside r_c has another
     timg = kcode >= 0;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         const float e = 0.5f * fa.Lf[c] - oh[c] - 1.0f;
-        timg = timg && e > 0.f && e * e > fa.scr_c2;
+        timg = timg && e > 0.f && e * e > limp;
     }
     return cnt;
 }
@@ -601,12 +737,15 @@ __device__ __forceinline__ void octet_visit(const ForceArgs& fa, const float4* _
                                             const typename F::Extra& x, unsigned char* __restrict__ list, bool diag,
                                             int jmin, int jlim, bool uni, int kcode, double tab,
                                             double* __restrict__ acc, double (&S)[MEAS ? NSCAL : 1],
-                                            double* __restrict__ row, bool& used)
+                                            double* __restrict__ row, bool& used, float tile_p,
+                                            const double4* __restrict__ pos, int C)
 {
     const int lane = threadIdx.x & 31;
     const typename F::Target t = F::target(posq, R, s, R * PB + s < n);
     bool timg;
-    const int cnt = octet_list_any<F>(fa, uni, box, tile, x, jlim, jmin, list, kcode, timg);
+    const float limp = octet_lim<SIM>(fa, box[0].w, tile_p);
+    const float lim1 = SIM == SIM_NUCLEON ? fa.scr_n2 : limp;
+    const int cnt = octet_list_any<F, SIM == SIM_NUCLEON>(fa, uni, box, limp, lim1, tile, x, jlim, jmin, list, kcode, timg);
     if (cnt == 0) return;
     if (REACT && !used) {
         used = true;
@@ -616,8 +755,26 @@ __device__ __forceinline__ void octet_visit(const ForceArgs& fa, const float4* _
     }
     OctetSum<MEAS> sum;
     sum.zero();
-    if (timg && !diag) F::template eval<SIM, MEAS, RANGE, true, REACT>(fa, t, -1, kcode, cnt, tile, list, tab, sum, row);
-    else F::template eval<SIM, MEAS, RANGE, false, REACT>(fa, t, diag ? s : -1, kcode, cnt, tile, list, tab, sum, row);
+    const double4* pos_t = pos + (size_t)R * PB + s;
+    const double4* pos_s = pos + (size_t)C * PB;
+    const int lim = diag ? s : -1;
+    auto eval = [&](auto timg_c, auto coul_c) {
+        F::template eval<SIM, MEAS, RANGE, decltype(timg_c)::value, REACT, decltype(coul_c)::value>(
+            fa, t, lim, kcode, cnt, tile, list, tab, sum, row, pos_t, pos_s);
+    };
+    const bool ti = timg && !diag;
+    bool plain = true;
+    if constexpr (SIM == SIM_NUCLEON) {
+        if (fa.coulomb_on && box[0].w != 0.f && tile_p != 0.f) {
+            plain = false;
+            if (ti) eval(std::true_type{}, std::true_type{});
+            else eval(std::false_type{}, std::true_type{});
+        }
+    }
+    if (plain) {
+        if (ti) eval(std::true_type{}, std::false_type{});
+        else eval(std::false_type{}, std::false_type{});
+    }
     // the target sums over the four source lanes
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -676,7 +833,7 @@ __device__ __forceinline__ bool octets_job(OctetSmem<F>& sm, const ForceArgs& fa
             // lane o < 16: octet o against the tile's box
             bool uni;
             int kc;
-            const bool reach = octet_reach(fa, sm.box[lane & 15][0], sm.box[lane & 15][1], bx.tbox[2 * C],
+            const bool reach = octet_reach<SIM>(fa, sm.box[lane & 15][0], sm.box[lane & 15][1], bx.tbox[2 * C],
                                            bx.tbox[2 * C + 1], uni, kc) && lane < OCTETS;
             unsigned om = __ballot_sync(0xffffffffu, reach);
             const unsigned um = __ballot_sync(0xffffffffu, uni);
@@ -693,7 +850,7 @@ __device__ __forceinline__ bool octets_job(OctetSmem<F>& sm, const ForceArgs& fa
                 octet_visit<F, SIM, MEAS, RANGE, true>(fa, bx.posq, n, R, s, sm.box[o], sm.tile, sm.x, sm.list, diag,
                                                        max(diag ? 8 * o + 1 : 0, w0), jlim, ((um >> o) & 1u) != 0,
                                                        __shfl_sync(0xffffffffu, kc, o), tab, sm.acc + 3 * s, S, sm.row,
-                                                       used);
+                                                       used, bx.tbox[2 * C].w, bx.pos, C);
             }
             const long long u = tri_index(C, R);
             if (!used && w0 == 0 && w1 == PB) {
@@ -1092,7 +1249,8 @@ k_force_octets_all(OctetBox bx, int chunks, int len, double* __restrict__ part, 
             const float4 tc = bx.tbox[2 * (Cb + lane)], th = bx.tbox[2 * (Cb + lane) + 1];
 #pragma unroll
             for (int o = 0; o < 4; ++o)
-                on = on || box_dist2(fa, tc, th, sm.box[o][0], sm.box[o][1]) <= fa.scr_c2;
+                on = on || box_dist2(fa, tc, th, sm.box[o][0], sm.box[o][1]) <=
+                               octet_lim<SIM>(fa, tc.w, sm.box[o][0].w);
         }
         unsigned tiles = single ? 1u : __ballot_sync(0xffffffffu, on), ahead = tiles, asked = q;
 #pragma unroll
@@ -1108,7 +1266,7 @@ k_force_octets_all(OctetBox bx, int chunks, int len, double* __restrict__ part, 
             const int st = q & 1;
             bool uni;
             int kc;
-            const bool reach = octet_reach(fa, sm.box[lane & 3][0], sm.box[lane & 3][1], bx.tbox[2 * C],
+            const bool reach = octet_reach<SIM>(fa, sm.box[lane & 3][0], sm.box[lane & 3][1], bx.tbox[2 * C],
                                            bx.tbox[2 * C + 1], uni, kc) && lane < 4;
             unsigned om = __ballot_sync(0xffffffffu, reach);
             const unsigned um = __ballot_sync(0xffffffffu, uni);
@@ -1126,7 +1284,8 @@ k_force_octets_all(OctetBox bx, int chunks, int len, double* __restrict__ part, 
                 octet_visit<F, SIM, MEAS, RANGE, false>(fa, bx.posq, n, R, 32 * (g % (PB / 32)) + 8 * o + a, sm.box[o],
                                                         sm.tile[st], sm.x, sm.list, diag, jmin, jlim,
                                                         ((um >> o) & 1u) != 0, __shfl_sync(0xffffffffu, kc, o), tab,
-                                                        sm.acc + 3 * (8 * o + a), S, nullptr, used);
+                                                        sm.acc + 3 * (8 * o + a), S, nullptr, used, bx.tbox[2 * C].w,
+                                                        bx.pos, C);
             }
             if (ahead) {
                 if (lane == 0) issue(Cb + __ffs(ahead) - 1, asked);

@@ -1,4 +1,5 @@
-// yk_octets32.cuh -- the octet kernels' mixed form (Form32, ions with fa.lo).
+// yk_octets32.cuh -- the octet kernels' mixed form (Form32: ions with fa.lo,
+// nucleons with fa.hilo).
 //
 // The arithmetic of a pair is that of disp_tile_x2 / screen_d_x2 and
 // ion_terms_x2: exact FP32 differences of grid-rounded coordinates plus a
@@ -158,6 +159,131 @@ __device__ __forceinline__ void octet_batch32(const ForceArgs& fa, const Target3
     }
 }
 
+// octet_batch32 for nucleons (fa.hilo; pair_group_nn_lo's arithmetic).  With
+// per-pair images a pair whose hi-part displacement is hLmin or more on an
+// axis takes the reference's conditional image of the FP64 positions (pt the
+// target's, ps the tile's), unless no term reaches that far (no Coulomb term
+// and fa.nn_short).  The terms inside rncut are taken only where a lane of
+// the warp has such a pair, and, with COUL, the p-p Coulomb terms of proton
+// pairs inside rccut.  Every pair from both sides: no reactions.
+template <bool MEAS, bool COUL, bool TIMG, int NQ>
+__device__ __forceinline__ void octet_batch32_nn(const ForceArgs& fa, const Target32& t, unsigned w, int sw, int lim,
+                                                 const float4* __restrict__ tile, OctetSum<MEAS>& sum,
+                                                 Sum32<MEAS>& ms,
+                                                 const double4* __restrict__ pt, const double4* __restrict__ ps)
+{
+    constexpr int SEC = PB / 2 + OCT_GAP;
+    const float rn2 = fminf(fa.rn2f, 1e35f);              // (pads and empty slots are at 1e36 or more)
+    float2 d[NQ][3], r2[NQ], wj[NQ], f[3];
+    unsigned ok = ~0u, fl = 0;                            // bits 2q, 2q + 1: the two pairs of entry q
+    f[0] = f[1] = f[2] = oct_dup(0.f);
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        const int p = (int)__byte_perm(w, 0, 0x4440u | (unsigned)(q ^ sw));
+        const float4 A = tile[p], B = tile[p + SEC], Cc = tile[p + 2 * SEC];
+        const float2 Dz = *reinterpret_cast<const float2*>(&tile[p + 3 * SEC]);
+        const float2 xh[3] = {make_float2(A.x, A.y), make_float2(A.z, A.w), make_float2(B.x, B.y)};
+        const float2 xl[3] = {make_float2(Cc.x, Cc.y), make_float2(Cc.z, Cc.w), Dz};
+        wj[q] = make_float2(B.z, B.w);
+        if constexpr (!TIMG) {
+            if (2 * p == lim) ok &= ~(1u << (2 * q));
+            if (2 * p + 1 == lim) ok &= ~(2u << (2 * q));
+        }
+        float2 mx = oct_dup(0.f);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const float2 dh = __fadd2_rn(xh[c], oct_dup(t.h[c]));             // exact
+            float2 dl = __fadd2_rn(xl[c], oct_dup(t.l[c]));
+            if constexpr (TIMG) {
+                d[q][c] = __fadd2_rn(dh, dl);
+            } else {
+                const float2 MAG = oct_dup(12582912.0f), NMAG = oct_dup(-12582912.0f);
+                const float2 k = __fadd2_rn(__ffma2_rn(dh, oct_dup(fa.invLf[c]), MAG), NMAG);
+                const float2 d1 = __ffma2_rn(oct_dup(-fa.Lh[c]), k, dh);      // exact
+                mx = make_float2(fmaxf(mx.x, fabsf(d1.x)), fmaxf(mx.y, fabsf(d1.y)));
+                dl = __ffma2_rn(oct_dup(-fa.Ll[c]), k, dl);
+                d[q][c] = __fadd2_rn(d1, dl);
+            }
+        }
+        if constexpr (!TIMG) {
+            if (mx.x >= fa.hLmin) fl |= 1u << (2 * q);
+            if (mx.y >= fa.hLmin) fl |= 2u << (2 * q);
+        }
+    }
+    if constexpr (!TIMG) {
+        if ((COUL || !fa.nn_short) && __any_sync(0xffffffffu, (fl & ok) != 0)) {
+            // d = x_j - x_i from the reference's d = x_i - x_j and its image; a
+            // pad, an empty slot or an empty target (|d| far on x) has no FP64
+            // position
+#pragma unroll
+            for (int q = 0; q < NQ; ++q) {
+                const int p = (int)__byte_perm(w, 0, 0x4440u | (unsigned)(q ^ sw));
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    if (((fl & ok) >> (2 * q + h) & 1u) && fabsf(h ? d[q][0].y : d[q][0].x) < 1e17f) {
+                        const double4 pi = *pt, pj = ps[2 * p + h];
+                        const float ex = -__double2float_rn(min_image(__dsub_rn(pi.x, pj.x), fa.xl[0], fa.hlb[0]));
+                        const float ey = -__double2float_rn(min_image(__dsub_rn(pi.y, pj.y), fa.xl[1], fa.hlb[1]));
+                        const float ez = -__double2float_rn(min_image(__dsub_rn(pi.z, pj.z), fa.xl[2], fa.hlb[2]));
+                        if (h) d[q][0].y = ex, d[q][1].y = ey, d[q][2].y = ez;
+                        else d[q][0].x = ex, d[q][1].x = ey, d[q][2].x = ez;
+                    }
+                }
+            }
+        }
+    }
+    unsigned mn = 0;
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        r2[q] = __fmul2_rn(d[q][2], d[q][2]);
+        r2[q] = __ffma2_rn(d[q][1], d[q][1], r2[q]);
+        r2[q] = __ffma2_rn(d[q][0], d[q][0], r2[q]);
+        if (r2[q].x <= rn2) mn |= 1u << (2 * q);
+        if (r2[q].y <= rn2) mn |= 2u << (2 * q);
+    }
+    mn = fa.nuclear_on ? mn & ok : 0u;
+    const bool any = __any_sync(0xffffffffu, mn != 0);
+    if (!COUL && !any) return;
+    float2 fs[NQ], u[NQ], wv[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) fs[q] = u[q] = wv[q] = oct_dup(0.f);
+    if constexpr (COUL) {
+        const bool ip = t.w == 1.f;
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            const bool cx = ip && wj[q].x == 1.f && r2[q].x <= fa.rc2f && (TIMG || (ok >> (2 * q) & 1u));
+            const bool cy = ip && wj[q].y == 1.f && r2[q].y <= fa.rc2f && (TIMG || (ok >> (2 * q + 1) & 1u));
+            coulomb_terms_x2<MEAS>(fa, r2[q], make_float2(cx ? 1.f : 0.f, cy ? 1.f : 0.f), fs[q], u[q], wv[q]);
+        }
+    }
+    if (any) {
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) {
+            const float2 Bc = make_float2(wj[q].x == t.w ? fa.bpcf : fa.bmcf, wj[q].y == t.w ? fa.bpcf : fa.bmcf);
+            nuclear_terms_x2<MEAS>(fa, r2[q], make_float2(mn >> (2 * q) & 1u ? 1.f : 0.f,
+                                                          mn >> (2 * q + 1) & 1u ? 1.f : 0.f), Bc, fs[q], u[q], wv[q]);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+        if constexpr (MEAS) {
+            ms.s[0] = __fadd2_rn(ms.s[0], u[q]);
+            ms.s[1] = __fadd2_rn(ms.s[1], wv[q]);
+            const int P[6] = {0, 0, 0, 1, 1, 2}, Q[6] = {0, 1, 2, 1, 2, 2};
+            float2 gd[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) gd[c] = __fmul2_rn(fs[q], d[q][c]);
+#pragma unroll
+            for (int k = 0; k < 6; ++k) ms.s[2 + k] = __ffma2_rn(d[q][P[k]], gd[Q[k]], ms.s[2 + k]);
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) f[c] = __ffma2_rn(fs[q], d[q][c], f[c]);
+    }
+    // d = x_j - x_i: the target's terms carry a minus sign (int_nn.f:230-240)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) sum.f[c] -= (double)(f[c].x + f[c].y);
+}
+
 struct Form32 {
     static constexpr int PREC = PREC_MIXED, SECTIONS = 4, SEC = PB / 2, ROW = (PB + 2) * 3;
     struct Extra {};
@@ -213,10 +339,10 @@ struct Form32 {
     static __device__ __forceinline__ double weight(const Target& t) { return (double)t.w; }
 
     // lane l tests pairs l and l + 32, both sources at once
-    template <bool UNI>
+    template <bool UNI, bool NUC>
     static __device__ __forceinline__ int list(const ForceArgs& fa, const float (&oc)[3], const float (&oh)[3],
-                                               const float4* __restrict__ tile, const Extra&, int jlim, int jmin,
-                                               unsigned char* __restrict__ l, int& kcode)
+                                               float limp, float lim, const float4* __restrict__ tile, const Extra&,
+                                               int jlim, int jmin, unsigned char* __restrict__ l, int& kcode)
     {
         const int lane = threadIdx.x & 31;
         const unsigned below = (1u << lane) - 1u;
@@ -252,8 +378,14 @@ struct Form32 {
                 d2 = __ffma2_rn(m, m, d2);
             }
             const unsigned span = (unsigned)(jlim - jmin);
-            const bool n0 = (unsigned)(2 * p - jmin) < span && d2.x <= fa.scr_c2;
-            const bool n1 = (unsigned)(2 * p + 1 - jmin) < span && d2.y <= fa.scr_c2;
+            bool n0 = d2.x <= lim, n1 = d2.y <= lim;
+            if constexpr (NUC) {
+                const float2 wj = reinterpret_cast<const float2*>(&tile[p + SMEM_SEC])[1];
+                n0 = n0 || (d2.x <= limp && wj.x == 1.f);
+                n1 = n1 || (d2.y <= limp && wj.y == 1.f);
+            }
+            n0 = n0 && (unsigned)(2 * p - jmin) < span;
+            n1 = n1 && (unsigned)(2 * p + 1 - jmin) < span;
             if constexpr (!UNI) {
                 if (n0) {
                     c_and &= c0;
@@ -278,10 +410,11 @@ struct Form32 {
         return cnt;
     }
 
-    template <int SIM, bool MEAS, bool RANGE, bool TIMG, bool REACT>
+    template <int SIM, bool MEAS, bool RANGE, bool TIMG, bool REACT, bool COUL>
     static __device__ __forceinline__ void eval(const ForceArgs& fa, Target t, int lim, int kcode, int cnt,
                                                 const float4* __restrict__ tile, const unsigned char* __restrict__ l,
-                                                double, OctetSum<MEAS>& sum, double* __restrict__ row)
+                                                double, OctetSum<MEAS>& sum, double* __restrict__ row,
+                                                const double4* __restrict__ pt, const double4* __restrict__ ps)
     {
         const int lane = threadIdx.x & 31, a = lane & 7, b = lane >> 3;
         const int sw4 = 2 * ((a >> 2) & 1) + ((a >> 1) & 1), sw2 = (a >> 2) & 1;
@@ -300,11 +433,17 @@ struct Form32 {
 #pragma unroll 1
         for (; cnt - k > 8; k += 16) {
             const unsigned w = *reinterpret_cast<const unsigned*>(&l[k + 4 * b]);
-            octet_batch32<SIM, MEAS, TIMG, REACT, 4>(fa, t, w, sw4, lim, tile, sum, ms, row);
+            if constexpr (SIM == SIM_NUCLEON)
+                octet_batch32_nn<MEAS, COUL, TIMG, 4>(fa, t, w, sw4, lim, tile, sum, ms, pt, ps);
+            else
+                octet_batch32<SIM, MEAS, TIMG, REACT, 4>(fa, t, w, sw4, lim, tile, sum, ms, row);
         }
         if (k < cnt) {
             const unsigned w = *reinterpret_cast<const unsigned short*>(&l[k + 2 * b]);
-            octet_batch32<SIM, MEAS, TIMG, REACT, 2>(fa, t, w, sw2, lim, tile, sum, ms, row);
+            if constexpr (SIM == SIM_NUCLEON)
+                octet_batch32_nn<MEAS, COUL, TIMG, 2>(fa, t, w, sw2, lim, tile, sum, ms, pt, ps);
+            else
+                octet_batch32<SIM, MEAS, TIMG, REACT, 2>(fa, t, w, sw2, lim, tile, sum, ms, row);
         }
         if constexpr (MEAS) {
 #pragma unroll
