@@ -213,27 +213,56 @@ k_b_post(const int2* __restrict__ vb, const RepDesc* __restrict__ rd, const int*
     if constexpr (KIN) block_sum_store<NKIN>(tk, red, kpart + (size_t)blockIdx.x * NKIN);
 }
 
-// The persistent force kernel over the work items of jobs[0 .. *njobs); the
-// items of boxes whose step budget is spent are passed over.
+// Whether a box takes the mixed hi/lo displacement (LO below): its own
+// property, so its results do not depend on the other boxes.
+__host__ __device__ inline bool box_lo(int sim, int prec, const ForceArgs& fa)
+{
+    return prec == PREC_MIXED && (sim == SIM_NUCLEON ? fa.hilo : fa.lo) != 0;
+}
+
+// Bounding box of every tile on the FP32 shadow hi parts, for the boxes whose
+// kernel looks at them (k_tile_boxes): one CTA per tile.
+__global__ void __launch_bounds__(PB)
+k_b_tile_boxes(const int* __restrict__ tile_rep, const RepDesc* __restrict__ rd, const int* __restrict__ left,
+               const float* __restrict__ posf, float* __restrict__ tbox)
+{
+    const int r = tile_rep[blockIdx.x];
+    if (r < 0 || left[r] <= 0) return;
+    const RepDesc* d = rd + r;
+    if (!d->fa.lo) return;
+    const int T0 = d->S / PB;
+    tile_box(posf + (size_t)blockIdx.x * SHADOW_FLOATS, ((int)blockIdx.x - T0) * PB, d->fa.n, d->fa.Lf,
+             tbox + 8 * (size_t)blockIdx.x);
+}
+
+// The persistent force kernels over the batch's work items: the boxes that take
+// the mixed hi/lo displacement (LO: items 0 .. nj[0]) and the others (nj[0] ..
+// nj[1]) have a kernel each, so that a box which cannot (r_c close to half an
+// edge) does not put the others on the general form; both are launched whatever
+// the batch holds, so a captured graph stays valid when boxes come and go.
+// The items of boxes whose step budget is spent are passed over.
 template <int SIM, int PREC, bool MEAS, bool LO = false>
 // (6 CTAs per SM for the mixed hi/lo form: at 7, the box descriptors spill)
 __global__ void __launch_bounds__(PB, (pairs_ctas_per_sm<SIM_MIX, PREC, LO>()))
 k_force_pairs_batch(const double4* __restrict__ pos, const float* __restrict__ posf,
-                    const int4* __restrict__ jobs, const int* __restrict__ njobs_p, int* __restrict__ counter,
-                    const RepDesc* __restrict__ rd, const int* __restrict__ left, double* __restrict__ Si,
-                    row_t<PREC>* __restrict__ Sj, double* __restrict__ Sm, unsigned* __restrict__ err)
+                    const int4* __restrict__ jobs, const int* __restrict__ nj, int* __restrict__ counter,
+                    const RepDesc* __restrict__ rd, const int* __restrict__ left, const float* __restrict__ tbox,
+                    unsigned char* __restrict__ Sjf, double* __restrict__ Si, row_t<PREC>* __restrict__ Sj,
+                    double* __restrict__ Sm, unsigned* __restrict__ err)
 {
     __shared__ __align__(128) PairSmem<row_t<PREC>> sm;
     __shared__ __align__(16) ForceArgs sfa;
     __shared__ int4 sjob;
+    constexpr bool TB = pairs_tile_boxes<SIM, PREC, LO>();
+    const int first = LO ? 0 : nj[0], njobs = LO ? nj[0] : nj[1];
+    if (first >= njobs) return;
     pairs_smem_init(sm);
-    const int njobs = *njobs_p;
     unsigned q = 0;
     for (;;) {
         if (threadIdx.x == 0) {
             int4 jb;
             do {
-                const int j = atomicAdd(counter, 1);
+                const int j = first + atomicAdd(counter, 1);
                 jb = j < njobs ? jobs[j] : make_int4(-1, 0, 0, 0);
             } while (jb.x >= 0 && left[jb.x] <= 0);
             sjob = jb;
@@ -250,54 +279,72 @@ k_force_pairs_batch(const double4* __restrict__ pos, const float* __restrict__ p
         bx.posf = posf + (size_t)(d->S / SHADOW_TILE) * SHADOW_FLOATS;
         bx.Si = Si + d->Si_off;
         bx.Sj = Sj + d->Sj_off;
-        bx.tbox = nullptr;
-        bx.Sjf = nullptr;
+        bx.tbox = TB ? tbox + 8 * (size_t)(d->S / PB) : nullptr;
+        bx.Sjf = Sjf + d->Sj_off / (PB * 3);
         bx.n = sfa.n;
         bx.M = d->T;
         bx.nseg_max = d->nseg;
         const int C0 = jb.y + jb.z * d->seg;
-        if (!pairs_job<SIM, PREC, MEAS, LO ? 1 : 2>(sm, sfa, bx, jb.y, C0, min(C0 + d->seg, bx.M), jb.z,
-                                                    Sm + (size_t)(d->sm_off + jb.w) * NSCAL, err, q))
+        if (!pairs_job<SIM, PREC, MEAS, LO ? 1 : 0, false, TB>(sm, sfa, bx, jb.y, C0, min(C0 + d->seg, bx.M),
+                                                              jb.z, Sm + (size_t)(d->sm_off + jb.w) * NSCAL, err, q))
             return;
     }
 }
 
 // Per slot of the boxes in sel (all if NULL) whose budget is not spent: the
 // fixed-order sum of its partials, the reference's scaling, and the store to
-// the caller's order (as k_combine).  tile_rep: box of every tile, -1 unused.
+// the caller's order: one CTA per tile, as k_combine (the thread groups'
+// shares, and only the source-side rows that were written: Sjf).  tile_rep: box
+// of every tile, -1 unused.
 template <int SIM, int PREC>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(COMB_THREADS)
 k_b_combine(const int* __restrict__ tile_rep, const RepDesc* __restrict__ rd, const int* __restrict__ sel,
             const int* __restrict__ left, const double* __restrict__ Si, const row_t<PREC>* __restrict__ Sj,
-            const int* __restrict__ perm, const double* __restrict__ zii, const double* __restrict__ aii,
-            double* __restrict__ a, int total_slots)
+            const unsigned char* __restrict__ Sjf, const int* __restrict__ perm, const double* __restrict__ zii,
+            const double* __restrict__ aii, double* __restrict__ a)
 {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= total_slots) return;
-    const int r = tile_rep[p >> 7];
+    __shared__ double part[COMB_GROUPS][PB * 3];
+    const int r = tile_rep[blockIdx.x];
     if (r < 0 || (sel && !sel[r]) || left[r] <= 0) return;
     const RepDesc* d = rd + r;
-    const int pl = p - d->S;
-    if (pl >= d->fa.n) return;
-    const int R = pl / PB, l = pl % PB;
+    const int R = (int)blockIdx.x - d->S / PB;
+    const int g = threadIdx.x / (PB * 3), t = threadIdx.x % (PB * 3), lane = threadIdx.x & 31;
+    constexpr size_t ROW = (size_t)PB * 3;
     const int nseg = (d->T - R + d->seg - 1) / d->seg;
-    double F[3] = {0.0, 0.0, 0.0};
-    const double* si = Si + d->Si_off + ((size_t)R * d->nseg * PB + l) * 3;
-    for (int s = 0; s < nseg; ++s) {
-        const double* e = si + (size_t)s * PB * 3;
-        F[0] += e[0];
-        F[1] += e[1];
-        F[2] += e[2];
+    double F = 0.0;
+    const double* si = Si + d->Si_off + (size_t)R * d->nseg * ROW + t;
+#pragma unroll 4
+    for (int s = g; s < nseg; s += COMB_GROUPS) F += si[(size_t)s * ROW];
+    const row_t<PREC>* sj = Sj + d->Sj_off + (size_t)tri_index(R, 0) * ROW + t;
+    const unsigned char* fl = Sjf + d->Sj_off / (PB * 3) + tri_index(R, 0);
+    // the written rows, 32 units at a time (the warps of a group agree)
+    for (int b = g; b <= R; b += 32 * COMB_GROUPS) {
+        const int R2 = b + COMB_GROUPS * lane;
+        unsigned m = __ballot_sync(0xffffffffu, R2 <= R && fl[min(R2, R)] != 0);
+        while (m) {
+            double v[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                v[k] = m ? (double)sj[(size_t)(b + COMB_GROUPS * (__ffs(m) - 1)) * ROW] : 0.0;
+                m &= m - 1;
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) F += v[k];
+        }
     }
-    const row_t<PREC>* sj = Sj + d->Sj_off + ((size_t)tri_index(R, 0) * PB + l) * 3;
-    for (int R2 = 0; R2 <= R; ++R2) {
-        const row_t<PREC>* e = sj + (size_t)R2 * PB * 3;
-        F[0] += e[0];
-        F[1] += e[1];
-        F[2] += e[2];
+    part[g][t] = F;
+    __syncthreads();
+    const int l = threadIdx.x;
+    if (l >= PB || R * PB + l >= d->fa.n) return;
+    double Fv[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        Fv[c] = part[0][3 * l + c];
+#pragma unroll
+        for (int q = 1; q < COMB_GROUPS; ++q) Fv[c] += part[q][3 * l + c];
     }
-    const int orig = perm[p];
-    store_accel<SIM>(d->fa, orig - d->P, zii[orig], aii + d->P, F, a + d->A);
+    const int orig = perm[blockIdx.x * PB + l];
+    store_accel<SIM>(d->fa, orig - d->P, zii[orig], aii + d->P, Fv, a + d->A);
 }
 
 // One block per slot.  kin_mode / meas as in k_finish; the series entry of
@@ -389,7 +436,7 @@ struct yk_batch {
     int dev = 0;
     int sim = 0, prec = 0;          // SIM_MIX or SIM_NUCLEON; PREC_*
     int prec_api = 0;
-    cudaStream_t stream = nullptr;
+    cudaStream_t stream = nullptr, stream2 = nullptr;
     std::vector<char> held;
     std::vector<int> n;
     std::vector<double> time, dt;
@@ -411,7 +458,9 @@ struct yk_batch {
     int* sel = nullptr;             // boxes being admitted
     int4* jobs = nullptr;           // work items of all held boxes
     int4* jobs_sel = nullptr;       // ... of the boxes being admitted
-    int* njobs_dev = nullptr;       // [0] all, [1] admitted
+    int* njobs_dev = nullptr;       // ends of the hi/lo boxes' items and of all items; the same of the admitted boxes'
+    float* tbox = nullptr;          // tile boxes (hi/lo ion boxes)
+    unsigned char* Sjf = nullptr;   // per half-pair unit: its Sj row was written
     int njobs = 0, njobs_sel = 0;
     int* counter = nullptr;
     int* tile_rep = nullptr;
@@ -424,13 +473,13 @@ struct yk_batch {
     int series_cap = 0;
     int* series_idx = nullptr;
     int force_grid = 0, force_grid_lo = 0;
-    bool all_lo = false;            // every held box allows the mixed hi/lo displacement (fa.lo / fa.hilo)
     int seg = BATCH_SEG, graph_steps = BATCH_GRAPH_STEPS;
     int sort_every = BATCH_SORT_EVERY;
     int since_sort = 0;             // steps run since the last re-ordering (eager steps)
     std::vector<RepDesc> hrd;       // host copy of the descriptors
     bool pos_dirty = false;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;   // of the force kernels' second stream
     std::vector<GraphB> graphs;
     unsigned long long graph_clock = 0;
     std::string errmsg;
@@ -491,26 +540,33 @@ static int launch_force_b(yk_batch* b, bool sel_new)
         b->force_grid_lo = std::max(1, per_sm_lo) * std::max(1, sms);
     }
     const int4* jobs = sel_new ? b->jobs_sel : b->jobs;
-    const int* njp = b->njobs_dev + (sel_new ? 1 : 0);
-    cudaMemsetAsync(b->counter, 0, sizeof(int), b->stream);
-    bool launched = false;
+    const int* nj = b->njobs_dev + (sel_new ? 2 : 0);
+    row_t<PREC>* Sj = static_cast<row_t<PREC>*>(b->Sj);
+    int k = 2;
+    cudaMemsetAsync(b->counter, 0, 2 * sizeof(int), b->stream);
+    // the two kernels side by side: the second's CTAs come in as the first's
+    // run out of items
     if constexpr (PREC == PREC_MIXED) {
-        if (b->all_lo) {
-            k_force_pairs_batch<SIM, PREC, MEAS, true><<<b->force_grid_lo, PB, 0, b->stream>>>(
-                b->pos, b->posf, jobs, njp, b->counter, b->rd, b->left, b->Si, static_cast<row_t<PREC>*>(b->Sj),
-                b->Sm, b->err);
-            launched = true;
-        }
+        cudaEventRecord(b->fork, b->stream);
+        cudaStreamWaitEvent(b->stream2, b->fork, 0);
     }
-    if (!launched)
-        k_force_pairs_batch<SIM, PREC, MEAS><<<b->force_grid, PB, 0, b->stream>>>(
-            b->pos, b->posf, jobs, njp, b->counter, b->rd, b->left, b->Si, static_cast<row_t<PREC>*>(b->Sj),
-            b->Sm, b->err);
-    k_b_combine<SIM, PREC><<<(b->tcap * PB + 255) / 256, 256, 0, b->stream>>>(b->tile_rep, b->rd, sel_new ? b->sel : nullptr,
-                                                                 b->left, b->Si, static_cast<row_t<PREC>*>(b->Sj),
-                                                                 b->perm, b->zii, b->aii,
-                                                                 b->a, b->tcap * PB);
-    return 2;
+    k_force_pairs_batch<SIM, PREC, MEAS><<<b->force_grid, PB, 0, b->stream>>>(
+        b->pos, b->posf, jobs, nj, b->counter, b->rd, b->left, b->tbox, b->Sjf, b->Si, Sj, b->Sm, b->err);
+    if constexpr (PREC == PREC_MIXED) {
+        if (pairs_tile_boxes<SIM, PREC, true>()) {
+            k_b_tile_boxes<<<b->tcap, PB, 0, b->stream2>>>(b->tile_rep, b->rd, b->left, b->posf, b->tbox);
+            ++k;
+        }
+        k_force_pairs_batch<SIM, PREC, MEAS, true><<<b->force_grid_lo, PB, 0, b->stream2>>>(
+            b->pos, b->posf, jobs, nj, b->counter + 1, b->rd, b->left, b->tbox, b->Sjf, b->Si, Sj, b->Sm, b->err);
+        ++k;
+        cudaEventRecord(b->join, b->stream2);
+        cudaStreamWaitEvent(b->stream, b->join, 0);
+    }
+    k_b_combine<SIM, PREC><<<b->tcap, COMB_THREADS, 0, b->stream>>>(b->tile_rep, b->rd, sel_new ? b->sel : nullptr,
+                                                                    b->left, b->Si, Sj, b->Sjf, b->perm, b->zii,
+                                                                    b->aii, b->a);
+    return k;
 }
 
 template <int SIM>
@@ -639,23 +695,44 @@ static void box_jobs(int r, int T, int seg, std::vector<int4>& jobs, std::vector
         }
 }
 
-static void costliest_first(std::vector<int4>& jobs, const std::vector<int>& cost)
+// Orders the items: those of hi/lo boxes first (k_force_pairs_batch), each
+// part the costliest first.  Returns the number of the former.
+static int order_jobs(const std::vector<char>& lo, std::vector<int4>& jobs, const std::vector<int>& cost)
 {
     std::vector<int> order(jobs.size());
     for (size_t k = 0; k < order.size(); ++k) order[k] = (int)k;
-    std::stable_sort(order.begin(), order.end(), [&](int u, int w) { return cost[u] > cost[w]; });
+    std::stable_sort(order.begin(), order.end(), [&](int u, int w) {
+        const bool lu = lo[jobs[u].x] != 0, lw = lo[jobs[w].x] != 0;
+        return lu != lw ? lu : cost[u] > cost[w];
+    });
+    const int nlo = (int)std::count_if(jobs.begin(), jobs.end(), [&](const int4& j) { return lo[j.x] != 0; });
     std::vector<int4> out(jobs.size());
     for (size_t k = 0; k < order.size(); ++k) out[k] = jobs[order[k]];
     jobs.swap(out);
+    return nlo;
 }
 
 static long long units_of(int T) { return (long long)T * (T + 1) / 2; }
 static long long nseg_of(int T, int seg) { return (T + seg - 1) / seg; }
 
+// Source tiles per work item of a box of T tiles: at most seg, and at least
+// BOX_SEGS items for the longest row of a small box, whose few long items
+// would otherwise keep a step waiting.  The box's own property: its sums do not
+// depend on the other boxes.  Mixed, 50 steps, with 8 tiles for every box / 16
+// items / 32 items: 6 boxes of 500 to 2,000 ions 20.1 / 5.5 / 5.3 ms, 24 boxes of
+// 1,000 to 20,000 62.1 / 51.0 / 52.8.
+constexpr int BOX_SEGS = 16;
+
+static int box_seg(int T, int seg) { return std::max(1, std::min(seg, (T + BOX_SEGS - 1) / BOX_SEGS)); }
+
 // Si rows and jobs that boxes of at most `units` half-pair units on at most
-// `tiles` tiles can need with segments of `seg` tiles: a box of T tiles takes
-// T ceil(T / seg) <= T^2 / seg + T <= 2 units / seg + T of each.
-static long long jobs_bound(long long units, long long tiles, int seg) { return 2 * units / seg + 2 * tiles; }
+// `tiles` tiles can need with segments of up to `seg` tiles: a box of T tiles
+// takes T ceil(T / box_seg) of each at most: T ceil(T / seg) <= T^2 / seg + T <=
+// 2 units / seg + T, or T BOX_SEGS.
+static long long jobs_bound(long long units, long long tiles, int seg)
+{
+    return 2 * units / seg + (BOX_SEGS + 2) * tiles;
+}
 
 // Si, Sm and the job tables sized for segment length seg.
 static int alloc_job_scratch(yk_batch* b, int seg)
@@ -693,7 +770,7 @@ static int relayout(yk_batch* b, int seg, const std::vector<char>& newsel)
     std::vector<int2> vblocks;
     std::vector<int> tile_rep(b->tcap, -1), seg_b(b->nslots, 0), seg_e(b->nslots, 0), segn_b(b->nslots, 0),
         segn_e(b->nslots, 0), selv(b->nslots, 0);
-    bool all_lo = true;
+    std::vector<char> lo(b->nslots, 0);
     int held = 0;
     for (int r = 0; r < b->nslots; ++r) {
         RepDesc& d = b->hrd[r];
@@ -703,13 +780,13 @@ static int relayout(yk_batch* b, int seg, const std::vector<char>& newsel)
         }
         ++held;
         d.active = 1;
-        d.seg = seg;
-        d.nseg = (int)nseg_of(d.T, seg);
+        d.seg = box_seg(d.T, seg);
+        d.nseg = (int)nseg_of(d.T, d.seg);
         d.Sj_off = sj;
         d.Si_off = si;
         d.sm_off = smo;
         const size_t j0 = jobs.size();
-        box_jobs(r, d.T, seg, jobs, cost);
+        box_jobs(r, d.T, d.seg, jobs, cost);
         d.njobs = (int)(jobs.size() - j0);
         if (!newsel.empty() && newsel[r]) {
             for (size_t k = j0; k < jobs.size(); ++k) {
@@ -730,20 +807,18 @@ static int relayout(yk_batch* b, int seg, const std::vector<char>& newsel)
         for (int t = 0; t < d.T; ++t) tile_rep[d.S / PB + t] = r;
         seg_b[r] = d.P;
         seg_e[r] = d.P + d.fa.n;
-        all_lo = all_lo && (b->sim == SIM_NUCLEON ? d.fa.hilo : d.fa.lo) != 0;
+        lo[r] = box_lo(b->sim, b->prec, d.fa);
     }
     if (sj > b->sj_cap || si > b->si_cap || (long long)smo * NSCAL > b->sm_cap ||
         (long long)jobs.size() > b->jobs_cap || (int)vblocks.size() > b->vb_cap)
         return bfail(b, YK_ERR_NOMEM, "the boxes need more half-pair scratch than the batch holds");
-    costliest_first(jobs, cost);
-    costliest_first(jobs_sel, cost_sel);
+    const int nlo = order_jobs(lo, jobs, cost), nlo_sel = order_jobs(lo, jobs_sel, cost_sel);
     vblocks.resize(b->vb_cap, make_int2(-1, 0));
     b->njobs = (int)jobs.size();
     b->njobs_sel = (int)jobs_sel.size();
     b->seg = seg;
     b->nrep = held;
-    b->all_lo = held > 0 && all_lo;
-    const int nj[2] = {b->njobs, b->njobs_sel};
+    const int nj[4] = {nlo, b->njobs, nlo_sel, b->njobs_sel};
     cudaStream_t st = b->stream;
     BCK(b, cudaMemcpyAsync(b->rd, b->hrd.data(), sizeof(RepDesc) * b->nslots, cudaMemcpyHostToDevice, st));
     if (!jobs.empty())
@@ -980,7 +1055,7 @@ int yk_batch_destroy(yk_batch* b)
                     b->pos,     b->posf,   b->perm,    b->iperm,    b->keys0,   b->keys1,   b->idx0,
                     b->idx1,    b->seg_b,  b->seg_e,   b->segn_b,   b->segn_e,  b->cub_tmp, b->rd,
                     b->left,    b->sel,    b->jobs,    b->jobs_sel, b->njobs_dev, b->counter, b->tile_rep,
-                    b->vblocks, b->Si,     b->Sj,      b->Sm,       b->kpart,   b->ds,      b->err,
+                    b->tbox,    b->Sjf,    b->vblocks, b->Si,     b->Sj,      b->Sm,       b->kpart,   b->ds,      b->err,
                     b->series,  b->series_idx};
     if (b->stream) {
         for (void* p : bufs)
@@ -989,6 +1064,9 @@ int yk_batch_destroy(yk_batch* b)
     }
     if (b->e0) cudaEventDestroy(b->e0);
     if (b->e1) cudaEventDestroy(b->e1);
+    if (b->fork) cudaEventDestroy(b->fork);
+    if (b->join) cudaEventDestroy(b->join);
+    if (b->stream2) cudaStreamDestroy(b->stream2);
     if (b->stream) cudaStreamDestroy(b->stream);
     delete b;
     return YK_OK;
@@ -1036,7 +1114,7 @@ static int create_empty(int sim, int prec_api, int nslots, long long max_units, 
     const size_t need = sj_elem * (size_t)b->sj_cap + sizeof(double) * (size_t)(14 * U + jb * PB * 3 + NSCAL * jb +
                                                   (long long)NKIN * b->vb_cap) +
                         sizeof(double4) * S + sizeof(float) * (SHADOW_FLOATS / SHADOW_TILE) * S +
-                        sizeof(int) * (4 * U + S + max_tiles) + sizeof(unsigned) * 2 * U + cub_bytes +
+                        sizeof(int) * (4 * U + S + max_tiles) + sizeof(float) * 8 * max_tiles + (size_t)max_pair_units + sizeof(unsigned) * 2 * U + cub_bytes +
                         sizeof(RepDesc) * nslots + sizeof(int4) * 2 * jb + (64u << 20);
     size_t free_b = 0, total_b = 0;
     pool_setup(device);
@@ -1046,7 +1124,10 @@ static int create_empty(int sim, int prec_api, int nslots, long long max_units, 
         delete b;
         return bfail(nullptr, YK_ERR_NOMEM, "batch needs %zu bytes, %zu free", need, free_b);
     }
-    if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) {
+    if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&b->stream2, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&b->join, cudaEventDisableTiming) != cudaSuccess) {
         yk_batch_destroy(b);
         return bfail(nullptr, YK_ERR_CUDA, "stream creation failed");
     }
@@ -1080,8 +1161,10 @@ static int create_empty(int sim, int prec_api, int nslots, long long max_units, 
     BALLOC(b->rd, nslots);
     BALLOC(b->left, nslots);
     BALLOC(b->sel, nslots);
-    BALLOC(b->njobs_dev, 2);
-    BALLOC(b->counter, 1);
+    BALLOC(b->njobs_dev, 4);
+    BALLOC(b->counter, 2);
+    BALLOC(b->tbox, 8 * max_tiles);
+    BALLOC(b->Sjf, max_pair_units);
     BALLOC(b->tile_rep, max_tiles);
     BALLOC(b->vblocks, b->vb_cap);
     if (cudaMallocAsync(&b->Sj, (b->prec == PREC_MIXED ? sizeof(float) : sizeof(double)) * (size_t)b->sj_cap,

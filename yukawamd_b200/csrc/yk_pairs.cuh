@@ -68,17 +68,16 @@ struct PairJobs {
                                   // 0 if the row is zero and was not written
 };
 
-// Bounding box of each 128-slot tile on the FP32 shadow hi parts (the
-// coordinates near_groups screens), with the warp box's rounding margin:
-// one CTA of PB threads per tile.
-static __global__ void __launch_bounds__(PB)
-k_tile_boxes(const float* __restrict__ posf, int n, ForceArgs fa, float* __restrict__ tbox)
+// Bounding box of a 128-slot tile (shadow t, its first particle j0 of the n) on
+// the FP32 shadow hi parts (the coordinates near_groups screens), with the
+// warp box's rounding margin: a CTA of PB threads.
+__device__ __forceinline__ void tile_box(const float* __restrict__ t, int j0, int n, const float (&Lf)[3],
+                                         float* __restrict__ out)
 {
     __shared__ float red[PWARPS][6];
-    const int C = blockIdx.x, j = threadIdx.x, lane = j & 31, warp = j >> 5;
+    const int j = threadIdx.x, lane = j & 31, warp = j >> 5;
     const float inf = __int_as_float(0x7f800000);
-    const bool on = C * PB + j < n;
-    const float* t = posf + (size_t)C * SHADOW_FLOATS;
+    const bool on = j0 + j < n;
     float lo[3], hi[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
@@ -106,12 +105,20 @@ k_tile_boxes(const float* __restrict__ posf, int n, ForceArgs fa, float* __restr
             a = fminf(a, red[w][j]);
             b = fmaxf(b, red[w][3 + j]);
         }
-        const float mu = fmaf(3.814697265625e-6f, fa.Lf[j], (float)(2.0 * SHADOW_Q));
-        tbox[8 * C + j] = 0.5f * (a + b);
-        tbox[8 * C + 4 + j] = fmaf(0.5f, b - a, mu);
+        const float mu = fmaf(3.814697265625e-6f, Lf[j], (float)(2.0 * SHADOW_Q));
+        out[j] = 0.5f * (a + b);
+        out[4 + j] = fmaf(0.5f, b - a, mu);
     } else if (j == 3 || j == 7) {
-        tbox[8 * C + j] = 0.f;
+        out[j] = 0.f;
     }
+}
+
+// One CTA per tile.
+static __global__ void __launch_bounds__(PB)
+k_tile_boxes(const float* __restrict__ posf, int n, ForceArgs fa, float* __restrict__ tbox)
+{
+    const int C = blockIdx.x;
+    tile_box(posf + (size_t)C * SHADOW_FLOATS, C * PB, n, fa.Lf, tbox + 8 * C);
 }
 
 __host__ __device__ __forceinline__ long long tri_index(int C, int R)
