@@ -14,8 +14,9 @@ import pytest
 
 from oracle.oracle import Oracle
 from yukawamd_b200 import abi, configs
+from yukawamd_b200.engine import Engine
 
-from test_gpu_parity import check_accel, workload
+from test_gpu_parity import check_accel, rel_norm, workload
 
 pytestmark = pytest.mark.gpu
 
@@ -110,3 +111,35 @@ def test_small_nucleon_boxes(gpu, orc, n, prec, terms):
         w.params["xl"] = [edge] * 3
     check_accel(orc, w, prec, True)
     check_accel(orc, w, prec, False)
+
+
+@PRECS
+@pytest.mark.parametrize("n", [700, 12000])
+@pytest.mark.parametrize("integrator", [1, 2])
+def test_another_kernel_after_octet_steps(gpu, orc, n, prec, integrator):
+    """Octet steps gather the positions themselves and leave the FP32 shadow
+    behind: a kernel that reads it, chosen between steps with the slot order
+    kept, must see the moved positions.  (The steps move every particle by
+    far more than the tolerance.)"""
+    w = workload("mix", n, 40 + n)
+    w.params["integrator"] = integrator
+    w.params["precision"] = prec
+    p = w.yk_params(precision=prec)
+    with Engine(p, w.x, w.v, w.zii, w.aii) as e:
+        e.set_tuning(sort_every=-1)
+        e.accel(True)
+        # (read now: the last entry is also e.scalars, which the next call fills)
+        series = [(q.ev, q.ek) for q in e.run(12, 5, series=True)]
+        e.set_tuning(force_kernel=abi.KERNEL_ROWS, sort_every=-1)
+        s = e.accel(True)
+        a = e.a.copy()
+        x = e.get_state()[0]
+    a_ref, s_ref = orc.accel(p, x, w.zii, w.aii, True)
+    tol = 1e-12 if prec == abi.YK_PREC_FP64 else 1e-6
+    assert rel_norm(a[:3 * n], a_ref[:3 * n]) <= tol
+    assert abs(s.ev - s_ref.ev) <= tol * abs(s_ref.ev)
+    # a step that measures nothing leaves zeros in its entry (integrator 2)
+    for k in range(12):
+        assert (series[k][0] != 0.0) == ((k + 1) % 5 == 0), k
+        if integrator == 2:
+            assert (series[k][1] != 0.0) == ((k + 1) % 5 == 0), k

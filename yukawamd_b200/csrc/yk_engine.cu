@@ -202,6 +202,10 @@ struct yk_ctx {
     long long step_count = 0;       // integrator steps since create
     double time = 0.0;
     bool pos_dirty = true;          // positions changed on the host: repack
+    // set around a step's force call: the octet pack gathers the drifted
+    // positions; the combine ends the step
+    bool oct_gather = false, oct_tail = false;
+    StepTail tail{};
     bool need_sort = true;
     // timers
     bool perf_on = false;
@@ -556,6 +560,7 @@ static size_t pair_scratch_bytes(int n, int seg, int dev, int precision)
 
 static void free_pairs(yk_ctx* c)
 {
+    c->pos_dirty = true;                 // the next kernel may read the FP32 shadow, which octet steps leave behind
     cudaFree(c->Si);
     cudaFree(c->Sj);
     cudaFree(c->Sm);
@@ -828,7 +833,12 @@ static int launch_octets(yk_ctx* c)
     // (nucleons: always, inside octet_batch_nn)
     constexpr bool RANGE = F::PREC == PREC_FP64 && SIM != SIM_NUCLEON;
     const bool range = RANGE && !c->fa.exp_ok;
-    k_octet_pack<F><<<M, PB, 0, st>>>(c->pos, c->n, c->fa, c->posq, c->obox, tbox);
+    if (c->oct_gather)
+        k_octet_pack<F, true><<<M, PB, 0, st>>>(c->pos, c->n, c->fa, c->posq, c->obox, tbox, c->perm, c->x,
+                                                c->sa.pack_w ? c->zii : nullptr);
+    else
+        k_octet_pack<F, false><<<M, PB, 0, st>>>(c->pos, c->n, c->fa, c->posq, c->obox, tbox, nullptr, nullptr,
+                                                 nullptr);
     int k = 3;
     if (c->oct_chunks) {
         const OctetBox bx{c->pos, c->posq, c->obox, tbox, nullptr, nullptr, nullptr, c->Sm, nullptr, nullptr, c->n, M};
@@ -839,8 +849,12 @@ static int launch_octets(yk_ctx* c)
         else
             k_force_octets_all<F, SIM, MEAS, false><<<grid, 32, 0, st>>>(bx, c->oct_chunks, c->oct_len, c->Si, c->fa,
                                                                          c->err);
-        k_octet_all_combine<SIM, MEAS><<<M, COMB_THREADS, 0, st>>>(c->Si, c->Sm, c->oct_chunks, M, c->perm, c->zii,
-                                                                   c->aii, c->fa, c->a, c->rsum);
+        if (!MEAS && c->oct_tail)
+            k_octet_all_combine<SIM, MEAS, !MEAS><<<M, COMB_THREADS, 0, st>>>(
+                c->Si, c->Sm, c->oct_chunks, M, c->perm, c->zii, c->aii, c->fa, c->a, c->rsum, c->tail);
+        else
+            k_octet_all_combine<SIM, MEAS, false><<<M, COMB_THREADS, 0, st>>>(
+                c->Si, c->Sm, c->oct_chunks, M, c->perm, c->zii, c->aii, c->fa, c->a, c->rsum, StepTail{});
         return k;
     }
     if constexpr (SIM != SIM_NUCLEON) {
@@ -964,7 +978,7 @@ static int enqueue_force(yk_ctx* c, bool meas, bool timed = false)
     return k;
 }
 
-static int enqueue_finish(yk_ctx* c, bool meas, int kin_mode, bool series)
+static FinishArgs finish_args(const yk_ctx* c, bool meas, int kin_mode)
 {
     FinishArgs z = c->fz_base;
     const bool has_force = c->p.sim_type != YK_SIM_BFIELD;
@@ -979,6 +993,12 @@ static int enqueue_finish(yk_ctx* c, bool meas, int kin_mode, bool series)
     }
     z.kin_mode = kin_mode;
     z.nkp = (kin_mode == 2) ? c->nvb : 0;
+    return z;
+}
+
+static int enqueue_finish(yk_ctx* c, bool meas, int kin_mode, bool series)
+{
+    const FinishArgs z = finish_args(c, meas, kin_mode);
     k_finish<<<1, 256, 0, c->stream>>>(c->kernel >= 2 ? (c->oct ? c->rsum : c->Sm) : c->fpart, c->kpart, z, c->a, c->ds,
                                        series ? c->series : nullptr, c->series_idx);
     return 1;
@@ -1007,10 +1027,22 @@ static int enqueue_newton(yk_ctx* c, bool meas, bool series, bool resort, bool t
         k_drift_vv2<<<nb3, VBLOCK, 0, st>>>(c->x, c->v, c->vold, c->a, s);
         break;
     }
-    k_pack_slots<<<nb, VBLOCK, 0, st>>>(c->perm, c->x, c->zii, c->pos, c->posf, c->n, s.pack_w);
+    ++k;
+    c->oct_gather = c->kernel == 2 && c->oct && c->p.sim_type != YK_SIM_BFIELD;
+    if (!c->oct_gather) {
+        k_pack_slots<<<nb, VBLOCK, 0, st>>>(c->perm, c->x, c->zii, c->pos, c->posf, c->n, s.pack_w);
+        ++k;
+    }
     c->pos_dirty = false;
-    k += 2;
+    c->oct_tail = c->oct_gather && c->oct_chunks && !meas && c->p.integrator != YK_VV1 &&
+                  c->p.integrator != YK_VV3 && c->p.bfield == 0.0;
+    if (c->oct_tail)
+        c->tail = StepTail{c->v, c->vold, s.dt, finish_args(c, false, 1), c->ds, series ? c->series : nullptr,
+                           c->series_idx};
+    const bool ended = c->oct_tail;
     k += enqueue_force(c, meas, timed);
+    c->oct_gather = c->oct_tail = false;
+    if (ended) return k;
     int kin_mode;
     switch (c->p.integrator) {
     case YK_VV1:
@@ -1046,8 +1078,7 @@ static bool sort_due(const yk_ctx* c, long long step)
 // Copy scalars and the error word back and wait for the stream.
 static int sync_and_check(yk_ctx* c)
 {
-    CK(c, cudaMemcpyAsync(c->h_ds, c->ds, sizeof(DevScalars), cudaMemcpyDeviceToHost, c->stream));
-    CK(c, cudaMemcpyAsync(c->h_err, c->err, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
+    CK(c, cudaMemcpyAsync(c->h_ds, c->ds, sizeof(DevScalars) + sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
     CK(c, cudaGetLastError());
     if (*c->h_err) {
@@ -1254,7 +1285,7 @@ int yk_destroy(yk_ctx* c)
     free_pairs(c);
     void* bufs[] = {c->x, c->v, c->vold, c->a, c->zii, c->aii, c->pos, c->posf, c->perm, c->iperm,
                     c->keys0, c->keys1, c->idx0, c->cub_tmp, c->fpart, c->kpart, c->vpart, c->vsums,
-                    c->ds, c->err,
+                    c->ds,      // (and err)
                     c->series, c->series_idx, c->job_counter, c->flush_buf, c->snap, c->a_vtot, c->gofr,
                     c->stage, c->nonfinite};
     for (void* b : bufs) cudaFree(b);
@@ -1262,7 +1293,6 @@ int yk_destroy(yk_ctx* c)
     if (c->snap_done) cudaEventDestroy(c->snap_done);
     if (c->snap_stream) cudaStreamDestroy(c->snap_stream);
     cudaFreeHost(c->h_ds);
-    cudaFreeHost(c->h_err);
     for (cudaEvent_t e : c->ev_pool) cudaEventDestroy(e);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
@@ -1356,8 +1386,9 @@ int yk_create(const yk_params* p, int n, const double* x, const double* v, const
     ALLOC(c->kpart, NKIN * (size_t)c->nvb);
     ALLOC(c->vpart, NVSUM * (size_t)c->nvb);
     ALLOC(c->vsums, 8);
-    ALLOC(c->ds, 1);
-    ALLOC(c->err, 1);
+    // the error word behind the scalars, here and in h_ds: one copy brings both
+    ALLOC(c->ds, 2);
+    c->err = reinterpret_cast<unsigned*>(c->ds + 1);
     ALLOC(c->series_idx, 1);
     ALLOC(c->job_counter, 1);
 #undef ALLOC
@@ -1366,11 +1397,11 @@ int yk_create(const yk_params* p, int n, const double* x, const double* v, const
         yk_destroy(c);
         return fail(nullptr, YK_ERR_NOMEM, "sort scratch");
     }
-    if (cudaMallocHost((void**)&c->h_ds, sizeof(DevScalars)) != cudaSuccess ||
-        cudaMallocHost((void**)&c->h_err, sizeof(unsigned)) != cudaSuccess) {
+    if (cudaMallocHost((void**)&c->h_ds, 2 * sizeof(DevScalars)) != cudaSuccess) {
         yk_destroy(c);
         return fail(nullptr, YK_ERR_NOMEM, "pinned host staging failed");
     }
+    c->h_err = reinterpret_cast<unsigned*>(c->h_ds + 1);
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) {
         yk_destroy(c);
         return fail(nullptr, YK_ERR_CUDA, "stream creation failed");
@@ -2074,7 +2105,7 @@ static NoallocLayout noalloc_layout(int n, bool oct)
 
 // FP64 ions: k_force_octets_all (every pair from both sides).
 template <int SIM, bool MEAS>
-static void noalloc_octets(cudaStream_t st, const NoallocLayout& L, unsigned char* b, const double4* pos,
+static void noalloc_octets(cudaStream_t st, const NoallocLayout& L, unsigned char* b, double4* pos,
                            const ForceArgs& fa, unsigned* err, const int* perm, const double* zii, const double* aii,
                            double* a)
 {
@@ -2083,13 +2114,13 @@ static void noalloc_octets(cudaStream_t st, const NoallocLayout& L, unsigned cha
     float4* tbox = reinterpret_cast<float4*>(b + L.tbox);
     double* part = reinterpret_cast<double*>(b + L.Si);
     double* Sm = reinterpret_cast<double*>(b + L.Sm);
-    k_octet_pack<Form64><<<L.M, PB, 0, st>>>(pos, fa.n, fa, posq, obox, tbox);
+    k_octet_pack<Form64, false><<<L.M, PB, 0, st>>>(pos, fa.n, fa, posq, obox, tbox, nullptr, nullptr, nullptr);
     const OctetBox bx{pos, posq, obox, tbox, nullptr, nullptr, nullptr, Sm, nullptr, nullptr, fa.n, L.M};
     const int grid = L.M * (PB / 32) * L.chunks;
     if (fa.exp_ok) k_force_octets_all<Form64, SIM, MEAS, false><<<grid, 32, 0, st>>>(bx, L.chunks, L.len, part, fa, err);
     else k_force_octets_all<Form64, SIM, MEAS, true><<<grid, 32, 0, st>>>(bx, L.chunks, L.len, part, fa, err);
-    k_octet_all_combine<SIM, MEAS><<<L.M, COMB_THREADS, 0, st>>>(part, Sm, L.chunks, L.M, perm, zii, aii, fa, a,
-                                                                reinterpret_cast<double*>(b + L.rsum));
+    k_octet_all_combine<SIM, MEAS, false><<<L.M, COMB_THREADS, 0, st>>>(
+        part, Sm, L.chunks, L.M, perm, zii, aii, fa, a, reinterpret_cast<double*>(b + L.rsum), StepTail{});
 }
 
 template <int SIM, int PREC, bool MEAS>

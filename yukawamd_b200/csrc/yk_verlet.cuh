@@ -342,6 +342,55 @@ __device__ __forceinline__ void finish_body(const double* __restrict__ fpart, co
     }
 }
 
+// finish_body for a step that measures nothing (do_meas 0, kin_mode 1: no
+// partials, every value 0 but what the B-field case keeps, force_mode 0), by
+// one warp: a lane per value.
+__device__ __forceinline__ void finish_quiet(const FinishArgs& fz, double* __restrict__ a,
+                                             DevScalars* __restrict__ ds, double* __restrict__ series)
+{
+    const int t = threadIdx.x & 31;
+    if (t < 9 && fz.force_mode == 1) a[3 * (size_t)fz.n + t] = 0.0;
+    if (t < 13) {
+        double* f = reinterpret_cast<double*>(ds) + t;      // ev, vir, px, ek, pp[9]
+        const double v = (t < 3 && fz.force_mode == 0) ? *f : 0.0;
+        *f = v;
+        if (series) series[t] = v;
+    }
+}
+
+// The end of such a step with vel_verlet_2, for the kernel that has just stored
+// the accelerations (k_octet_all_combine): the velocities (k_post_vv2's
+// arithmetic) and, in block 0, the scalars and the series entry.
+struct StepTail {
+    double* v;
+    const double* vold;
+    double dt;
+    FinishArgs fz;
+    DevScalars* ds;
+    double* series;
+    int* series_idx;
+};
+
+// Particle i, whose a(3,i) this thread has written.
+__device__ __forceinline__ void step_tail_particle(const StepTail& tl, const double* a, int i)
+{
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const double vp = __dadd_rn(tl.vold[3 * i + k], __dmul_rn(tl.dt, a[3 * i + k]));
+        tl.v[3 * i + k] = __dmul_rn(0.5, __dadd_rn(tl.v[3 * i + k], vp));
+    }
+}
+
+// One warp of the grid.
+__device__ __forceinline__ void step_tail_finish(const StepTail& tl, double* a)
+{
+    double* slot = nullptr;
+    if (tl.series) slot = tl.series + (size_t)(*tl.series_idx) * 13;
+    finish_quiet(tl.fz, a, tl.ds, slot);
+    __syncwarp();
+    if (tl.series && (threadIdx.x & 31) == 0) *tl.series_idx += 1;
+}
+
 // Single box: one block of 256; the series slot is taken from *series_idx.
 static __global__ void __launch_bounds__(256)
 k_finish(const double* __restrict__ fpart, const double* __restrict__ kpart, FinishArgs fz,
@@ -350,7 +399,14 @@ k_finish(const double* __restrict__ fpart, const double* __restrict__ kpart, Fin
 {
     double* slot = nullptr;
     if (series) slot = series + (size_t)(*series_idx) * 13;
-    finish_body(fpart, kpart, fz, a, ds, slot);
+    if (fz.kin_mode == 1 && !fz.do_meas) {
+        if (threadIdx.x < 32) {
+            finish_quiet(fz, a, ds, slot);
+            __syncwarp();
+        }
+    } else {
+        finish_body(fpart, kpart, fz, a, ds, slot);
+    }
     if (series && threadIdx.x == 0) *series_idx += 1;
 }
 
