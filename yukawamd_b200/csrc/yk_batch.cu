@@ -285,8 +285,8 @@ k_force_pairs_batch(const double4* __restrict__ pos, const float* __restrict__ p
         bx.M = d->T;
         bx.nseg_max = d->nseg;
         const int C0 = jb.y + jb.z * d->seg;
-        if (!pairs_job<SIM, PREC, MEAS, LO ? 1 : 0, false, TB>(sm, sfa, bx, jb.y, C0, min(C0 + d->seg, bx.M),
-                                                              jb.z, Sm + (size_t)(d->sm_off + jb.w) * NSCAL, err, q))
+        if (!pairs_job<SIM, PREC, MEAS, LO, TB>(sm, sfa, bx, jb.y, C0, min(C0 + d->seg, bx.M), jb.z,
+                                                Sm + (size_t)(d->sm_off + jb.w) * NSCAL, err, q))
             return;
     }
 }

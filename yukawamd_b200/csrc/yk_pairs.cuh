@@ -194,27 +194,17 @@ __device__ __forceinline__ void reduce_scatter4(T (&r)[4][3], T (&t)[3])
 // one at 2 (sw ^ 2)), so each step's image integers are plain registers.
 // CHECK: the tile is partial, diagonal, or the CTA has inactive targets, so
 // every pair needs the validity test.
-// TILEIMG (ions): the tile's reachable sources share one image, folded into
-// th (the screen's target hi parts) and pit (the FP64 target position), so no
-// pair takes its own image.
-template <int SIM, int PREC, bool MEAS, bool CHECK, bool IMGK = false, bool TILEIMG = false>
+template <int SIM, int PREC, bool MEAS, bool CHECK>
 __device__ __forceinline__ void pair_group(const ForceArgs& fa, const double4& pi, const ScreenI& si,
                                            real_t<PREC> wi, const double4* tl, const float* tlf,
                                            int j0, int jlim, bool diag, bool active, int tid,
-                                           int sw, TargetAcc<PREC, MEAS>& acc, row_t<PREC>* my_acc,
-                                           const float2 (&th)[3] = {}, const double4& pit = double4{})
+                                           int sw, TargetAcc<PREC, MEAS>& acc, row_t<PREC>* my_acc)
 {
     using R_t = real_t<PREC>;
     const int g = j0 >> 2;
     float2 ka[3], kb[3];
-    float2 ra, rb;
-    if constexpr (TILEIMG) {
-        ra = screen_r2_tile_x2(th, tlf, g, 2 * sw);
-        rb = screen_r2_tile_x2(th, tlf, g, 2 * (sw ^ 2));
-    } else {
-        ra = screen_r2k_x2(fa, si, tlf, g, 2 * sw, ka);
-        rb = screen_r2k_x2(fa, si, tlf, g, 2 * (sw ^ 2), kb);
-    }
+    const float2 ra = screen_r2k_x2(fa, si, tlf, g, 2 * sw, ka);
+    const float2 rb = screen_r2k_x2(fa, si, tlf, g, 2 * (sw ^ 2), kb);
     const float* tw = tlf + 6 * SHADOW_TILE + j0;
     unsigned m = (ra.x <= screen_lim<SIM>(fa, si.w, tw[sw]) ? 1u : 0u) |
                  (ra.y <= screen_lim<SIM>(fa, si.w, tw[sw ^ 1]) ? 2u : 0u) |
@@ -242,14 +232,10 @@ __device__ __forceinline__ void pair_group(const ForceArgs& fa, const double4& p
         for (int jj = 0; jj < 4; ++jj) {
             const double4 pjv = tl[j0 + (jj ^ sw)];
             PairOut<R_t> o;
-            if constexpr (TILEIMG) {
-                ion_pair_tile<PREC, MEAS>(fa, pit, pjv, ((m >> jj) & 1u) != 0, o);
-            } else {
-                const float k[3] = {jj == 0 ? ka[0].x : jj == 1 ? ka[0].y : jj == 2 ? kb[0].x : kb[0].y,
-                                    jj == 0 ? ka[1].x : jj == 1 ? ka[1].y : jj == 2 ? kb[1].x : kb[1].y,
-                                    jj == 0 ? ka[2].x : jj == 1 ? ka[2].y : jj == 2 ? kb[2].x : kb[2].y};
-                ion_pair_nb<PREC, MEAS, IMGK>(fa, pi, pjv, ((m >> jj) & 1u) != 0, k, o);
-            }
+            const float k[3] = {jj == 0 ? ka[0].x : jj == 1 ? ka[0].y : jj == 2 ? kb[0].x : kb[0].y,
+                                jj == 0 ? ka[1].x : jj == 1 ? ka[1].y : jj == 2 ? kb[1].x : kb[1].y,
+                                jj == 0 ? ka[2].x : jj == 1 ? ka[2].y : jj == 2 ? kb[2].x : kb[2].y};
+            ion_pair_nb<PREC, MEAS>(fa, pi, pjv, ((m >> jj) & 1u) != 0, k, o);
             if constexpr (PREC == PREC_FP64) acc.add(o, SIM == SIM_MIX ? (R_t)pjv.w : (R_t)1);
             else gs.add(o, SIM == SIM_MIX ? (R_t)pjv.w : (R_t)1);
             const R_t fsj = o.fs * wi;               // 0 unless the pair interacts
@@ -852,11 +838,9 @@ __device__ __forceinline__ void pairs_issue(PairSmem<RowT>& sm, const BoxView& b
 // only after that copy has landed, so it never overwrites rows that are
 // still being summed.  Warps may thus run up to one tile apart, which absorbs
 // the uneven work of the four target groups.
-// LOMODE: whether the mixed ion path takes its displacement from the shadow's
-// hi/lo parts (pair_group_lo): 0 never, 1 always (the caller has checked
-// fa.lo; the FP64-tile path is then not compiled in, which frees its
-// registers), 2 as fa.lo says (boxes of a batch differ).
-template <int SIM, int PREC, bool MEAS, int LOMODE = 2, bool IMGK = false, bool TB = false>
+// LO: the mixed form takes its displacement from the shadow's hi/lo parts
+// (the caller has checked fa.lo, for nucleons fa.hilo): no FP64 source tiles.
+template <int SIM, int PREC, bool MEAS, bool LO, bool TB = false>
 __device__ __forceinline__ bool pairs_job(PairSmem<row_t<PREC>>& sm, const ForceArgs& fa, const BoxView& bx, int R,
                                           int C0, int C1, int sg, double* __restrict__ sm_row,
                                           unsigned* __restrict__ err, unsigned& q)
@@ -882,12 +866,10 @@ __device__ __forceinline__ bool pairs_job(PairSmem<row_t<PREC>>& sm, const Force
     const bool all_p = SIM == SIM_NUCLEON && box.has_p && __all_sync(0xffffffffu, !active || pi.w == 1.0);
     TargetAcc<PREC, MEAS> acc;
     acc.zero();
-    // the mixed form on a box that allows it: FP32 displacements from the
-    // shadow's hi/lo parts, no FP64 source tiles (ions: fa.lo; nucleons:
-    // fa.hilo, with the FP64 positions read from global memory for the rare
-    // pairs near |d| = L/2)
-    const bool lo = (PREC == PREC_MIXED) &&
-                    (LOMODE == 1 || (LOMODE == 2 && (SIM == SIM_NUCLEON ? fa.hilo != 0 : fa.lo != 0)));
+    // FP32 displacements from the shadow's hi/lo parts, no FP64 source tiles
+    // (nucleons read the FP64 positions from global memory for the rare pairs
+    // near |d| = L/2)
+    constexpr bool lo = PREC == PREC_MIXED && LO;
     float nli[3] = {0.f, 0.f, 0.f};
     if (lo) {
 #pragma unroll
@@ -928,8 +910,8 @@ __device__ __forceinline__ bool pairs_job(PairSmem<row_t<PREC>>& sm, const Force
             // on the diagonal tile only sources after the warp's first target count
             const int jmin = max(diag ? 32 * warp + 1 : 0, w0);
             const bool full = !diag && jlim == PB && all_active && w0 == 0;
-            if (lo) {
-                if constexpr (PREC == PREC_MIXED && SIM == SIM_NUCLEON) {
+            if constexpr (lo) {
+                if constexpr (SIM == SIM_NUCLEON) {
                     unsigned gm = near_groups<SIM>(fa, box, tlf, jlim, jmin);
                     open_row(gm);
                     const float* tll = reinterpret_cast<const float*>(tl);
@@ -963,7 +945,7 @@ __device__ __forceinline__ bool pairs_job(PairSmem<row_t<PREC>>& sm, const Force
                     else if (mode == NN_NOP) run(std::integral_constant<int, NN_NOP>());
                     else run(std::integral_constant<int, NN_ANY>());
                 }
-                if constexpr (PREC == PREC_MIXED && (SIM == SIM_PURE || SIM == SIM_MIX)) {
+                if constexpr (SIM == SIM_PURE || SIM == SIM_MIX) {
                     int kcode = -1;
                     unsigned gm = near_groups_img(fa, box, tlf, jlim, jmin, kcode);
                     open_row(gm);
@@ -1004,57 +986,16 @@ __device__ __forceinline__ bool pairs_job(PairSmem<row_t<PREC>>& sm, const Force
                         }
                     }
                 }
-            } else if (IMGK && (SIM == SIM_PURE || SIM == SIM_MIX)) {
-                // ions whose screen image integers are exact: the tile image
-                // when the tile has one, else each pair's own
-                if constexpr (IMGK && (SIM == SIM_PURE || SIM == SIM_MIX)) {
-                    int kcode = -1;
-                    unsigned gm = near_groups_img(fa, box, tlf, jlim, jmin, kcode);
-                    open_row(gm);
-                    if (box.tile_img && kcode >= 0) {
-                        float2 th[3];
-                        const float nh[3] = {si.nx, si.ny, si.nz};
-                        const double pc[3] = {pi.x, pi.y, pi.z};
-                        double pt[3];
-#pragma unroll
-                        for (int c = 0; c < 3; ++c) {
-                            const float k = img_of(kcode, c);
-                            const float h = fmaf(-k, fa.Lh[c], nh[c]);       // exact
-                            th[c] = make_float2(h, h);
-                            pt[c] = __fma_rn((double)k, fa.xl[c], pc[c]);
-                        }
-                        const double4 pit = make_double4(pt[0], pt[1], pt[2], pi.w);
-                        if (full) {
-                            for (; gm; gm &= gm - 1)
-                                pair_group<SIM, PREC, MEAS, false, true, true>(fa, pi, si, wi, tl, tlf,
-                                                                               4 * (__ffs(gm) - 1), jlim, diag, active,
-                                                                               tid, sw, acc, my_acc, th, pit);
-                        } else {
-                            for (; gm; gm &= gm - 1)
-                                pair_group<SIM, PREC, MEAS, true, true, true>(fa, pi, si, wi, tl, tlf,
-                                                                              4 * (__ffs(gm) - 1), jlim, diag, active,
-                                                                              tid, sw, acc, my_acc, th, pit);
-                        }
-                    } else if (full) {
-                        for (; gm; gm &= gm - 1)
-                            pair_group<SIM, PREC, MEAS, false, true>(fa, pi, si, wi, tl, tlf, 4 * (__ffs(gm) - 1), jlim,
-                                                                     diag, active, tid, sw, acc, my_acc);
-                    } else {
-                        for (; gm; gm &= gm - 1)
-                            pair_group<SIM, PREC, MEAS, true, true>(fa, pi, si, wi, tl, tlf, 4 * (__ffs(gm) - 1), jlim,
-                                                                    diag, active, tid, sw, acc, my_acc);
-                    }
-                }
             } else {
                 unsigned gm = near_groups<SIM>(fa, box, tlf, jlim, jmin);
                 open_row(gm);
                 if (full) {
                     for (; gm; gm &= gm - 1)
-                        pair_group<SIM, PREC, MEAS, false, IMGK>(fa, pi, si, wi, tl, tlf, 4 * (__ffs(gm) - 1), jlim,
+                        pair_group<SIM, PREC, MEAS, false>(fa, pi, si, wi, tl, tlf, 4 * (__ffs(gm) - 1), jlim,
                                                                  diag, active, tid, sw, acc, my_acc);
                 } else {
                     for (; gm; gm &= gm - 1)
-                        pair_group<SIM, PREC, MEAS, true, IMGK>(fa, pi, si, wi, tl, tlf, 4 * (__ffs(gm) - 1), jlim,
+                        pair_group<SIM, PREC, MEAS, true>(fa, pi, si, wi, tl, tlf, 4 * (__ffs(gm) - 1), jlim,
                                                                 diag, active, tid, sw, acc, my_acc);
                 }
             }
@@ -1137,10 +1078,8 @@ constexpr bool pairs_tile_boxes()
     return PREC == PREC_MIXED && LO && SIM != SIM_NUCLEON;
 }
 
-// LO: the mixed ion kernel for boxes with fa.lo (pair_group_lo); IMGK: a
-// kernel for ion boxes with fa.img_k (the screen's image integers replace the
-// exact minimum-image comparisons, which are then not compiled in).
-template <int SIM, int PREC, bool MEAS, bool LO = false, bool IMGK = false>
+// LO: the mixed kernel for boxes with fa.lo (nucleons: fa.hilo).
+template <int SIM, int PREC, bool MEAS, bool LO = false>
 __global__ void __launch_bounds__(PB, (pairs_ctas_per_sm<SIM, PREC, LO, MEAS>()))
 k_force_pairs(const double4* __restrict__ pos, const float* __restrict__ posf, PairJobs pj,
               int* __restrict__ job_counter, ForceArgs fa, double* __restrict__ Si,
@@ -1166,8 +1105,8 @@ k_force_pairs(const double4* __restrict__ pos, const float* __restrict__ posf, P
         if (job >= pj.njobs) break;
         const int4 js = pj.jobs[job];
         constexpr bool TB = pairs_tile_boxes<SIM, PREC, LO>();
-        if (!pairs_job<SIM, PREC, MEAS, LO ? 1 : 0, IMGK, TB>(sm, fa, bx, js.x, js.y, js.z, js.w,
-                                                              Sm + (size_t)job * NSCAL, err, q))
+        if (!pairs_job<SIM, PREC, MEAS, LO, TB>(sm, fa, bx, js.x, js.y, js.z, js.w, Sm + (size_t)job * NSCAL, err,
+                                                q))
             return;
     }
 }
