@@ -221,18 +221,25 @@ __host__ __device__ inline bool box_lo(int sim, int prec, const ForceArgs& fa)
 }
 
 // Bounding box of every tile on the FP32 shadow hi parts, for the boxes whose
-// kernel looks at them (k_tile_boxes): one CTA per tile.
+// kernel looks at them (k_tile_boxes).  This kernel and the combine go over the
+// list of the held tiles (tiles[0 .. *ntiles)) with a grid of at most
+// TILE_GRID CTAs: a slot batch has room for many more tiles than it holds, and
+// a CTA for each of them would cost more than the work.
+constexpr int TILE_GRID = 148 * 16;
+
 __global__ void __launch_bounds__(PB)
-k_b_tile_boxes(const int* __restrict__ tile_rep, const RepDesc* __restrict__ rd, const int* __restrict__ left,
-               const float* __restrict__ posf, float* __restrict__ tbox)
+k_b_tile_boxes(const int* __restrict__ tiles, const int* __restrict__ ntiles, const int* __restrict__ tile_rep,
+               const RepDesc* __restrict__ rd, const int* __restrict__ left, const float* __restrict__ posf,
+               float* __restrict__ tbox)
 {
-    const int r = tile_rep[blockIdx.x];
-    if (r < 0 || left[r] <= 0) return;
-    const RepDesc* d = rd + r;
-    if (!d->fa.lo) return;
-    const int T0 = d->S / PB;
-    tile_box(posf + (size_t)blockIdx.x * SHADOW_FLOATS, ((int)blockIdx.x - T0) * PB, d->fa.n, d->fa.Lf,
-             tbox + 8 * (size_t)blockIdx.x);
+    const int nt = *ntiles;
+    for (int k = blockIdx.x; k < nt; k += gridDim.x) {
+        const int C = tiles[k], r = tile_rep[C];
+        const RepDesc* d = rd + r;
+        if (left[r] <= 0 || !d->fa.lo) continue;
+        tile_box(posf + (size_t)C * SHADOW_FLOATS, (C - d->S / PB) * PB, d->fa.n, d->fa.Lf, tbox + 8 * (size_t)C);
+        __syncthreads();
+    }
 }
 
 // The persistent force kernels over the batch's work items: the boxes that take
@@ -293,58 +300,64 @@ k_force_pairs_batch(const double4* __restrict__ pos, const float* __restrict__ p
 
 // Per slot of the boxes in sel (all if NULL) whose budget is not spent: the
 // fixed-order sum of its partials, the reference's scaling, and the store to
-// the caller's order: one CTA per tile, as k_combine (the thread groups'
-// shares, and only the source-side rows that were written: Sjf).  tile_rep: box
-// of every tile, -1 unused.
+// the caller's order: a CTA takes a tile at a time, as k_combine (the thread
+// groups' shares, and only the source-side rows that were written: Sjf).
+// tile_rep: box of every tile.
 template <int SIM, int PREC>
 __global__ void __launch_bounds__(COMB_THREADS)
-k_b_combine(const int* __restrict__ tile_rep, const RepDesc* __restrict__ rd, const int* __restrict__ sel,
-            const int* __restrict__ left, const double* __restrict__ Si, const row_t<PREC>* __restrict__ Sj,
-            const unsigned char* __restrict__ Sjf, const int* __restrict__ perm, const double* __restrict__ zii,
-            const double* __restrict__ aii, double* __restrict__ a)
+k_b_combine(const int* __restrict__ tiles, const int* __restrict__ ntiles, const int* __restrict__ tile_rep,
+            const RepDesc* __restrict__ rd, const int* __restrict__ sel, const int* __restrict__ left,
+            const double* __restrict__ Si, const row_t<PREC>* __restrict__ Sj, const unsigned char* __restrict__ Sjf,
+            const int* __restrict__ perm, const double* __restrict__ zii, const double* __restrict__ aii,
+            double* __restrict__ a)
 {
     __shared__ double part[COMB_GROUPS][PB * 3];
-    const int r = tile_rep[blockIdx.x];
-    if (r < 0 || (sel && !sel[r]) || left[r] <= 0) return;
-    const RepDesc* d = rd + r;
-    const int R = (int)blockIdx.x - d->S / PB;
     const int g = threadIdx.x / (PB * 3), t = threadIdx.x % (PB * 3), lane = threadIdx.x & 31;
     constexpr size_t ROW = (size_t)PB * 3;
-    const int nseg = (d->T - R + d->seg - 1) / d->seg;
-    double F = 0.0;
-    const double* si = Si + d->Si_off + (size_t)R * d->nseg * ROW + t;
+    const int nt = *ntiles;
+    for (int k = blockIdx.x; k < nt; k += gridDim.x) {
+        const int C = tiles[k], r = tile_rep[C];
+        if ((sel && !sel[r]) || left[r] <= 0) continue;
+        const RepDesc* d = rd + r;
+        const int R = C - d->S / PB;
+        const int nseg = (d->T - R + d->seg - 1) / d->seg;
+        double F = 0.0;
+        const double* si = Si + d->Si_off + (size_t)R * d->nseg * ROW + t;
 #pragma unroll 4
-    for (int s = g; s < nseg; s += COMB_GROUPS) F += si[(size_t)s * ROW];
-    const row_t<PREC>* sj = Sj + d->Sj_off + (size_t)tri_index(R, 0) * ROW + t;
-    const unsigned char* fl = Sjf + d->Sj_off / (PB * 3) + tri_index(R, 0);
-    // the written rows, 32 units at a time (the warps of a group agree)
-    for (int b = g; b <= R; b += 32 * COMB_GROUPS) {
-        const int R2 = b + COMB_GROUPS * lane;
-        unsigned m = __ballot_sync(0xffffffffu, R2 <= R && fl[min(R2, R)] != 0);
-        while (m) {
-            double v[4];
+        for (int s = g; s < nseg; s += COMB_GROUPS) F += si[(size_t)s * ROW];
+        const row_t<PREC>* sj = Sj + d->Sj_off + (size_t)tri_index(R, 0) * ROW + t;
+        const unsigned char* fl = Sjf + d->Sj_off / (PB * 3) + tri_index(R, 0);
+        // the written rows, 32 units at a time (the warps of a group agree)
+        for (int b = g; b <= R; b += 32 * COMB_GROUPS) {
+            const int R2 = b + COMB_GROUPS * lane;
+            unsigned m = __ballot_sync(0xffffffffu, R2 <= R && fl[min(R2, R)] != 0);
+            while (m) {
+                double v[4];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                v[k] = m ? (double)sj[(size_t)(b + COMB_GROUPS * (__ffs(m) - 1)) * ROW] : 0.0;
-                m &= m - 1;
+                for (int u = 0; u < 4; ++u) {
+                    v[u] = m ? (double)sj[(size_t)(b + COMB_GROUPS * (__ffs(m) - 1)) * ROW] : 0.0;
+                    m &= m - 1;
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) F += v[u];
             }
-#pragma unroll
-            for (int k = 0; k < 4; ++k) F += v[k];
         }
-    }
-    part[g][t] = F;
-    __syncthreads();
-    const int l = threadIdx.x;
-    if (l >= PB || R * PB + l >= d->fa.n) return;
-    double Fv[3];
+        part[g][t] = F;
+        __syncthreads();
+        const int l = threadIdx.x;
+        if (l < PB && R * PB + l < d->fa.n) {
+            double Fv[3];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        Fv[c] = part[0][3 * l + c];
+            for (int c = 0; c < 3; ++c) {
+                Fv[c] = part[0][3 * l + c];
 #pragma unroll
-        for (int q = 1; q < COMB_GROUPS; ++q) Fv[c] += part[q][3 * l + c];
+                for (int q = 1; q < COMB_GROUPS; ++q) Fv[c] += part[q][3 * l + c];
+            }
+            const int orig = perm[C * PB + l];
+            store_accel<SIM>(d->fa, orig - d->P, zii[orig], aii + d->P, Fv, a + d->A);
+        }
+        __syncthreads();
     }
-    const int orig = perm[blockIdx.x * PB + l];
-    store_accel<SIM>(d->fa, orig - d->P, zii[orig], aii + d->P, Fv, a + d->A);
 }
 
 // One block per slot.  kin_mode / meas as in k_finish; the series entry of
@@ -459,6 +472,7 @@ struct yk_batch {
     int4* jobs = nullptr;           // work items of all held boxes
     int4* jobs_sel = nullptr;       // ... of the boxes being admitted
     int* njobs_dev = nullptr;       // ends of the hi/lo boxes' items and of all items; the same of the admitted boxes'
+    int* tiles = nullptr;           // the held tiles; their number is njobs_dev[4]
     float* tbox = nullptr;          // tile boxes (hi/lo ion boxes)
     unsigned char* Sjf = nullptr;   // per half-pair unit: its Sj row was written
     int njobs = 0, njobs_sel = 0;
@@ -542,6 +556,7 @@ static int launch_force_b(yk_batch* b, bool sel_new)
     const int4* jobs = sel_new ? b->jobs_sel : b->jobs;
     const int* nj = b->njobs_dev + (sel_new ? 2 : 0);
     row_t<PREC>* Sj = static_cast<row_t<PREC>*>(b->Sj);
+    const int tile_grid = (int)std::min<long long>(b->tcap, TILE_GRID);
     int k = 2;
     cudaMemsetAsync(b->counter, 0, 2 * sizeof(int), b->stream);
     // the two kernels side by side: the second's CTAs come in as the first's
@@ -554,7 +569,8 @@ static int launch_force_b(yk_batch* b, bool sel_new)
         b->pos, b->posf, jobs, nj, b->counter, b->rd, b->left, b->tbox, b->Sjf, b->Si, Sj, b->Sm, b->err);
     if constexpr (PREC == PREC_MIXED) {
         if (pairs_tile_boxes<SIM, PREC, true>()) {
-            k_b_tile_boxes<<<b->tcap, PB, 0, b->stream2>>>(b->tile_rep, b->rd, b->left, b->posf, b->tbox);
+            k_b_tile_boxes<<<tile_grid, PB, 0, b->stream2>>>(b->tiles, b->njobs_dev + 4, b->tile_rep, b->rd, b->left,
+                                                             b->posf, b->tbox);
             ++k;
         }
         k_force_pairs_batch<SIM, PREC, MEAS, true><<<b->force_grid_lo, PB, 0, b->stream2>>>(
@@ -563,9 +579,9 @@ static int launch_force_b(yk_batch* b, bool sel_new)
         cudaEventRecord(b->join, b->stream2);
         cudaStreamWaitEvent(b->stream, b->join, 0);
     }
-    k_b_combine<SIM, PREC><<<b->tcap, COMB_THREADS, 0, b->stream>>>(b->tile_rep, b->rd, sel_new ? b->sel : nullptr,
-                                                                    b->left, b->Si, Sj, b->Sjf, b->perm, b->zii,
-                                                                    b->aii, b->a);
+    k_b_combine<SIM, PREC><<<tile_grid, COMB_THREADS, 0, b->stream>>>(
+        b->tiles, b->njobs_dev + 4, b->tile_rep, b->rd, sel_new ? b->sel : nullptr, b->left, b->Si, Sj, b->Sjf,
+        b->perm, b->zii, b->aii, b->a);
     return k;
 }
 
@@ -696,18 +712,18 @@ static void box_jobs(int r, int T, int seg, std::vector<int4>& jobs, std::vector
 }
 
 // Orders the items: those of hi/lo boxes first (k_force_pairs_batch), each
-// part the costliest first.  Returns the number of the former.
+// part the costliest first, by counting (every admission orders all items).
+// Returns the number of the former.
 static int order_jobs(const std::vector<char>& lo, std::vector<int4>& jobs, const std::vector<int>& cost)
 {
-    std::vector<int> order(jobs.size());
-    for (size_t k = 0; k < order.size(); ++k) order[k] = (int)k;
-    std::stable_sort(order.begin(), order.end(), [&](int u, int w) {
-        const bool lu = lo[jobs[u].x] != 0, lw = lo[jobs[w].x] != 0;
-        return lu != lw ? lu : cost[u] > cost[w];
-    });
-    const int nlo = (int)std::count_if(jobs.begin(), jobs.end(), [&](const int4& j) { return lo[j.x] != 0; });
+    const int top = jobs.empty() ? 0 : *std::max_element(cost.begin(), cost.end());
+    auto key = [&](size_t k) { return (lo[jobs[k].x] ? 0 : top + 1) + top - cost[k]; };
+    std::vector<int> at(2 * (size_t)top + 3, 0);
+    for (size_t k = 0; k < jobs.size(); ++k) ++at[key(k) + 1];
+    for (size_t q = 1; q < at.size(); ++q) at[q] += at[q - 1];
+    const int nlo = at[top + 1];
     std::vector<int4> out(jobs.size());
-    for (size_t k = 0; k < order.size(); ++k) out[k] = jobs[order[k]];
+    for (size_t k = 0; k < jobs.size(); ++k) out[at[key(k)]++] = jobs[k];
     jobs.swap(out);
     return nlo;
 }
@@ -771,6 +787,7 @@ static int relayout(yk_batch* b, int seg, const std::vector<char>& newsel)
     std::vector<int> tile_rep(b->tcap, -1), seg_b(b->nslots, 0), seg_e(b->nslots, 0), segn_b(b->nslots, 0),
         segn_e(b->nslots, 0), selv(b->nslots, 0);
     std::vector<char> lo(b->nslots, 0);
+    std::vector<int> tiles;
     int held = 0;
     for (int r = 0; r < b->nslots; ++r) {
         RepDesc& d = b->hrd[r];
@@ -804,7 +821,11 @@ static int relayout(yk_batch* b, int seg, const std::vector<char>& newsel)
         d.kb0 = (int)vblocks.size();
         d.nkb = nb;
         for (int q = 0; q < nb; ++q) vblocks.push_back(make_int2(r, q));
-        for (int t = 0; t < d.T; ++t) tile_rep[d.S / PB + t] = r;
+        // the last tiles first: they have the most rows to sum
+        for (int t = d.T - 1; t >= 0; --t) {
+            tile_rep[d.S / PB + t] = r;
+            tiles.push_back(d.S / PB + t);
+        }
         seg_b[r] = d.P;
         seg_e[r] = d.P + d.fa.n;
         lo[r] = box_lo(b->sim, b->prec, d.fa);
@@ -818,7 +839,7 @@ static int relayout(yk_batch* b, int seg, const std::vector<char>& newsel)
     b->njobs_sel = (int)jobs_sel.size();
     b->seg = seg;
     b->nrep = held;
-    const int nj[4] = {nlo, b->njobs, nlo_sel, b->njobs_sel};
+    const int nj[5] = {nlo, b->njobs, nlo_sel, b->njobs_sel, (int)tiles.size()};
     cudaStream_t st = b->stream;
     BCK(b, cudaMemcpyAsync(b->rd, b->hrd.data(), sizeof(RepDesc) * b->nslots, cudaMemcpyHostToDevice, st));
     if (!jobs.empty())
@@ -827,6 +848,8 @@ static int relayout(yk_batch* b, int seg, const std::vector<char>& newsel)
         BCK(b, cudaMemcpyAsync(b->jobs_sel, jobs_sel.data(), sizeof(int4) * jobs_sel.size(),
                                cudaMemcpyHostToDevice, st));
     BCK(b, cudaMemcpyAsync(b->njobs_dev, nj, sizeof nj, cudaMemcpyHostToDevice, st));
+    if (!tiles.empty())
+        BCK(b, cudaMemcpyAsync(b->tiles, tiles.data(), sizeof(int) * tiles.size(), cudaMemcpyHostToDevice, st));
     BCK(b, cudaMemcpyAsync(b->vblocks, vblocks.data(), sizeof(int2) * vblocks.size(), cudaMemcpyHostToDevice, st));
     BCK(b, cudaMemcpyAsync(b->tile_rep, tile_rep.data(), sizeof(int) * tile_rep.size(), cudaMemcpyHostToDevice,
                            st));
@@ -1055,7 +1078,7 @@ int yk_batch_destroy(yk_batch* b)
                     b->pos,     b->posf,   b->perm,    b->iperm,    b->keys0,   b->keys1,   b->idx0,
                     b->idx1,    b->seg_b,  b->seg_e,   b->segn_b,   b->segn_e,  b->cub_tmp, b->rd,
                     b->left,    b->sel,    b->jobs,    b->jobs_sel, b->njobs_dev, b->counter, b->tile_rep,
-                    b->tbox,    b->Sjf,    b->vblocks, b->Si,     b->Sj,      b->Sm,       b->kpart,   b->ds,      b->err,
+                    b->tbox,    b->Sjf,    b->tiles,    b->vblocks, b->Si,     b->Sj,      b->Sm,       b->kpart,   b->ds,      b->err,
                     b->series,  b->series_idx};
     if (b->stream) {
         for (void* p : bufs)
@@ -1114,7 +1137,7 @@ static int create_empty(int sim, int prec_api, int nslots, long long max_units, 
     const size_t need = sj_elem * (size_t)b->sj_cap + sizeof(double) * (size_t)(14 * U + jb * PB * 3 + NSCAL * jb +
                                                   (long long)NKIN * b->vb_cap) +
                         sizeof(double4) * S + sizeof(float) * (SHADOW_FLOATS / SHADOW_TILE) * S +
-                        sizeof(int) * (4 * U + S + max_tiles) + sizeof(float) * 8 * max_tiles + (size_t)max_pair_units + sizeof(unsigned) * 2 * U + cub_bytes +
+                        sizeof(int) * (4 * U + S + 2 * max_tiles) + sizeof(float) * 8 * max_tiles + (size_t)max_pair_units + sizeof(unsigned) * 2 * U + cub_bytes +
                         sizeof(RepDesc) * nslots + sizeof(int4) * 2 * jb + (64u << 20);
     size_t free_b = 0, total_b = 0;
     pool_setup(device);
@@ -1161,7 +1184,8 @@ static int create_empty(int sim, int prec_api, int nslots, long long max_units, 
     BALLOC(b->rd, nslots);
     BALLOC(b->left, nslots);
     BALLOC(b->sel, nslots);
-    BALLOC(b->njobs_dev, 4);
+    BALLOC(b->njobs_dev, 5);
+    BALLOC(b->tiles, max_tiles);
     BALLOC(b->counter, 2);
     BALLOC(b->tbox, 8 * max_tiles);
     BALLOC(b->Sjf, max_pair_units);
