@@ -132,6 +132,26 @@ __device__ __forceinline__ double min_image_abs(double d, double L)
     return __dadd_rn(d, far ? __hiloint2double(hi, __double2loint(L)) : 0.0);
 }
 
+// The image numbers of an octet's sources, rint(d / L) per axis, packed 10 bits
+// each (from the low bits of the magic sum d / L + 1.5 2^23).
+__device__ __forceinline__ unsigned octet_image(float magic_sum, int c)
+{
+    return (__float_as_uint(magic_sum) & 0x3ffu) << (10 * c);
+}
+
+__device__ __forceinline__ int octet_image_of(int code, int c) { return (int)((unsigned)code << (22 - 10 * c)) >> 22; }
+
+// Whether a fold by the packed images is the reference's image of a pair within
+// L/2: it takes one edge at most (particles 3/2 L or more apart, outside the
+// box, keep the rest).
+__device__ __forceinline__ bool octet_image_single(int code)
+{
+    bool one = true;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) one = one && abs(octet_image_of(code, c)) <= 1;
+    return one;
+}
+
 // Sums of one lane over the batches of an octet on a tile.
 template <bool MEAS>
 struct OctetSum {
@@ -383,7 +403,7 @@ __device__ __forceinline__ int octet_list(const ForceArgs& fa, const float (&oc)
     const float MAGIC = 12582912.0f;
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
-    unsigned c_and = 0x3fu, c_or = 0u;
+    unsigned c_and = 0x3fffffffu, c_or = 0u;
     reinterpret_cast<unsigned*>(list)[lane] = OCT_PAD * 0x01010101u;
     __syncwarp();
     int cnt = 0;
@@ -399,7 +419,7 @@ __device__ __forceinline__ int octet_list(const ForceArgs& fa, const float (&oc)
             if constexpr (!UNI) {
                 const float kb = fmaf(v, fa.invLf[c], MAGIC);
                 v = fmaf(-fa.Lf[c], kb - MAGIC, v);
-                code |= (__float_as_uint(kb) & 3u) << (2 * c);
+                code |= octet_image(kb, c);
             }
             const float m = fmaxf(fabsf(v) - oh[c], 0.f);
             dist2 = fmaf(m, m, dist2);
@@ -436,9 +456,9 @@ __device__ __forceinline__ void octet_eval(const ForceArgs& fa, double4 pt, int 
     const int sw4 = 2 * ((a >> 2) & 1) + ((a >> 1) & 1), sw2 = (a >> 2) & 1;
     const int dup = ((a & 1) ? 4 : 0) | ((a & 3) ? 2 : 0);
     if constexpr (TIMG) {
-        pt.x = __fma_rn((double)img_of(kcode, 0), fa.xl[0], pt.x);
-        pt.y = __fma_rn((double)img_of(kcode, 1), fa.xl[1], pt.y);
-        pt.z = __fma_rn((double)img_of(kcode, 2), fa.xl[2], pt.z);
+        pt.x = __fma_rn((double)octet_image_of(kcode, 0), fa.xl[0], pt.x);
+        pt.y = __fma_rn((double)octet_image_of(kcode, 1), fa.xl[1], pt.y);
+        pt.z = __fma_rn((double)octet_image_of(kcode, 2), fa.xl[2], pt.z);
     }
     int k = 0;
 #pragma unroll 1
@@ -581,10 +601,10 @@ __device__ __forceinline__ float octet_lim(const ForceArgs& fa, float p1, float 
 }
 
 // Whether an octet (box oc, oh) reaches a tile (box tc, th).  uni: seen from the
-// octet's centre every source of the tile has the image kc (packed code), and
-// that is the minimum image of every pair that counts: either no pair is as
-// far as L/2 on any axis, or none within the cutoff is (warp_box_of's
-// argument).
+// octet's centre every source of the tile has the image kc (octet_image), and
+// that is the reference's image of every pair that counts: it takes one edge at
+// most (octet_image_single), and either no pair is as far as L/2 on any axis, or
+// none within the cutoff is (warp_box_of's argument).
 template <int SIM>
 __device__ __forceinline__ bool octet_reach(const ForceArgs& fa, const float4& oc, const float4& oh, const float4& tc,
                                             const float4& th, bool& uni, int& kc)
@@ -600,7 +620,7 @@ __device__ __forceinline__ bool octet_reach(const ForceArgs& fa, const float4& o
     for (int c = 0; c < 3; ++c) {
         const float kb = fmaf(td[c], fa.invLf[c], MAGIC);
         const float dm = fabsf(fmaf(-fa.Lf[c], kb - MAGIC, td[c]));
-        kc |= (int)(__float_as_uint(kb) & 3u) << (2 * c);
+        kc |= (int)octet_image(kb, c);
         const float m = fmaxf(dm - ohv[c] - thv[c], 0.f);
         dist2 = fmaf(m, m, dist2);
         const float half = 0.5f * fa.Lf[c] - 1.0f;
@@ -608,7 +628,7 @@ __device__ __forceinline__ bool octet_reach(const ForceArgs& fa, const float4& o
         const float s = half - ohv[c];
         cut = cut && (dm + thv[c] + ohv[c] < half || (s > 0.f && s * s > lim));
     }
-    uni = one && cut;
+    uni = one && cut && octet_image_single(kc);
     return dist2 <= lim;
 }
 
@@ -713,12 +733,12 @@ __device__ __forceinline__ int octet_list_any(const ForceArgs& fa, bool uni, con
     timg = uni;
     if (uni) {
 #pragma unroll
-        for (int c = 0; c < 3; ++c) oc[c] = fmaf(img_of(kcode, c), fa.Lf[c], oc[c]);
+        for (int c = 0; c < 3; ++c) oc[c] = fmaf((float)octet_image_of(kcode, c), fa.Lf[c], oc[c]);
         return F::template list<true, NUC>(fa, oc, oh, limp, lim, tile, x, jlim, jmin, list, kcode);
     }
     const int cnt = F::template list<false, NUC>(fa, oc, oh, limp, lim, tile, x, jlim, jmin, list, kcode);
     // the listed sources' one image, where no pair inside r_c has another
-    timg = kcode >= 0;
+    timg = kcode >= 0 && octet_image_single(kcode);
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         const float e = 0.5f * fa.Lf[c] - oh[c] - 1.0f;

@@ -346,7 +346,7 @@ struct Form32 {
     {
         const int lane = threadIdx.x & 31;
         const unsigned below = (1u << lane) - 1u;
-        unsigned c_and = 0x3fu, c_or = 0u;
+        unsigned c_and = 0x3fffffffu, c_or = 0u;
         reinterpret_cast<unsigned short*>(l)[lane] = SEC * 0x0101;
         __syncwarp();
         int cnt = 0;
@@ -371,8 +371,8 @@ struct Form32 {
                     float2 v = __fadd2_rn(x[c], oct_dup(-oc[c]));
                     const float2 kb = __ffma2_rn(v, oct_dup(fa.invLf[c]), oct_dup(12582912.0f));
                     v = __ffma2_rn(oct_dup(-fa.Lf[c]), __fadd2_rn(kb, oct_dup(-12582912.0f)), v);
-                    c0 |= (__float_as_uint(kb.x) & 3u) << (2 * c);
-                    c1 |= (__float_as_uint(kb.y) & 3u) << (2 * c);
+                    c0 |= octet_image(kb.x, c);
+                    c1 |= octet_image(kb.y, c);
                     m = make_float2(fmaxf(fabsf(v.x) - oh[c], 0.f), fmaxf(fabsf(v.y) - oh[c], 0.f));
                 }
                 d2 = __ffma2_rn(m, m, d2);
@@ -421,7 +421,7 @@ struct Form32 {
         if constexpr (TIMG) {
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                const float k = img_of(kcode, c);
+                const float k = (float)octet_image_of(kcode, c);
                 t.h[c] = fmaf(-k, fa.Lh[c], t.h[c]);          // exact
                 t.l[c] = fmaf(-k, fa.Ll[c], t.l[c]);
             }
