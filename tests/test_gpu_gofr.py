@@ -41,3 +41,20 @@ def test_counts_equal_oracle(gpu, kind, xl, nbin):
     p = w.yk_params()
     with Engine(p, w.x, w.v, w.zii, w.aii) as e:
         assert np.array_equal(e.gofr_counts(nbin), Oracle("double").gofr_counts(p, w.x, nbin))
+
+
+def test_counters_hold_every_pair_of_a_cta(gpu):
+    """2.8 million particles in a 1 : 1 : 60 box with the most bins (fewest
+    CTAs): nearly all pairs are past the last bin's inner edge and end in that
+    one 32-bit counter of each CTA, 4.3e9 of them if the resident CTAs alone
+    took all units.  The counts add up to n (n - 1) / 2."""
+    n = 2800000
+    w = configs.pure_ion_ocp(3, 128)
+    xl = np.array([100.0, 100.0, 6000.0])
+    w.params["xl"] = list(xl)
+    w.params["rccut"] = 30.0
+    x = np.ascontiguousarray((np.random.default_rng(4).random((n, 3)) * xl).reshape(-1))
+    with Engine(w.yk_params(), x, np.zeros(3 * n), np.full(n, 8.0), np.full(n, 16.0)) as e:
+        c = e.gofr_counts(8192)
+    assert c[-1] > 0.9 * c.sum()
+    assert int(c.sum()) == n * (n - 1) // 2

@@ -1554,10 +1554,12 @@ int yk_gofr_counts(yk_ctx* c, int nbin, double* counts)
     const size_t smem = 3 * GOFR_BLOCK * sizeof(float) + sizeof(unsigned) * ((size_t)nbin + 1);
     CK(c, cudaFuncSetAttribute(k_gofr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     // as many CTAs as are resident at once: 10 per SM by registers, fewer with
-    // many bins (27,000 ions, 500 bins: 8 per SM 494 us a call, 10 489)
+    // many bins (27,000 ions, 500 bins: 8 per SM 494 us a call, 10 489), and
+    // more where their counters could overflow
     int per_sm = 0;
     CK(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gofr, GOFR_BLOCK, smem));
-    const int grid = (int)std::min<long long>(units, (long long)std::max(per_sm, 1) * c->sms);
+    const int grid = (int)std::min<long long>(units, std::max<long long>((long long)std::max(per_sm, 1) * c->sms,
+                                                                         (units + GOFR_CTA_UNITS - 1) / GOFR_CTA_UNITS));
     CK(c, cudaMemsetAsync(c->gofr, 0, sizeof(unsigned long long) * (size_t)nbin, c->stream));
     k_gofr<<<grid, GOFR_BLOCK, smem, c->stream>>>(c->pos, g, c->gofr);
     g_launches += k + 1;

@@ -11,8 +11,9 @@
 //
 // Work: units (target tile R, source tile C >= R) of 128 x 128 slot pairs,
 // spread over a fixed grid; each CTA keeps one histogram in shared memory over
-// all its units (32-bit counters, at most 128 x 128 x units-per-CTA pairs,
-// far below 2^32) and adds it to the 64-bit global histogram once at the end.
+// all its units (32-bit counters; a CTA takes at most GOFR_CTA_UNITS units, so that
+// even all its pairs in one bin stay below 2^32) and adds it to the 64-bit
+// global histogram once at the end.
 //
 // The exact arithmetic is about 30 FP64 instructions and a square root per
 // pair, but it only matters for a pair whose distance is next to a bin edge.
@@ -35,6 +36,7 @@ namespace yk {
 
 constexpr int GOFR_BLOCK = 128;
 constexpr int GOFR_MAX_BINS = 8192;          // 32 KB of shared counters
+constexpr long long GOFR_CTA_UNITS = (1LL << 32) / (GOFR_BLOCK * GOFR_BLOCK) - 1;
 
 struct GofrArgs {
     double xl[3];
