@@ -58,3 +58,21 @@ def test_counters_hold_every_pair_of_a_cta(gpu):
         c = e.gofr_counts(8192)
     assert c[-1] > 0.9 * c.sum()
     assert int(c.sum()) == n * (n - 1) // 2
+
+
+@pytest.mark.parametrize("kind,xl", [("lattice", (64.0, 64.0, 64.0)), ("faces", (71.3, 71.3, 71.3)),
+                                     ("outside", (71.3, 71.3, 71.3)), ("uniform", (1.7e4, 1.7e4, 1.7e4)),
+                                     ("uniform", (40.0, 40.0, 2000.0))])
+@pytest.mark.parametrize("n,nbin", [(1153, 80), (1153, 4100), (1153, 4200), (4097, 150), (4097, 7400), (4097, 7600)])
+def test_counts_at_the_widest_place(gpu, kind, xl, n, nbin):
+    """The largest bin counts that are placed in FP32 (in a cube 4,100 up to
+    4,096 particles, where the bound is 0.005 of a bin, and 7,400 above, where
+    it is 0.009) and the next, whose pairs are all taken exactly; 80 and 150
+    bins are the largest in the 1 : 1 : 50 box."""
+    w = configs.pure_ion_ocp(3, n)
+    w.x = np.ascontiguousarray(_points(kind, n, xl, np.random.default_rng(nbin)).reshape(-1))
+    w.params["xl"] = list(xl)
+    w.params["rccut"] = 0.3 * min(xl)
+    p = w.yk_params()
+    with Engine(p, w.x, w.v, w.zii, w.aii) as e:
+        assert np.array_equal(e.gofr_counts(nbin), Oracle("double").gofr_counts(p, w.x, nbin))

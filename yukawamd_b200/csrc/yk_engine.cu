@@ -1549,19 +1549,22 @@ int yk_gofr_counts(yk_ctx* c, int nbin, double* counts)
     g.nbin = nbin;
     g.n = c->n;
     g.M = (c->n + GOFR_BLOCK - 1) / GOFR_BLOCK;
-    gofr_place(g);
+    const bool place = gofr_place(g);
+    const auto kernel = place ? k_gofr : k_gofr_exact;
     const long long units = (long long)g.M * (g.M + 1) / 2;
-    const size_t smem = 3 * GOFR_BLOCK * sizeof(float) + sizeof(unsigned) * ((size_t)nbin + 1);
-    CK(c, cudaFuncSetAttribute(k_gofr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const size_t smem = GOFR_BLOCK * (place ? 3 * sizeof(float) : sizeof(double4)) +
+                        sizeof(unsigned) * ((size_t)nbin + 1);
+    CK(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     // as many CTAs as are resident at once: 10 per SM by registers, fewer with
-    // many bins (27,000 ions, 500 bins: 8 per SM 494 us a call, 10 489), and
-    // more where their counters could overflow
+    // many bins (27,000 ions, 500 bins: 8 per SM 494 us a call, 10 489), the exact
+    // kernel at least 8 (8,192 bins: 6 per SM 1,091 us, 8 1,070), and more where
+    // their counters could overflow
     int per_sm = 0;
-    CK(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gofr, GOFR_BLOCK, smem));
-    const int grid = (int)std::min<long long>(units, std::max<long long>((long long)std::max(per_sm, 1) * c->sms,
+    CK(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, GOFR_BLOCK, smem));
+    const int grid = (int)std::min<long long>(units, std::max<long long>((long long)std::max(per_sm, place ? 1 : 8) * c->sms,
                                                                          (units + GOFR_CTA_UNITS - 1) / GOFR_CTA_UNITS));
     CK(c, cudaMemsetAsync(c->gofr, 0, sizeof(unsigned long long) * (size_t)nbin, c->stream));
-    k_gofr<<<grid, GOFR_BLOCK, smem, c->stream>>>(c->pos, g, c->gofr);
+    kernel<<<grid, GOFR_BLOCK, smem, c->stream>>>(c->pos, g, c->gofr);
     g_launches += k + 1;
     std::vector<unsigned long long> h(nbin);
     CK(c, cudaMemcpyAsync(h.data(), c->gofr, sizeof(unsigned long long) * (size_t)nbin, cudaMemcpyDeviceToHost,

@@ -11,8 +11,8 @@
 //
 // Work: units (target tile R, source tile C >= R) of 128 x 128 slot pairs,
 // spread over a fixed grid; each CTA keeps one histogram in shared memory over
-// all its units (32-bit counters; a CTA takes at most GOFR_CTA_UNITS units, so that
-// even all its pairs in one bin stay below 2^32) and adds it to the 64-bit
+// all its units (32-bit counters; a CTA takes at most GOFR_CTA_UNITS units, so
+// that even all its pairs in one bin stay below 2^32) and adds it to the 64-bit
 // global histogram once at the end.
 //
 // The exact arithmetic is about 30 FP64 instructions and a square root per
@@ -24,7 +24,10 @@
 // (1 in 1,000 on 500 bins) take the exact arithmetic.  27,000 ions, 500 bins:
 // 1,037 -> 489 us a call, bound by instruction issue.  (min(|d|, L - |d|) is
 // continuous in d, and |d - L rint(d / L)| is the same value, so no pair's
-// image matters to the bound.)
+// image matters to the bound.)  The bound grows with the bins and with the
+// box's longest edge over its shortest, and a warp takes the exact arithmetic
+// as soon as one of its pairs needs it: past GOFR_PLACE_EPS every pair takes it
+// in a kernel of its own (k_gofr_exact).
 #pragma once
 
 #include <algorithm>
@@ -43,10 +46,19 @@ struct GofrArgs {
     double fac2;                             // (double)(REAL*4 2*nbin/sqrt(3)) / xlmin
     double tiny;                             // (double)1.e-15f
     int nbin, n, M;                          // bins, particles, 128-slot tiles
-    // FP32 place: box, 1 / box, fac2, and half a bin less eps (negative: every
-    // pair takes the exact arithmetic)
+    // FP32 place: box, 1 / box, fac2, and half a bin less eps
     float xlf[3], ixlf[3], fac2f, in_bin;
 };
+
+// Widest bound of the FP32 place, and that of small boxes, whose few units wait
+// for each other's exact pairs.  FP32 place / every pair exact: 27,000 ions 4,000
+// bins (eps 0.005) 731 / 1,045 us, 2,000 bins at an edge ratio of 4 (0.0089) 890
+// / 1,041, 8,192 bins (0.0098) 1,037 / 1,069, 4,000 bins at 4 (0.018) 1,140 /
+// 1,045; 8,000 ions 6,000 bins (0.0072) 138 / 157, 8,192 bins 169 / 157; 4,000
+// ions 4,000 bins 82 / 85, 6,000 bins 92 / 90; 2,000 ions 4,000 bins 74 / 75,
+// 2,000 bins at 4 78 / 70.
+constexpr double GOFR_PLACE_EPS = 0.009, GOFR_PLACE_EPS_SMALL = 0.005;
+constexpr int GOFR_SMALL_N = 4096;
 
 // eps: the largest difference of the FP32 place from the reference's, in bins,
 // for coordinates from -L/8 to 9L/8 on each axis (then |d| <= 5L/4, where the
@@ -58,7 +70,9 @@ struct GofrArgs {
 // with a margin.  fac2 as FP32, its product with r and the subtraction of one
 // half add three roundings of at most fac2 r + 1 (4 with the reference's own,
 // far smaller, ones and its 1.e-15).
-inline void gofr_place(GofrArgs& g)
+//
+// Fills in the place's values; returns whether it is to be used.
+inline bool gofr_place(GofrArgs& g)
 {
     const double u = 1.0 / 16777216.0;
     const double lmax = std::max(g.xl[0], std::max(g.xl[1], g.xl[2]));
@@ -69,8 +83,9 @@ inline void gofr_place(GofrArgs& g)
         g.ixlf[k] = (float)(1.0 / g.xl[k]);
     }
     g.fac2f = (float)g.fac2;
-    // no FP32 place for boxes whose squares leave its range or with bins below it
-    g.in_bin = (wmax < 1e6 && lmax < 1e18 && lmax > 1e-15) ? (float)(0.5 - eps) - 1e-6f : -1.0f;
+    g.in_bin = (float)(0.5 - eps) - 1e-6f;
+    // none for boxes whose squares leave its range or with bins below it
+    return eps <= (g.n <= GOFR_SMALL_N ? GOFR_PLACE_EPS_SMALL : GOFR_PLACE_EPS) && wmax < 1e6 && lmax < 1e18 && lmax > 1e-15;
 }
 
 // The reference's bin (0-based) of the pair.
@@ -86,6 +101,42 @@ __device__ __forceinline__ int gofr_bin(const GofrArgs& g, const double4& pi, co
     }
     rr = __dadd_rn(__dsqrt_rn(rr), g.tiny);
     return min(g.nbin, __double2int_rz(__dadd_rn(__dmul_rn(g.fac2, rr), 1.0))) - 1;
+}
+
+// Unit u = C (C + 1) / 2 + R with 0 <= R <= C.
+__device__ __forceinline__ void gofr_tiles(long long u, int& R, int& C)
+{
+    C = (int)((sqrt(8.0 * (double)u + 1.0) - 1.0) * 0.5);
+    while ((long long)(C + 1) * (C + 2) / 2 <= u) ++C;
+    while ((long long)C * (C + 1) / 2 > u) --C;
+    R = (int)(u - (long long)C * (C + 1) / 2);
+}
+
+// Every pair by the exact arithmetic.
+static __global__ void __launch_bounds__(GOFR_BLOCK)
+k_gofr_exact(const double4* __restrict__ pos, GofrArgs g, unsigned long long* __restrict__ hist)
+{
+    extern __shared__ __align__(16) unsigned char gsm[];
+    double4* tile = reinterpret_cast<double4*>(gsm);
+    unsigned* h = reinterpret_cast<unsigned*>(gsm + GOFR_BLOCK * sizeof(double4));
+    const int tid = threadIdx.x;
+    for (int b = tid; b < g.nbin; b += GOFR_BLOCK) h[b] = 0u;
+    const long long units = (long long)g.M * (g.M + 1) / 2;
+    for (long long u = blockIdx.x; u < units; u += gridDim.x) {
+        int R, C;
+        gofr_tiles(u, R, C);
+        const int j0 = C * GOFR_BLOCK, i = R * GOFR_BLOCK + tid;
+        const int cnt = min(GOFR_BLOCK, g.n - j0);
+        __syncthreads();                     // the previous unit's tile is no longer read
+        if (tid < cnt) tile[tid] = pos[j0 + tid];
+        __syncthreads();
+        if (i >= g.n) continue;
+        const double4 pi = pos[i];
+        for (int jj = C == R ? tid + 1 : 0; jj < cnt; ++jj) atomicAdd(&h[gofr_bin(g, pi, tile[jj])], 1u);
+    }
+    __syncthreads();
+    for (int b = tid; b < g.nbin; b += GOFR_BLOCK)
+        if (h[b]) atomicAdd(&hist[b], (unsigned long long)h[b]);
 }
 
 // The unit loop's constants, held in registers: opaque moves, because the
@@ -164,11 +215,8 @@ k_gofr(const double4* __restrict__ pos, GofrArgs g, unsigned long long* __restri
     k.f2 = gofr_keep(g.fac2f);
     const long long units = (long long)g.M * (g.M + 1) / 2;
     for (long long u = blockIdx.x; u < units; u += gridDim.x) {
-        // u = C (C + 1) / 2 + R with 0 <= R <= C
-        int C = (int)((sqrt(8.0 * (double)u + 1.0) - 1.0) * 0.5);
-        while ((long long)(C + 1) * (C + 2) / 2 <= u) ++C;
-        while ((long long)C * (C + 1) / 2 > u) --C;
-        const int R = (int)(u - (long long)C * (C + 1) / 2);
+        int R, C;
+        gofr_tiles(u, R, C);
         const int j0 = C * GOFR_BLOCK;
         const int cnt = min(GOFR_BLOCK, g.n - j0);
         const int i = R * GOFR_BLOCK + tid;
@@ -177,7 +225,7 @@ k_gofr(const double4* __restrict__ pos, GofrArgs g, unsigned long long* __restri
         const float xi[3] = {__double2float_rn(pi.x), __double2float_rn(pi.y), __double2float_rn(pi.z)};
         const double4 pj = pos[min(j0 + tid, g.n - 1)];
         const float xj[3] = {__double2float_rn(pj.x), __double2float_rn(pj.y), __double2float_rn(pj.z)};
-        bool in = g.in_bin >= 0.0f;
+        bool in = true;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             const float mid = 0.5f * g.xlf[c], reach = 0.624f * g.xlf[c];
