@@ -414,9 +414,10 @@ YK_API int yk_accel_noalloc(const yk_params* p, int n,
 /* Failure-path check of the device-side waits.  The reference has no device
  * and no error codes (a fatal error calls md_exit, md_utils.f:158-183); the
  * engine's kernels instead bound every wait on a tile copy and report
- * YK_ERR_TIMEOUT.  This launches one CTA on ctx's stream that waits, with
- * both of the kernels' wait forms limited to `spins` polls (1 .. 2^22), on a
- * barrier that no copy ever completes, so every wait gives up.  Returns
+ * YK_ERR_TIMEOUT.  This launches one CTA on ctx's stream that waits, with the
+ * kernels' wait forms limited to `spins` polls (1 .. 2^22), on a barrier that
+ * no copy ever completes (in the form whose warp gives up together, half of
+ * the lanes do), so every wait gives up.  Returns
  * YK_ERR_TIMEOUT through the same error word and check as yk_accel, clears
  * it, and leaves the context usable; *gave_up (may be NULL) receives the
  * number of threads that gave up (128).  Any other return is a failure of

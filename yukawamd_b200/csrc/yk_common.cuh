@@ -84,6 +84,14 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, unsigned parity
     return false;
 }
 
+// As mbar_wait_bounded, for a warp whose lanes go on together: each lane polls
+// (and so sees the copy), and all give up if one has.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, unsigned parity, unsigned* err,
+                                               long long limit = SPIN_LIMIT)
+{
+    return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, err, limit));
+}
+
 // As mbar_wait_bounded, for the warps of a CTA that do not meet at a block
 // barrier between waits: a waiter also gives up as soon as another thread has
 // raised *abort, and one that times out raises it.

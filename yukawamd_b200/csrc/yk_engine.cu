@@ -81,25 +81,30 @@ __global__ void k_commit_state(const double* __restrict__ src, double* __restric
 // threads waits on an mbarrier that no copy is ever issued against, so its
 // phase 0 never completes.  Warps 0-1 wait as the pair kernels' warps do
 // (mbar_wait_abortable: the first to give up raises the abort flag, the
-// others then leave), warps 2-3 as the row kernel does (mbar_wait_bounded).
+// others then leave), warp 2 as the row kernel does (mbar_wait_bounded), warp 3
+// as the octet kernels do (mbar_wait_warp), with the lanes at odds: its barrier
+// is complete, and the odd lanes may not poll at all, so all must give up.
 // Every wait ends after at most `spins` polls and sets ERR_TIMEOUT in *err;
 // nothing is in flight when the CTA exits.  out[0] counts the threads that
 // gave up (all 128 when the path works).
 __global__ void __launch_bounds__(128) k_wait_selftest(long long spins, unsigned* __restrict__ err,
                                                        int* __restrict__ out)
 {
-    __shared__ uint64_t bar;
+    __shared__ uint64_t bar, complete;
     __shared__ int abort_flag;
     __shared__ int gave_up;
     if (threadIdx.x == 0) {
         mbar_init(&bar, 1);
+        mbar_init(&complete, 1);
         fence_mbar_init();
+        mbar_arrive_expect_tx(&complete, 0u);
         abort_flag = 0;
         gave_up = 0;
     }
     __syncthreads();
-    const bool ok = threadIdx.x < 64 ? mbar_wait_abortable(&bar, 0u, err, &abort_flag, spins)
-                                     : mbar_wait_bounded(&bar, 0u, err, spins);
+    const bool ok = threadIdx.x < 64   ? mbar_wait_abortable(&bar, 0u, err, &abort_flag, spins)
+                    : threadIdx.x < 96 ? mbar_wait_bounded(&bar, 0u, err, spins)
+                                       : mbar_wait_warp(&complete, 0u, err, (threadIdx.x & 1) ? 0 : spins);
     if (!ok) atomicAdd(&gave_up, 1);
     __syncthreads();
     if (threadIdx.x == 0) out[0] = gave_up;

@@ -870,7 +870,7 @@ __device__ __forceinline__ bool octets_job(OctetSmem<F>& sm, const ForceArgs& fa
                                            bx.tbox[2 * C + 1], uni, kc) && lane < OCTETS;
             unsigned om = __ballot_sync(0xffffffffu, reach);
             const unsigned um = __ballot_sync(0xffffffffu, uni);
-            if (!mbar_wait_bounded(&sm.bar, q & 1u, err)) return false;
+            if (!mbar_wait_warp(&sm.bar, q & 1u, err)) return false;
             const bool diag = C == R;
             const int w0 = max(0, (s0 - C * OCT_WPT) * OCT_WIN), w1 = min(PB, (s1 - C * OCT_WPT) * OCT_WIN);
             const int jlim = min(n - C * PB, w1);
@@ -1303,7 +1303,7 @@ k_force_octets_all(OctetBox bx, int chunks, int len, double* __restrict__ part, 
                                            bx.tbox[2 * C + 1], uni, kc) && lane < 4;
             unsigned om = __ballot_sync(0xffffffffu, reach);
             const unsigned um = __ballot_sync(0xffffffffu, uni);
-            if (!mbar_wait_bounded(&sm.bar[st], (q >> 1) & 1u, err)) {
+            if (!mbar_wait_warp(&sm.bar[st], (q >> 1) & 1u, err)) {
                 ok = false;
                 break;
             }
