@@ -36,3 +36,37 @@ def test_particles_whole_edges_apart(gpu, orc, kind, n, edges, cut):
     w.params["rccut"] = cut if cut > 1 else cut * L
     check_accel(orc, w, abi.YK_PREC_FP64, True)
     check_accel(orc, w, abi.YK_PREC_FP64, False)
+
+
+@pytest.mark.parametrize("n,prec", [(9300, abi.YK_PREC_FP64), (24700, abi.YK_PREC_MIXED)], ids=["fp64", "mixed"])
+@pytest.mark.parametrize("sort_every", [4, -1])
+@pytest.mark.parametrize("accel_first", [True, False], ids=["accel", "fresh"])
+def test_run_equals_newton_on_cut_jobs(gpu, n, prec, sort_every, accel_first):
+    """The boxes whose jobs are cut on the device: yk_run gives the bits of the
+    same steps through yk_newton over several replays of its graph, also when
+    the table has not been cut before the run."""
+    w = configs.pure_ion_ocp(51, n)
+    # in an order that is spatial without a sort, moving fast: a cut at other
+    # positions is another cut
+    L = w.params["xl"][0]
+    x = w.x.reshape(-1, 3)
+    cell = np.floor(x / L * 8).astype(int)
+    w.x = np.ascontiguousarray(x[np.lexsort((cell[:, 2], cell[:, 1], cell[:, 0]))].reshape(-1))
+    w.v = np.random.default_rng(5).standard_normal(3 * n) * 0.01 * L / w.params["dt"]
+    w.params["rccut"] = 0.25 * L
+    p = w.yk_params(precision=prec)
+    steps, me = 23, 5
+    out = []
+    for run in (False, True):
+        with Engine(p, w.x, w.v, w.zii, w.aii) as e:
+            e.set_tuning(sort_every=sort_every, graph_steps=5)
+            if accel_first:
+                e.accel(True)
+            if run:
+                ser = e.run(steps, me)
+            else:
+                ser = [abi.YkScalars.from_buffer_copy(e.newton(g % me == 0)) for g in range(1, steps + 1)]
+            out.append((e.get_state(), [bytes(t) for t in ser]))
+    for A, B in zip(out[0][0], out[1][0]):
+        assert np.array_equal(A, B)
+    assert out[0][1] == out[1][1]

@@ -1075,6 +1075,12 @@ static int enqueue_newton(yk_ctx* c, bool meas, bool series, bool resort, bool t
     return k;
 }
 
+// Whether the next force call of the octet kernel cuts its jobs (launch_octets).
+static bool cut_due(const yk_ctx* c)
+{
+    return c->kernel == 2 && c->oct && !c->oct_chunks && c->oct_jobs_due;
+}
+
 static bool sort_due(const yk_ctx* c, long long step)
 {
     return c->sort_every > 0 && step % c->sort_every == 0;
@@ -1159,7 +1165,9 @@ static int finish_run(yk_ctx* c, int nsteps, bool want_series, yk_scalars* serie
 
 // Graph of K steps starting at a step count divisible by sort_every (so the
 // sort falls on local step 0) with measuring phase `phase` (local step l,
-// 1-based, measures when (phase + l) % me == 0).
+// 1-based, measures when (phase + l) % me == 0).  Capturing runs nothing: what
+// is due stays due, and a graph cuts the octet kernel's jobs only next to its
+// own sorts.
 static GraphEntry* get_graph(yk_ctx* c, int K, int me, int phase, bool series, int* rc)
 {
     *rc = YK_OK;
@@ -1181,12 +1189,14 @@ static GraphEntry* get_graph(yk_ctx* c, int K, int me, int phase, bool series, i
         return nullptr;
     }
     int kernels = 0;
+    const bool due = c->oct_jobs_due;
     for (int l = 1; l <= K; ++l) {
         const bool meas = me > 0 && (phase + l) % me == 0;
         const bool resort = c->sort_every > 0 && (l - 1) % c->sort_every == 0;
         kernels += enqueue_newton(c, meas, series, resort);
     }
     e = cudaStreamEndCapture(c->stream, &g);
+    c->oct_jobs_due = due;
     if (e != cudaSuccess) {
         *rc = fail(c, YK_ERR_CUDA, "graph capture failed: %s", cudaGetErrorString(e));
         return nullptr;
@@ -1648,8 +1658,10 @@ int yk_run(yk_ctx* c, int nsteps, int meas_every, yk_scalars* series)
         c->perf.steps += nsteps;
         return finish_run(c, nsteps, want_series, series);
     }
-    // Eager steps until the step count is aligned with the sort cadence,
-    // then graphs of K steps, then the rest.  K is a multiple of sort_every
+    // Eager steps until the step count is aligned with the sort cadence (or,
+    // without a cadence, until the octet kernel's jobs are cut, which a graph
+    // would otherwise repeat on every replay), then graphs of K steps, then the
+    // rest.  K is a multiple of sort_every
     // and, when that keeps the graph within 4 graph_steps, of meas_every
     // too, so that every graph of the run starts at the same measuring
     // phase and one captured graph serves them all.
@@ -1660,7 +1672,7 @@ int yk_run(yk_ctx* c, int nsteps, int meas_every, yk_scalars* series)
         if (l <= 4LL * std::max(c->graph_steps, unit)) unit = (int)l;
     }
     const int K = c->sort_every > 0 || me > 0 ? unit * std::max(1, c->graph_steps / unit) : c->graph_steps;
-    while (s <= nsteps && c->sort_every > 0 && c->step_count % c->sort_every != 0) {
+    while (s <= nsteps && (c->sort_every > 0 ? c->step_count % c->sort_every != 0 : cut_due(c))) {
         k += enqueue_newton(c, meas_at(s), want_series, sort_due(c, c->step_count));
         c->step_count += 1;
         ++s;
@@ -1671,6 +1683,7 @@ int yk_run(yk_ctx* c, int nsteps, int meas_every, yk_scalars* series)
         GraphEntry* g = get_graph(c, K, me, me > 0 ? (s - 1) % me : 0, want_series, &rc);
         if (!g) return rc;
         CK(c, cudaGraphLaunch(g->exec, c->stream));
+        if (c->sort_every > 0) c->oct_jobs_due = false;     // cut after the graph's sorts
         k += g->kernels;
         c->step_count += K;
         s += K;
