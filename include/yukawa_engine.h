@@ -165,7 +165,10 @@ YK_API int yk_run(yk_ctx* ctx, int nsteps, int meas_every, yk_scalars* series);
 
 /* Host <-> device state sync points (before save_config / checkpoint /
  * dump_data and around host-side tnorm / cancel_vcom / strain).  Any pointer
- * may be NULL to skip that array.  a is double[3*n] (columns 0..n-1). */
+ * may be NULL to skip that array.  a is double[3*n] (columns 0..n-1).
+ * Positions set here keep the slots' spatial order until the next scheduled
+ * sort, or are put in order before the next force call when they are far (in
+ * all, since the last sort) from those that the order was made for. */
 YK_API int yk_get_state(yk_ctx* ctx, double* x, double* v, double* vold, double* a);
 YK_API int yk_set_state(yk_ctx* ctx, const double* x, const double* v,
                  const double* vold, const double* a);

@@ -70,3 +70,37 @@ def test_run_equals_newton_on_cut_jobs(gpu, n, prec, sort_every, accel_first):
     for A, B in zip(out[0][0], out[1][0]):
         assert np.array_equal(A, B)
     assert out[0][1] == out[1][1]
+
+
+@pytest.mark.parametrize("n,prec", [(7000, abi.YK_PREC_FP64), (9000, abi.YK_PREC_FP64), (9300, abi.YK_PREC_FP64),
+                                    (24700, abi.YK_PREC_MIXED)])
+@pytest.mark.parametrize("calls", [1, 30], ids=["at-once", "in-steps"])
+def test_other_positions_get_their_own_order(gpu, orc, n, prec, calls):
+    """Positions that the host sets far from the old ones, at once or little by
+    little, are put in order again before the next force call: the bits are
+    those of an engine created with them.  (In 30 calls of 0.32 to 0.35
+    spacings the boxes on all pairs sort at every fifth, 9,300 at every second,
+    24,700 at each.)"""
+    w = configs.pure_ion_ocp(61, n)
+    p = w.yk_params(precision=prec)
+    L = w.params["xl"][0]
+    # every particle along x, calls + 1 times the same way
+    step = np.zeros((n, 3))
+    step[:, 0] = np.random.default_rng(7).random(n) * L / calls
+    with Engine(p, w.x, w.v, w.zii, w.aii) as e:
+        e.accel(True)
+        for k in range(1, calls + 1):
+            x = np.ascontiguousarray(np.mod(w.x.reshape(-1, 3) + k * step, L).reshape(-1))
+            e.set_state(x=x)
+            s = e.accel(True)
+            a = e.a.copy()
+            ev = s.ev
+    with Engine(p, x, w.v, w.zii, w.aii) as e:
+        s = e.accel(True)
+        assert np.array_equal(e.a, a)
+        assert s.ev == ev
+    if calls == 1:
+        a_ref, s_ref = orc.accel(p, x, w.zii, w.aii, True)
+        tol = 1e-12 if prec == abi.YK_PREC_FP64 else 1e-6
+        assert np.linalg.norm(a[:3 * n] - a_ref[:3 * n]) <= tol * np.linalg.norm(a_ref[:3 * n])
+        assert abs(ev - s_ref.ev) <= tol * abs(s_ref.ev)

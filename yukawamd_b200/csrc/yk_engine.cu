@@ -77,6 +77,32 @@ __global__ void k_commit_state(const double* __restrict__ src, double* __restric
     if (i < cnt && *flag == 0) dst[i] = src[i];
 }
 
+// The same for positions, with the distance that they move (nearest image) in
+// units of 1/MOVED_UNIT of 1 / scale, at most MOVED_CAP of them, summed.
+constexpr int MOVED_UNIT = 1024, MOVED_CAP = 4;
+__global__ void __launch_bounds__(256)
+k_commit_positions(const double* __restrict__ src, double* __restrict__ dst, int n, const unsigned* __restrict__ flag,
+                   double lx, double ly, double lz, double scale, unsigned long long* __restrict__ moved)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned m = 0;
+    if (i < n && *flag == 0) {
+        const double L[3] = {lx, ly, lz};
+        double r2 = 0.0;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const double x = src[3 * (size_t)i + c];
+            double d = x - dst[3 * (size_t)i + c];
+            d -= L[c] * rint(d / L[c]);
+            r2 += d * d;
+            dst[3 * (size_t)i + c] = x;
+        }
+        m = (unsigned)(MOVED_UNIT * fmin(sqrt(r2) * scale, (double)MOVED_CAP));
+    }
+    m = __reduce_add_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0 && m) atomicAdd(moved, (unsigned long long)m);
+}
+
 // Failure path of the bounded waits (yk_wait_selftest): one CTA of 128
 // threads waits on an mbarrier that no copy is ever issued against, so its
 // phase 0 never completes.  Warps 0-1 wait as the pair kernels' warps do
@@ -212,6 +238,7 @@ struct yk_ctx {
     bool oct_gather = false, oct_tail = false;
     StepTail tail{};
     bool need_sort = true;
+    double moved = 0.0;             // mean distance that the host has moved the particles since the last sort, in spacings
     // timers
     bool perf_on = false;
     size_t flush_bytes = 0;
@@ -787,6 +814,7 @@ static int enqueue_order(yk_ctx* c, bool sort)
         }
         ++k;
         c->need_sort = false;
+        c->moved = 0.0;
         c->oct_jobs_due = true;
     }
     k_apply_perm<<<nb, VBLOCK, 0, st>>>(c->perm, c->iperm, c->x, c->zii, c->pos, c->posf, n,
@@ -1683,7 +1711,10 @@ int yk_run(yk_ctx* c, int nsteps, int meas_every, yk_scalars* series)
         GraphEntry* g = get_graph(c, K, me, me > 0 ? (s - 1) % me : 0, want_series, &rc);
         if (!g) return rc;
         CK(c, cudaGraphLaunch(g->exec, c->stream));
-        if (c->sort_every > 0) c->oct_jobs_due = false;     // cut after the graph's sorts
+        if (c->sort_every > 0) {                            // the graph has sorted, and cut
+            c->moved = 0.0;
+            c->oct_jobs_due = false;
+        }
         k += g->kernels;
         c->step_count += K;
         s += K;
@@ -1750,6 +1781,29 @@ int yk_snapshot_begin(yk_ctx* c, double* x, double* v, double* a)
     return YK_OK;
 }
 
+// Positions from the host keep the slot order, unless the octet kernels would
+// run on octets that have fallen apart: their lists only drop what is out of
+// reach of an octet's box.  Mean distance moved since the last sort, in particle
+// spacings, from which sorting (and cutting jobs) before a single force call is
+// no slower than that call without: half pairs ORDER_MOVED, up to ORDER_SMALL_N
+// particles ORDER_MOVED_SMALL; every pair from both sides ORDER_MOVED_ALL from
+// ORDER_ALL_N particles.  us per call of positions moved by 0.1, 0.5, 2 spacings
+// and of other ones, tiles of k_force_pairs / octets / octets sorted first (no
+// move): 55,296 FP64 983 1,045 1,427 7,325 / 674 1,036 2,483 27,785 / 555 (411),
+// 131,072 mixed 1,631 1,987 2,638 15,111 / 947 1,892 4,863 56,001 / 775 (570),
+// 12,345 FP64 229 241 303 500 / 208 318 551 1,461 / 258 (165), 9,000 FP64 180 191
+// 227 294 / 182 206 255 396 / 233 (170); 6,000 mixed 100 109 109 111 / 96 98 122
+// 122 / 160 (96).
+constexpr double ORDER_MOVED = 0.08, ORDER_MOVED_SMALL = 0.4, ORDER_MOVED_ALL = 1.5;
+constexpr int ORDER_SMALL_N = 16384, ORDER_ALL_N = 6144;
+
+static bool order_stale(const yk_ctx* c)
+{
+    if (c->kernel != 2 || !c->oct || c->sort_every <= 0) return false;
+    if (c->oct_chunks) return c->n > ORDER_ALL_N && c->moved > ORDER_MOVED_ALL;
+    return c->moved > (c->n <= ORDER_SMALL_N ? ORDER_MOVED_SMALL : ORDER_MOVED);
+}
+
 int yk_set_state(yk_ctx* c, const double* x, const double* v, const double* vold, const double* a)
 {
     if (!c) return fail(nullptr, YK_ERR_ARG, "ctx is NULL");
@@ -1758,14 +1812,15 @@ int yk_set_state(yk_ctx* c, const double* x, const double* v, const double* vold
     const size_t b = sizeof(double) * cnt;
     if (!c->stage) {
         CK(c, cudaMalloc((void**)&c->stage, 4 * b));
-        CK(c, cudaMalloc((void**)&c->nonfinite, sizeof(unsigned)));
+        CK(c, cudaMalloc((void**)&c->nonfinite, 2 * sizeof(unsigned long long)));   // and the distance moved
     }
     // The arrays are copied into a staging buffer and checked for NaN / Inf
     // on the device; only if all are finite does k_commit_state move them
     // into the state, so a rejected call leaves the state as it was.
     const double* src[4] = {x, v, vold, a};
     double* dst[4] = {c->x, c->v, c->vold, c->a};
-    CK(c, cudaMemsetAsync(c->nonfinite, 0, sizeof(unsigned), c->stream));
+    unsigned long long* moved = reinterpret_cast<unsigned long long*>(c->nonfinite) + 1;
+    CK(c, cudaMemsetAsync(c->nonfinite, 0, 2 * sizeof *moved, c->stream));
     int k = 0;
     for (int q = 0; q < 4; ++q) {
         if (!src[q]) continue;
@@ -1775,21 +1830,32 @@ int yk_set_state(yk_ctx* c, const double* x, const double* v, const double* vold
     }
     for (int q = 0; q < 4; ++q) {
         if (!src[q]) continue;
-        k_commit_state<<<(int)((cnt + 255) / 256), 256, 0, c->stream>>>(c->stage + q * cnt, dst[q], cnt,
-                                                                         c->nonfinite);
+        if (q == 0)
+            k_commit_positions<<<(c->n + 255) / 256, 256, 0, c->stream>>>(
+                c->stage, c->x, c->n, c->nonfinite, c->p.xl[0], c->p.xl[1], c->p.xl[2],
+                std::cbrt(c->n / (c->p.xl[0] * c->p.xl[1] * c->p.xl[2])), moved);
+        else
+            k_commit_state<<<(int)((cnt + 255) / 256), 256, 0, c->stream>>>(c->stage + q * cnt, dst[q], cnt,
+                                                                             c->nonfinite);
         ++k;
     }
-    unsigned bad = 0;
-    CK(c, cudaMemcpyAsync(c->h_err, c->nonfinite, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
+    unsigned long long* h = reinterpret_cast<unsigned long long*>(c->h_err);
+    CK(c, cudaMemcpyAsync(h, c->nonfinite, 2 * sizeof *h, cudaMemcpyDeviceToHost, c->stream));
     CK(c, cudaStreamSynchronize(c->stream));
-    bad = *c->h_err;
+    const bool bad = h[0] != 0;
+    const double dist = (double)h[1] / MOVED_UNIT / c->n;
     *c->h_err = 0;
     g_launches += k;
     if (bad) return fail(c, YK_ERR_NONFINITE, "NaN or Inf in a state array");
     // new positions keep the current slot order (the next scheduled sort
-    // refreshes it); the packed copies are rebuilt by the next call that
-    // reads them (a force call) or moves the positions first (a step)
-    if (x) c->pos_dirty = true;
+    // refreshes it) unless they are far from the old ones; the packed copies
+    // are rebuilt by the next call that reads them (a force call) or moves the
+    // positions first (a step)
+    if (x) {
+        c->pos_dirty = true;
+        c->moved += dist;
+        if (order_stale(c)) c->need_sort = true;
+    }
     return YK_OK;
 }
 
