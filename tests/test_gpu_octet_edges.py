@@ -104,3 +104,27 @@ def test_other_positions_get_their_own_order(gpu, orc, n, prec, calls):
         tol = 1e-12 if prec == abi.YK_PREC_FP64 else 1e-6
         assert np.linalg.norm(a[:3 * n] - a_ref[:3 * n]) <= tol * np.linalg.norm(a_ref[:3 * n])
         assert abs(ev - s_ref.ev) <= tol * abs(s_ref.ev)
+
+
+@pytest.mark.parametrize("n,cut", [(7168, 1e50), (7169, 1e50), (8704, 0.4), (8705, 0.4)])
+def test_sizes_around_the_wide_cutoffs_change(gpu, orc, n, cut):
+    """The FP64 sizes at which a box with a wide or no cutoff goes from every pair
+    from both sides to half pairs; a box that comes to such a cutoff by set_box."""
+    w = workload("mix", n, 800 + n)
+    L = w.params["xl"][0]
+    w.params["rccut"] = cut if cut > 1 else cut * L
+    check_accel(orc, w, abi.YK_PREC_FP64, True)
+    check_accel(orc, w, abi.YK_PREC_FP64, False)
+    p = w.yk_params()
+    wide = [t * 1.5 for t in w.params["xl"]]
+    p2 = w.yk_params(xl=wide)
+    x2 = np.ascontiguousarray(w.x * 1.5)
+    with Engine(p2, x2, w.v, w.zii, w.aii) as e:
+        e.accel(True)
+        e.set_box(w.params["xl"])
+        e.set_state(x=w.x)
+        s = e.accel(True)
+        a = e.a.copy()
+    with Engine(p, w.x, w.v, w.zii, w.aii) as e:
+        assert e.accel(True).ev == s.ev
+        assert np.linalg.norm(e.a - a) <= 1e-13 * np.linalg.norm(a)

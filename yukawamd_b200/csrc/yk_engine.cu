@@ -642,12 +642,19 @@ static bool octets_apply(const yk_ctx* c)
 }
 
 // Whether that is k_force_octets_all, every pair from both sides: half-pair
-// units of a small box are too few and too long to balance (FP64 step, before
-// / all pairs / half pairs: 500 ions 95 / 46 / 64 us; 3,000 61 / 42 / 75; 5,000
-// 100 / 89 / 109; 8,000 134 / 121 / 142; 10,000 155 / 150 / 145).
+// units of a small box are too few and too long to balance, while twice the
+// pairs cost the more the more of them are within the cutoff, measuring above
+// all.  FP64 step, force only and measuring, all pairs / half pairs: 6,000 ions
+// with r_c = 0.3 L 93 114 / 116 129 us, uncut 161 202 / 178 204; 8,000 at 0.3 L
+// 119 149 / 140 154, at 0.49 L 202 259 / 211 246, uncut 247 312 / 245 286; 9,216
+// at 0.2 L 103 126 / 112 123, at 0.3 L 142 175 / 146 164, at 0.4 L 189 241 / 189
+// 215, uncut 314 394 / 284 332.
 static bool octets_all(const yk_ctx* c)
 {
-    return c->n <= (c->p.precision == YK_PREC_FP64 ? OCT_ALL_MAX_N64 : OCT_ALL_MAX_N32);   // (all nucleon octets)
+    if (c->p.precision != YK_PREC_FP64) return c->n <= OCT_ALL_MAX_N32;      // (all nucleon octets)
+    const double Lmin = std::min(c->p.xl[0], std::min(c->p.xl[1], c->p.xl[2]));
+    if (c->p.rccut <= 0.35 * Lmin) return c->n <= OCT_ALL_MAX_N64;
+    return c->n <= (c->fa.img_k ? OCT_ALL_MAX_N64_WIDE : OCT_ALL_MAX_N64_UNCUT);
 }
 
 // Scratch of the octet kernels.
@@ -750,11 +757,12 @@ static int setup_or_rows(yk_ctx* c)
     return rc;
 }
 
-// A new box can change whether k_force_pairs2 applies (fa.img_k, fa.lo):
-// rebuild the job table when it does.
+// A new box can change whether k_force_pairs2 applies (fa.img_k, fa.lo) and which
+// octet kernel does: rebuild the job table when it does.
 static int refresh_pair_tt(yk_ctx* c)
 {
-    if (c->kernel == 2 && (pair_tt(c) != c->pj_tt || octets_apply(c) != c->oct)) {
+    if (c->kernel == 2 && (pair_tt(c) != c->pj_tt || octets_apply(c) != c->oct ||
+                           (c->oct && octets_all(c) != (c->oct_chunks != 0)))) {
         CK(c, cudaSetDevice(c->dev));
         CK(c, cudaStreamSynchronize(c->stream));
         return setup_or_rows(c);

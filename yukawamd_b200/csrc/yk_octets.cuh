@@ -1235,9 +1235,10 @@ inline int octet_all_len(int n, int n0 = 16)
     return len;
 }
 
-// Largest box that takes k_force_octets_all, by form (see the engine's
-// octets_apply).
-constexpr int OCT_ALL_MAX_N64 = 9216, OCT_ALL_MAX_N32 = 6144;
+// Largest box that takes k_force_octets_all, by form and for FP64 by cutoff (see
+// the engine's octets_all).
+constexpr int OCT_ALL_MAX_N64 = 9216, OCT_ALL_MAX_N64_WIDE = 8704, OCT_ALL_MAX_N64_UNCUT = 7168;
+constexpr int OCT_ALL_MAX_N32 = 6144;
 
 // posq etc. as OctetBox; part: target sums [chunk][slot][3], np slots; Sm: per job.
 template <class F, int SIM, bool MEAS, bool RANGE>
