@@ -56,6 +56,7 @@ using namespace yk;
 namespace {
 
 constexpr int BATCH_SEG = 8;
+constexpr size_t BATCH_SLACK = size_t(64) << 20;      // kept free beside a batch's arrays
 constexpr int BATCH_GRAPH_STEPS = 50;
 // Steps between the boxes' re-orderings inside a graph (each graph starts
 // with one): the single-box engine's cadence, for the same reason (the warp
@@ -73,7 +74,6 @@ struct RepDesc {
     int P;              // first particle unit (caller order)
     int S;              // first slot (multiple of 128)
     int T;              // tiles
-    int nseg;           // Si rows per target block
     long long Sj_off;   // values (row_t of the batch's form)
     long long Si_off;   // doubles
     long long A;        // first double of the box's a(3,0:n+2) = 3 P
@@ -213,6 +213,14 @@ k_b_post(const int2* __restrict__ vb, const RepDesc* __restrict__ rd, const int*
     if constexpr (KIN) block_sum_store<NKIN>(tk, red, kpart + (size_t)blockIdx.x * NKIN);
 }
 
+// Work items of target blocks that face 1, 2, .. T source tiles (a box of T
+// tiles), cut into segments of seg tiles.
+__host__ __device__ inline long long items_of(int T, int seg)
+{
+    const long long q = T / seg, r = T % seg;
+    return seg * q * (q + 1) / 2 + r * (q + 1);
+}
+
 // Whether a box takes the mixed hi/lo displacement (LO below): its own
 // property, so its results do not depend on the other boxes.
 __host__ __device__ inline bool box_lo(int sim, int prec, const ForceArgs& fa)
@@ -290,9 +298,9 @@ k_force_pairs_batch(const double4* __restrict__ pos, const float* __restrict__ p
         bx.Sjf = Sjf + d->Sj_off / (PB * 3);
         bx.n = sfa.n;
         bx.M = d->T;
-        bx.nseg_max = d->nseg;
+        bx.nseg_max = 0;                                 // the item's own row (jb.w)
         const int C0 = jb.y + jb.z * d->seg;
-        if (!pairs_job<SIM, PREC, MEAS, LO, TB>(sm, sfa, bx, jb.y, C0, min(C0 + d->seg, bx.M), jb.z,
+        if (!pairs_job<SIM, PREC, MEAS, LO, TB>(sm, sfa, bx, jb.y, C0, min(C0 + d->seg, bx.M), jb.w,
                                                 Sm + (size_t)(d->sm_off + jb.w) * NSCAL, err, q))
             return;
     }
@@ -322,7 +330,7 @@ k_b_combine(const int* __restrict__ tiles, const int* __restrict__ ntiles, const
         const int R = C - d->S / PB;
         const int nseg = (d->T - R + d->seg - 1) / d->seg;
         double F = 0.0;
-        const double* si = Si + d->Si_off + (size_t)R * d->nseg * ROW + t;
+        const double* si = Si + d->Si_off + (items_of(d->T, d->seg) - items_of(d->T - R, d->seg)) * ROW + t;
 #pragma unroll 4
         for (int s = g; s < nseg; s += COMB_GROUPS) F += si[(size_t)s * ROW];
         const row_t<PREC>* sj = Sj + d->Sj_off + (size_t)tri_index(R, 0) * ROW + t;
@@ -444,6 +452,7 @@ struct yk_batch {
     int ucap = 0, tcap = 0;         // particle units and tiles
     long long pair_cap = 0;         // half-pair units
     long long sj_cap = 0, si_cap = 0, sm_cap = 0, jobs_cap = 0;
+    int segs = 0;                   // least items for the longest row of a small box (box_seg)
     int cap_seg = 0;                // the shortest segment length si_cap / jobs_cap hold
     int vb_cap = 0;
     int dev = 0;
@@ -729,7 +738,6 @@ static int order_jobs(const std::vector<char>& lo, std::vector<int4>& jobs, cons
 }
 
 static long long units_of(int T) { return (long long)T * (T + 1) / 2; }
-static long long nseg_of(int T, int seg) { return (T + seg - 1) / seg; }
 
 // Source tiles per work item of a box of T tiles: at most seg, and at least
 // BOX_SEGS items for the longest row of a small box, whose few long items
@@ -739,28 +747,81 @@ static long long nseg_of(int T, int seg) { return (T + seg - 1) / seg; }
 // 1,000 to 20,000 62.1 / 51.0 / 52.8.
 constexpr int BOX_SEGS = 16;
 
-static int box_seg(int T, int seg) { return std::max(1, std::min(seg, (T + BOX_SEGS - 1) / BOX_SEGS)); }
+// (segs: BOX_SEGS, or 1 in a batch without the memory for the items' rows.)
+static int box_seg(int T, int seg, int segs) { return std::max(1, std::min(seg, (T + segs - 1) / segs)); }
 
-// Si rows and jobs that boxes of at most `units` half-pair units on at most
-// `tiles` tiles can need with segments of up to `seg` tiles: a box of T tiles
-// takes T ceil(T / box_seg) of each at most: T ceil(T / seg) <= T^2 / seg + T <=
-// 2 units / seg + T, or T BOX_SEGS.
-static long long jobs_bound(long long units, long long tiles, int seg)
+// Items (each with a row of Si) that boxes of at most `units` half-pair units on
+// at most `tiles` tiles can need with segments of up to `seg` tiles.  An item
+// takes one unit or more.  With segments of s tiles a box of T takes at most
+// T (T + 1) / 2s + T (s - 1) / s items: units / seg + T for s = seg, and with s =
+// ceil(T / segs) < seg, T <= segs s, at most T (segs / 2 + 1).
+static long long jobs_bound(long long units, long long tiles, int seg, int segs)
 {
-    return 2 * units / seg + (BOX_SEGS + 2) * tiles;
+    return std::min(units, units / seg + (segs / 2 + 1) * tiles);
 }
 
-// Si, Sm and the job tables sized for segment length seg.
+static size_t job_bytes(long long jobs)
+{
+    return (size_t)jobs * (sizeof(double) * (PB * 3 + NSCAL) + 2 * sizeof(int4));
+}
+
+// Batches are created and destroyed often (the serving loop creates one per
+// group), so their device arrays come from the device's stream-ordered memory
+// pool, which keeps up to POOL_KEEP bytes of freed memory cached between
+// batches.
+constexpr uint64_t POOL_KEEP = 8ull << 30;
+
+static void pool_setup(int dev)
+{
+    static std::mutex mu;
+    static std::vector<int> done;
+    std::lock_guard<std::mutex> lk(mu);
+    if (std::find(done.begin(), done.end(), dev) != done.end()) return;
+    cudaMemPool_t pool;
+    if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
+        uint64_t keep = POOL_KEEP;
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    }
+    done.push_back(dev);
+}
+
+// Bytes the pool holds cached but unused (free for the next batch).
+static size_t pool_cached(int dev)
+{
+    cudaMemPool_t pool;
+    uint64_t reserved = 0, used = 0;
+    if (cudaDeviceGetDefaultMemPool(&pool, dev) != cudaSuccess) return 0;
+    cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved);
+    cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used);
+    return reserved > used ? (size_t)(reserved - used) : 0;
+}
+
+// Bytes that a batch can still take on the current device.
+static size_t free_bytes(int dev)
+{
+    size_t free_b = 0, total_b = 0;
+    cudaMemGetInfo(&free_b, &total_b);
+    return free_b + pool_cached(dev);
+}
+
+// Si, Sm and the job tables sized for segment length seg.  A batch whose items
+// of small boxes would not fit beside what it holds takes whole segments.
 static int alloc_job_scratch(yk_batch* b, int seg)
 {
-    const long long jb = jobs_bound(b->pair_cap, b->tcap, seg);
     cudaStream_t st = b->stream;
     cudaFreeAsync(b->Si, st);
     cudaFreeAsync(b->Sm, st);
     cudaFreeAsync(b->jobs, st);
     cudaFreeAsync(b->jobs_sel, st);
+    cudaStreamSynchronize(st);
     b->Si = b->Sm = nullptr;
     b->jobs = b->jobs_sel = nullptr;
+    b->segs = BOX_SEGS;
+    long long jb = jobs_bound(b->pair_cap, b->tcap, seg, b->segs);
+    if (job_bytes(jb) + BATCH_SLACK > free_bytes(b->dev)) {
+        b->segs = 1;
+        jb = jobs_bound(b->pair_cap, b->tcap, seg, b->segs);
+    }
     b->si_cap = jb * PB * 3;
     b->jobs_cap = jb;
     b->sm_cap = NSCAL * jb;
@@ -797,8 +858,7 @@ static int relayout(yk_batch* b, int seg, const std::vector<char>& newsel)
         }
         ++held;
         d.active = 1;
-        d.seg = box_seg(d.T, seg);
-        d.nseg = (int)nseg_of(d.T, d.seg);
+        d.seg = box_seg(d.T, seg, b->segs);
         d.Sj_off = sj;
         d.Si_off = si;
         d.sm_off = smo;
@@ -815,7 +875,7 @@ static int relayout(yk_batch* b, int seg, const std::vector<char>& newsel)
             selv[r] = 1;
         }
         sj += units_of(d.T) * PB * 3;
-        si += (long long)d.T * d.nseg * PB * 3;
+        si += (long long)d.njobs * PB * 3;
         smo += d.njobs;
         const int nb = (d.fa.n + VBLOCK - 1) / VBLOCK;
         d.kb0 = (int)vblocks.size();
@@ -1000,37 +1060,6 @@ extern "C" {
 
 const char* yk_batch_last_error(const yk_batch* b) { return b ? b->errmsg.c_str() : g_batch_err.c_str(); }
 
-// Batches are created and destroyed often (the serving loop creates one per
-// group), so their device arrays come from the device's stream-ordered memory
-// pool, which keeps up to POOL_KEEP bytes of freed memory cached between
-// batches.
-constexpr uint64_t POOL_KEEP = 8ull << 30;
-
-static void pool_setup(int dev)
-{
-    static std::mutex mu;
-    static std::vector<int> done;
-    std::lock_guard<std::mutex> lk(mu);
-    if (std::find(done.begin(), done.end(), dev) != done.end()) return;
-    cudaMemPool_t pool;
-    if (cudaDeviceGetDefaultMemPool(&pool, dev) == cudaSuccess) {
-        uint64_t keep = POOL_KEEP;
-        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    }
-    done.push_back(dev);
-}
-
-// Bytes the pool holds cached but unused (free for the next batch).
-static size_t pool_cached(int dev)
-{
-    cudaMemPool_t pool;
-    uint64_t reserved = 0, used = 0;
-    if (cudaDeviceGetDefaultMemPool(&pool, dev) != cudaSuccess) return 0;
-    cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved);
-    cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used);
-    return reserved > used ? (size_t)(reserved - used) : 0;
-}
-
 int yk_batch_get_tuning(yk_batch* b, yk_tuning* out)
 {
     if (!b || !out) return bfail(b, YK_ERR_ARG, "batch and out are required");
@@ -1113,7 +1142,7 @@ static int create_empty(int sim, int prec_api, int nslots, long long max_units, 
     b->tcap = (int)max_tiles;
     b->pair_cap = max_pair_units;
     b->sj_cap = max_pair_units * PB * 3;
-    const long long jb = jobs_bound(max_pair_units, max_tiles, BATCH_SEG);
+    const long long jb = jobs_bound(max_pair_units, max_tiles, BATCH_SEG, 1);     // (alloc_job_scratch takes more if it can)
     b->vb_cap = (int)(max_units / VBLOCK + nslots);
     b->dev = device;
     b->sim = sim;
@@ -1134,15 +1163,13 @@ static int create_empty(int sim, int prec_api, int nslots, long long max_units, 
                                              (int*)nullptr, 0, b->key_bits);
     const long long U = max_units, S = max_tiles * PB;
     const size_t sj_elem = b->prec == PREC_MIXED ? sizeof(float) : sizeof(double);
-    const size_t need = sj_elem * (size_t)b->sj_cap + sizeof(double) * (size_t)(14 * U + jb * PB * 3 + NSCAL * jb +
-                                                  (long long)NKIN * b->vb_cap) +
-                        sizeof(double4) * S + sizeof(float) * (SHADOW_FLOATS / SHADOW_TILE) * S +
-                        sizeof(int) * (4 * U + S + 2 * max_tiles) + sizeof(float) * 8 * max_tiles + (size_t)max_pair_units + sizeof(unsigned) * 2 * U + cub_bytes +
-                        sizeof(RepDesc) * nslots + sizeof(int4) * 2 * jb + (64u << 20);
-    size_t free_b = 0, total_b = 0;
+    const size_t need = sj_elem * (size_t)b->sj_cap + job_bytes(jb) +
+                        sizeof(double) * (size_t)(14 * U + (long long)NKIN * b->vb_cap) + sizeof(double4) * S +
+                        sizeof(float) * (SHADOW_FLOATS / SHADOW_TILE) * S + sizeof(int) * (4 * U + S + 2 * max_tiles) +
+                        sizeof(float) * 8 * max_tiles + (size_t)max_pair_units + sizeof(unsigned) * 2 * U + cub_bytes +
+                        sizeof(RepDesc) * nslots + BATCH_SLACK;
     pool_setup(device);
-    cudaMemGetInfo(&free_b, &total_b);
-    free_b += pool_cached(device);
+    const size_t free_b = free_bytes(device);
     if (need > free_b) {
         delete b;
         return bfail(nullptr, YK_ERR_NOMEM, "batch needs %zu bytes, %zu free", need, free_b);

@@ -55,8 +55,10 @@ PARTICLE_BYTES = 300
 def unit_bytes(precision=abi.YK_PREC_FP64):
     """Device bytes per half-pair unit of reserved scratch: the source-side
     row (128 x 3 values: doubles in the FP64 form, floats in the mixed form)
-    plus the target-side rows (doubles) and job entries at the default
-    segment length (a quarter of a double row at most) and slack."""
+    plus a quarter of a double row and slack for the target-side rows (doubles)
+    and job entries.  The engine reserves an eighth of a row per unit at the
+    default segment length and nine rows per 128 particles, at most one per
+    unit; a group has many units per particle, so it stays within its budget."""
     sj = 3 * PB * (4 if precision == abi.YK_PREC_MIXED else 8)
     return sj + 3 * PB * 8 // 4 + 64
 
