@@ -352,10 +352,7 @@ def time_engine(w, precision, steps, warmup, meas_every, dist, flush=True, sampl
     e = Engine(w, precision=prec, device=dist.local)
     if KERNEL_CHOICE[0]:
         e.set_tuning(force_kernel=KERNEL_CHOICE[0])
-    t = e.tuning()
-    e.kernel_name = {1: "k_force_rows", 2: "half-pair force kernel (k_force_octets or k_force_pairs)", 3: "k_force_near"}.get(t.force_kernel, "?")
-    if t.force_kernel == 2 and t.targets_per_thread == 2:
-        e.kernel_name = "k_force_pairs2"
+    e.kernel_name = e.force_kernel()
     e.accel(True)                                  # md.F:69, initial forces
     if warmup:
         e.run(warmup, meas_every, series=False)

@@ -338,6 +338,14 @@ typedef struct yk_tuning {
 YK_API int yk_get_tuning(yk_ctx* ctx, yk_tuning* out);
 YK_API int yk_set_tuning(yk_ctx* ctx, const yk_tuning* t);
 
+/* Name of the kernel that a force call of ctx runs: k_force_rows,
+ * k_force_near, k_force_pairs, k_force_pairs2 (two targets per thread),
+ * k_force_octets (half pairs), k_force_octets_all (every pair from both
+ * sides), or "" for 'B-field'.  automatic != 0: the one that automatic tuning
+ * would run.  Static string; NULL if ctx is NULL.  No counterpart in the
+ * reference. */
+YK_API const char* yk_force_kernel(const yk_ctx* ctx, int automatic);
+
 /* The batch's tunables: pair_seg (source tiles per job, all boxes) and
  * graph_steps (steps per CUDA graph of yk_batch_run) and sort_every (steps
  * between the boxes' Hilbert re-orderings, counted from the start of each

@@ -55,6 +55,7 @@ SIGNATURES = {
     "yk_batch_steps_left": (C.c_int, [_ctx, C.POINTER(C.c_int)]),
     "yk_get_tuning": (C.c_int, [_ctx, C.POINTER(abi.YkTuning)]),
     "yk_set_tuning": (C.c_int, [_ctx, C.POINTER(abi.YkTuning)]),
+    "yk_force_kernel": (C.c_char_p, [_ctx, C.c_int]),
     "yk_perf_enable": (C.c_int, [_ctx, C.c_int, C.c_size_t]),
     "yk_perf_read": (C.c_int, [_ctx, C.POINTER(abi.YkPerf)]),
     "yk_peak_probe": (C.c_int, [C.c_int, C.c_int, C.POINTER(C.c_double)]),

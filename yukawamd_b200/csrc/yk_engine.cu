@@ -1535,6 +1535,32 @@ int yk_set_tuning(yk_ctx* c, const yk_tuning* t)
     return YK_OK;
 }
 
+const char* yk_force_kernel(const yk_ctx* c, int automatic)
+{
+    if (!c) return nullptr;
+    if (c->p.sim_type == YK_SIM_BFIELD) return "";
+    yk_ctx t;                                // what the choice depends on
+    t.p = c->p;
+    t.fa = c->fa;
+    t.n = c->n;
+    t.dev = c->dev;
+    t.sms = c->sms;
+    t.split = c->split;
+    t.seg = c->seg;
+    t.kernel_req = c->kernel_req;
+    t.tpt_req = c->tpt_req;
+    t.kernel = c->kernel;
+    if (automatic) {
+        t.kernel_req = t.tpt_req = 0;
+        t.split = 1;
+        t.seg = auto_pair_seg(&t);
+        t.kernel = half_pair_bytes(&t) <= PAIR_SCRATCH_BUDGET ? 2 : 1;
+    }
+    if (t.kernel != 2) return t.kernel == 1 ? "k_force_rows" : "k_force_near";
+    if (octets_apply(&t)) return octets_all(&t) ? "k_force_octets_all" : "k_force_octets";
+    return pair_tt(&t) == 2 ? "k_force_pairs2" : "k_force_pairs";
+}
+
 int yk_accel(yk_ctx* c, int do_meas, double* a_out, yk_scalars* out)
 {
     if (!c) return fail(nullptr, YK_ERR_ARG, "ctx is NULL");

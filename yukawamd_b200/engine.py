@@ -182,6 +182,11 @@ class Engine:
         check(self._lib.yk_set_tuning(self._ctx, C.byref(t)), self._ctx)
         return self.tuning()
 
+    def force_kernel(self, automatic=False):
+        """Name of the kernel that a force call runs (automatic: that it would
+        run under automatic tuning)."""
+        return self._lib.yk_force_kernel(self._ctx, int(bool(automatic))).decode()
+
     # -- timers (the reference's perf.f newton / accel timers) --------------
     def perf_enable(self, enable=True, flush_bytes=0):
         check(self._lib.yk_perf_enable(self._ctx, int(bool(enable)), int(flush_bytes)),
