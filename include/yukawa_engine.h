@@ -346,13 +346,17 @@ YK_API int yk_set_tuning(yk_ctx* ctx, const yk_tuning* t);
  * reference. */
 YK_API const char* yk_force_kernel(const yk_ctx* ctx, int automatic);
 
-/* The batch's tunables: pair_seg (source tiles per job, all boxes) and
- * graph_steps (steps per CUDA graph of yk_batch_run) and sort_every (steps
+/* The batch's tunables: pair_seg (most source tiles per work item; a small box
+ * takes fewer, so that its longest row still makes 16 items), graph_steps (steps per CUDA graph of yk_batch_run) and sort_every (steps
  * between the boxes' Hilbert re-orderings, counted from the start of each
  * graph, which always re-sorts; 0 = automatic: 4).  force_kernel must be 0
  * or 2.  Changing pair_seg rebuilds the job table and its scratch. */
 YK_API int yk_batch_get_tuning(yk_batch* b, yk_tuning* out);
 YK_API int yk_batch_set_tuning(yk_batch* b, const yk_tuning* t);
+
+/* Work items of the held boxes under the present cut; -YK_ERR_ARG if b is NULL.
+ * Two values of pair_seg with the same number of items cut the boxes alike. */
+YK_API int yk_batch_work_items(const yk_batch* b);
 
 /*
  * Timers, the counterpart of the reference's perf.f report (perf.f:60-178:

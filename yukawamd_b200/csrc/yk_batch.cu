@@ -1097,6 +1097,8 @@ int yk_batch_set_tuning(yk_batch* b, const yk_tuning* t)
     return relayout(b, seg, {});
 }
 
+int yk_batch_work_items(const yk_batch* b) { return b ? b->njobs : -YK_ERR_ARG; }
+
 int yk_batch_destroy(yk_batch* b)
 {
     if (!b) return bfail(nullptr, YK_ERR_ARG, "batch is NULL");

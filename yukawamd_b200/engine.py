@@ -268,6 +268,10 @@ class Batch:
         check_batch(self._lib.yk_batch_set_tuning(self._b, C.byref(t)), self._b)
         return self.tuning()
 
+    def work_items(self):
+        """Work items of the held boxes under the present cut."""
+        return int(self._lib.yk_batch_work_items(self._b))
+
     def accel(self, do_measurements=True):
         out = (abi.YkScalars * self.nrep)()
         check_batch(self._lib.yk_batch_accel(self._b, int(bool(do_measurements)), out), self._b)

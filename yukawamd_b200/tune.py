@@ -10,12 +10,16 @@ target, for small boxes), give each thread one or two targets
 the ion kernels); it refreshes
 the Hilbert order every `sort_every` steps.  Which choice is fastest depends on
 N, the cutoff radius relative to the box, the interaction and the precision,
-so the tuner measures candidates on the caller's own workload (CUDA-event
+so the tuner measures the candidates that differ on the caller's own workload
+(an ion box on the octet kernels, whose jobs are cut by cost, takes the same
+kernel whatever `pair_seg` and `source_split` say; CUDA-event
 time per step, sorts included, yk_perf, over a window of 16 steps: the force
 call slows down step by step after a sort as particles leave their
 neighbours, which a shorter window would not see) and remembers the winner per
 
-    (GPU name, sim type, precision, N bucket)      N bucket = round(2 log2 N)
+    (kernel revision, GPU name, sim type, precision, N bucket, automatic kernel)
+
+    N bucket = round(2 log2 N); automatic kernel = Engine.force_kernel(True)
 
 in a JSON cache (default ~/.cache/yukawamd_b200/tune.json, or $YK_TUNE_CACHE).
 Engine.autotune() / tune.apply(engine) use it transparently.
@@ -26,6 +30,10 @@ import os
 import time
 
 from . import abi
+
+# Raised when the kernels or the sizes at which they take over change: a winner
+# among other kernels (its entry has another key) is not applied.
+REVISION = 2
 
 # sort_every 0 is the engine's automatic cadence (4 steps)
 CANDIDATES = [
@@ -95,7 +103,18 @@ def bucket(n):
 
 def key_for(engine, device=0):
     p = engine.params
-    return "%s|sim%d|prec%d|nb%d" % (gpu_name(device), p.sim_type, p.precision, bucket(engine.n))
+    return "r%d|%s|sim%d|prec%d|nb%d|%s" % (REVISION, gpu_name(device), p.sim_type, p.precision, bucket(engine.n),
+                                            engine.force_kernel(automatic=True))
+
+
+def effective(engine):
+    """What the engine's tuning comes to: the kernel and the values that it
+    takes notice of (the others only have a meaning for other kernels)."""
+    t = engine.tuning()
+    kern = engine.force_kernel()
+    seg = t.pair_seg if kern in ("k_force_pairs", "k_force_pairs2", "k_force_near") else 0
+    split = t.source_split if kern == "k_force_pairs" else 1
+    return kern, (1 if split > 1 else seg), split, t.sort_every
 
 
 def measure(engine, cand, steps=16, warmup=2):
@@ -112,21 +131,28 @@ def measure(engine, cand, steps=16, warmup=2):
 
 
 def tune(engine, candidates=None, steps=16, warmup=2, device=0, save=True):
-    """Time every candidate on this engine's workload; apply and return the
-    one with the shortest step (the result's ms) and the list of (step ms,
-    candidate, error or None, force-call ms).  The engine's positions are
+    """Time every candidate on this engine's workload (those that come to the
+    same share one timing); apply and return the one with the shortest step
+    (the result's ms) and the list of (step ms, candidate, error or None,
+    force-call ms).  The engine's positions are
     restored afterwards, so tuning does not advance the caller's
     trajectory."""
     candidates = candidates or [c for c in CANDIDATES
                                 if c.get("source_split", 1) == 1 or engine.n <= SPLIT_MAX_N]
     x, v, vold, a = engine.get_state()
     results = []
+    timed = {}
     for cand in candidates:
         cand = dict(cand)
         cand.setdefault("source_split", 1)
         cand.setdefault("targets_per_thread", 1)
         try:
-            ms, fms = measure(engine, cand, steps, warmup)
+            engine.set_tuning(**cand)
+            eff = effective(engine)
+            if eff in timed:
+                results.append((timed[eff][0], cand, None, timed[eff][1]))
+                continue
+            ms, fms = timed[eff] = measure(engine, cand, steps, warmup)
         except Exception as exc:          # e.g. scratch too large for this N
             results.append((float("inf"), cand, str(exc), float("inf")))
             continue
@@ -149,25 +175,32 @@ BATCH_SEGS = (8, 4, 16, 2, 32)
 def batch_key(batch, device=0):
     import numpy as np
     p = batch.params[0]
-    return "%s|batch|sim%d|prec%d|nrep%d|nb%d" % (gpu_name(device), p.sim_type, p.precision, batch.nrep,
-                                                  bucket(int(np.sqrt(np.mean(np.square(batch.n))))))
+    return "r%d|%s|batch|sim%d|prec%d|nrep%d|nb%d" % (REVISION, gpu_name(device), p.sim_type, p.precision, batch.nrep,
+                                                      bucket(int(np.sqrt(np.mean(np.square(batch.n))))))
 
 
 def tune_batch(batch, segs=BATCH_SEGS, steps=50, device=0, save=True):
     """Time one graph of `steps` steps of the whole batch for every job
-    segment length (source tiles per work item) and keep the fastest.  The
-    boxes' states are restored afterwards.  Cached per (GPU, sim, precision,
-    box count, RMS box size bucket)."""
+    segment length (most source tiles per work item; lengths that cut the boxes
+    alike share one timing) and keep the fastest, the first named of equals.
+    The boxes' states are restored afterwards.  Cached per (kernel revision,
+    GPU, sim, precision, box count, RMS box size bucket)."""
     states = [batch.get_state(r) for r in range(batch.nrep)]
     results = []
+    timed = {}
     for seg in segs:
         batch.set_tuning(pair_seg=seg, graph_steps=steps)
+        items = batch.work_items()
+        if items in timed:
+            results.append((timed[items], seg))
+            continue
         batch.run(steps, 0, series=False)                  # capture + warm
         _, ms = batch.run(steps, 0, series=False)
+        timed[items] = ms
         results.append((ms, seg))
         for r, (x, v, vold, a) in enumerate(states):
             batch.set_state(r, x=x, v=v, vold=vold, a=a)
-    best_ms, best = min(results)
+    best_ms, best = min(results, key=lambda r: r[0])
     batch.set_tuning(pair_seg=best, graph_steps=steps)
     if save:
         doc = _load()
