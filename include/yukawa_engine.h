@@ -439,6 +439,13 @@ YK_API int yk_accel_noalloc(const yk_params* p, int n,
  * the check itself. */
 YK_API int yk_wait_selftest(yk_ctx* ctx, long long spins, int* gave_up);
 
+/* The FP64 pair arithmetic on its own, for tests: out[i] = f(in[i]) on device
+ * `device`, host arrays of n values.  what: 0 the hardware's estimate of
+ * 1/sqrt(x) for x > 0, 1 the octet kernels' 1/sqrt(x), 2 their e^{-t} for t >= 0,
+ * 3 and 4 the other kernels' 1/sqrt(x) and e^{-t}.  No counterpart in the
+ * reference. */
+YK_API int yk_math_selftest(int device, int what, int n, const double* in, double* out);
+
 /* Page-lock a caller-owned host buffer so that yk_get_state / yk_set_state
  * copy it by DMA.  Optional. */
 YK_API int yk_host_register(void* ptr, size_t bytes);

@@ -136,6 +136,21 @@ __global__ void __launch_bounds__(128) k_wait_selftest(long long spins, unsigned
     if (threadIdx.x == 0) out[0] = gave_up;
 }
 
+// The FP64 pair arithmetic of the force kernels on its own (yk_math_selftest): one
+// value per thread, whole warps.
+__global__ void k_math_selftest(int what, int n, const double* __restrict__ in, double* __restrict__ out)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const double v[1] = {in[min(i, n - 1)]};
+    double r[1], s[1];
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r[0]) : "d"(v[0]));
+    if (what == 1) rsqrt_h64_step<1>(v, r);
+    if (what == 2) exp_neg_f64_warp<true, 1>(v, exp2_32_lane(), s, r);
+    if (what == 3) r[0] = rsqrt_nr64(v[0]);
+    if (what == 4) r[0] = exp_neg_f64<true>(v[0]);
+    if (i < n) out[i] = r[0];
+}
+
 // Largest scratch the half-pair kernel may take before auto mode falls back
 // to the scratch-free row kernel.
 constexpr size_t PAIR_SCRATCH_BUDGET = size_t(8) << 30;
@@ -2100,6 +2115,23 @@ int yk_wait_selftest(yk_ctx* c, long long spins, int* gave_up)
     const int rc = sync_and_check(c);
     if (gave_up) *gave_up = h;
     return rc;
+}
+
+int yk_math_selftest(int device, int what, int n, const double* in, double* out)
+{
+    if (!in || !out || n < 1 || what < 0 || what > 4) return fail(nullptr, YK_ERR_ARG, "bad self-test arguments");
+    CK(nullptr, cudaSetDevice(device));
+    double* d = nullptr;
+    CK(nullptr, cudaMalloc((void**)&d, 2 * sizeof(double) * (size_t)n));
+    cudaError_t e = cudaMemcpy(d, in, sizeof(double) * (size_t)n, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        k_math_selftest<<<(n + 127) / 128, 128>>>(what, n, d, d + n);
+        g_launches += 1;
+        e = cudaMemcpy(out, d + n, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost);
+    }
+    cudaFree(d);
+    if (e != cudaSuccess) return fail(nullptr, YK_ERR_CUDA, "self-test: %s", cudaGetErrorString(e));
+    return YK_OK;
 }
 
 int yk_host_register(void* ptr, size_t bytes)

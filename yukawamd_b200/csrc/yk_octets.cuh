@@ -50,7 +50,8 @@ constexpr double OCT_FAR = 1e160;         // its coordinates: r^2 overflows, no 
 // (which takes the index mod 32), so every lane of the warp must call this
 // together.  The high word of the lane's entry is stored less l << 15: adding
 // (32 m + j) << 15 to it then puts m into the exponent in one integer
-// operation.  Two FP64 FMAs more than the 256-entry table, but the lookup
+// operation.  At most 1.01 ulp off (0.333 on average, t = 0 .. 690), exp_neg_f64
+// 1.31 (0.343).  Two FP64 FMAs more than the 256-entry table, but the lookup
 // takes 2 shuffle cycles of an SM instead of a divergent load from a 2 KB
 // table (about 4 cycles and a global-load latency).
 __device__ __forceinline__ double exp2_32_lane()
@@ -104,9 +105,11 @@ __device__ __forceinline__ void exp_neg_f64_warp(const double (&t)[NQ], double t
 
 // y = 1/sqrt(x) from the hardware's FP64 estimate (rsqrt.approx.ftz.f64), one
 // second-order correction as rsqrt_nr64.  The estimate's relative error is
-// 2^-20 (measured over 2^-48 .. 2^50), so the dropped third-order term
-// 5 e^3 / 16 is below 2^-60; it is one instruction in place of two conversions
-// and an FP32 estimate (2.0 against 6.3 cycles of an SM per warp).
+// below 2^-20 (2^-20.05 measured over 2^-1000 .. 2^1000), so e is below 2^-19 and
+// the dropped third-order term 5 e^3 / 16 below 2^-58.6, 0.02 ulp: measured over
+// r^2 from 1e-6 to 1e12, 0.990 ulp at most and 0.278 on average against 0.986 and
+// 0.278 of rsqrt_nr64.  It is one instruction in place of two conversions and
+// an FP32 estimate (2.0 against 6.3 cycles of an SM per warp).
 template <int NQ>
 __device__ __forceinline__ void rsqrt_h64_step(const double (&x)[NQ], double (&y)[NQ])
 {
