@@ -128,3 +128,35 @@ def test_sizes_around_the_wide_cutoffs_change(gpu, orc, n, cut):
     with Engine(p, w.x, w.v, w.zii, w.aii) as e:
         assert e.accel(True).ev == s.ev
         assert np.linalg.norm(e.a - a) <= 1e-13 * np.linalg.norm(a)
+
+
+@pytest.mark.parametrize("kind,n,prec", [("pure", 349, abi.YK_PREC_FP64), ("pure", 349, abi.YK_PREC_MIXED),
+                                         ("mix", 9500, abi.YK_PREC_FP64), ("mix", 24700, abi.YK_PREC_MIXED),
+                                         ("nn", 700, abi.YK_PREC_FP64), ("nn", 700, abi.YK_PREC_MIXED)])
+def test_coincident_particles_stay_by_themselves(gpu, orc, kind, n, prec):
+    """Two particles in one place get no finite force and, a step later, no finite
+    position.  The others do not notice them, as in the oracle."""
+    w = workload(kind, n, 30 + n)
+    m = int(np.ceil(n ** (1 / 3)))                     # apart from each other: a jittered lattice
+    rng = np.random.default_rng(n)
+    c = rng.permutation(m ** 3)[:n]
+    x = (np.stack([c // (m * m), c // m % m, c % m], axis=1) + 0.5 + 0.2 * (rng.random((n, 3)) - 0.5)) / m
+    if kind == "nn":
+        w.zii[:2] = w.zii[n // 2] = 1.0
+    else:
+        w.params["rccut"] = 0.3 * w.params["xl"][0]
+    x[n // 2] = x[1]
+    w.x = np.ascontiguousarray((x * np.array(w.params["xl"])).reshape(-1))
+    p = w.yk_params(precision=prec)
+    xr, vr, vo = w.x.copy(), w.v.copy(), np.zeros(3 * n)
+    ar, sr = orc.accel(p, xr, w.zii, w.aii, True)
+    with Engine(p, w.x, w.v, w.zii, w.aii) as e:
+        assert e.force_kernel().startswith("k_force_octets")
+        e.accel(True)
+        for step in range(3):
+            e.newton(step == 1)
+            orc.newton(p, xr, vr, vo, ar, w.zii, w.aii, step == 1, sr)
+            gx = e.get_state()[0]
+            lost = ~np.isfinite(xr)
+            assert lost.sum() == 6
+            assert np.array_equal(~np.isfinite(gx), lost), step

@@ -502,7 +502,10 @@ struct OctetBox {
     int n, M;
 };
 
-// One CTA of PB threads per tile.  GATHER: after a drift, the slots' positions
+// One CTA of PB threads per tile.  A particle without a finite position counts as
+// none: beyond every cutoff and, should there be others, beyond them too (the
+// reference's r <= r_c is false for it; a zero factor times its distance would
+// be NaN in every sum that it shares).  GATHER: after a drift, the slots' positions
 // (pos) are gathered from the caller's order here (k_pack_slots' part; the FP32
 // shadow is not written, no octet kernel reads it).
 template <class F, bool GATHER>
@@ -514,7 +517,7 @@ k_octet_pack(double4* __restrict__ pos, int n, ForceArgs fa, float4* __restrict_
     __shared__ float red[PWARPS][6];
     const int C = blockIdx.x, j = threadIdx.x, lane = j & 31, warp = j >> 5;
     const int i = C * PB + j;
-    const bool on = i < n;
+    bool on = i < n;
     double4 p = make_double4(OCT_FAR, OCT_FAR, OCT_FAR, 0.0);
     if (on) {
         if constexpr (GATHER) {
@@ -523,6 +526,11 @@ k_octet_pack(double4* __restrict__ pos, int n, ForceArgs fa, float4* __restrict_
             pos[i] = p;
         } else {
             p = pos[i];
+        }
+        on = isfinite(p.x) && isfinite(p.y) && isfinite(p.z);
+        if (!on) {
+            const double far = OCT_FAR * (2.0 + i);
+            p = make_double4(far, far, far, 0.0);
         }
     }
     F::pack(posq + (size_t)C * OCT_UNITS, j, p, on);

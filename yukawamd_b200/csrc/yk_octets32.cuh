@@ -342,7 +342,7 @@ struct Form32 {
 
     static __device__ __forceinline__ void tile_ready(const float4*, Extra&, int, int) {}
 
-    static __device__ __forceinline__ Target target(const float4* __restrict__ posq, int R, int s, bool on)
+    static __device__ __forceinline__ Target target(const float4* __restrict__ posq, int R, int s, bool)
     {
         const float* t = reinterpret_cast<const float*>(posq + (size_t)R * OCT_UNITS) + 4 * (s >> 1) + (s & 1);
         Target r;
@@ -350,7 +350,8 @@ struct Form32 {
         r.h[1] = -t[2];
         r.h[2] = -t[4 * SEC];
         r.w = t[4 * SEC + 2];
-        r.l[0] = on ? -t[8 * SEC] : OCT_FAR32;      // no target: far from every source, the empty slots' too
+        // no target: far from every source, the empty slots' too
+        r.l[0] = t[8 * SEC] == OCT_FAR32 ? OCT_FAR32 : -t[8 * SEC];
         r.l[1] = -t[8 * SEC + 2];
         r.l[2] = -t[12 * SEC];
         return r;
