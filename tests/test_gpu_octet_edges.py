@@ -160,3 +160,15 @@ def test_coincident_particles_stay_by_themselves(gpu, orc, kind, n, prec):
             lost = ~np.isfinite(xr)
             assert lost.sum() == 6
             assert np.array_equal(~np.isfinite(gx), lost), step
+
+
+@pytest.mark.parametrize("kind,n", [("pure", 7), ("pure", 300), ("nn", 300)])
+def test_negative_screening(gpu, orc, kind, n):
+    """xmuc < 0 is accepted: e^{-mu r} grows, and the FP64 form follows it (the
+    mixed form stays off the octets, whose far-away pads would count)."""
+    w = workload(kind, n, 17 + n)
+    w.params["xmuc"] = -0.3 / w.params["xl"][0]
+    w.params["rccut"] = 0.3 * w.params["xl"][0]
+    check_accel(orc, w, abi.YK_PREC_FP64, True)
+    with Engine(w, precision=abi.YK_PREC_MIXED) as e:
+        assert e.force_kernel() == "k_force_pairs"

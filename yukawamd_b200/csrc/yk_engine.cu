@@ -650,6 +650,8 @@ static void free_pairs(yk_ctx* c)
 static bool octets_apply(const yk_ctx* c)
 {
     if (c->kernel_req == 3 || pair_tt(c) != 1) return false;
+    // (the mixed form's masked pairs rely on e^{-mu r} vanishing far away)
+    if (c->p.precision != YK_PREC_FP64 && !(c->p.xmuc >= 0.0)) return false;
     if (c->p.sim_type == YK_SIM_NUCLEON)
         return c->p.precision == YK_PREC_FP64 ? c->n <= OCT_NN_MAX_N64 : c->n <= OCT_NN_MAX_N32 && c->fa.hilo;
     if (c->p.precision == YK_PREC_FP64) return true;
