@@ -295,7 +295,7 @@ k_force_pairs_batch(const double4* __restrict__ pos, const float* __restrict__ p
         bx.Si = Si + d->Si_off;
         bx.Sj = Sj + d->Sj_off;
         bx.tbox = TB ? tbox + 8 * (size_t)(d->S / PB) : nullptr;
-        bx.Sjf = Sjf + d->Sj_off / (PB * 3);
+        bx.Sjf = TB ? Sjf + d->Sj_off / (PB * 3) : nullptr;
         bx.n = sfa.n;
         bx.M = d->T;
         bx.nseg_max = 0;                                 // the item's own row (jb.w)
@@ -334,21 +334,26 @@ k_b_combine(const int* __restrict__ tiles, const int* __restrict__ ntiles, const
 #pragma unroll 4
         for (int s = g; s < nseg; s += COMB_GROUPS) F += si[(size_t)s * ROW];
         const row_t<PREC>* sj = Sj + d->Sj_off + (size_t)tri_index(R, 0) * ROW + t;
-        const unsigned char* fl = Sjf + d->Sj_off / (PB * 3) + tri_index(R, 0);
-        // the written rows, 32 units at a time (the warps of a group agree)
-        for (int b = g; b <= R; b += 32 * COMB_GROUPS) {
-            const int R2 = b + COMB_GROUPS * lane;
-            unsigned m = __ballot_sync(0xffffffffu, R2 <= R && fl[min(R2, R)] != 0);
-            while (m) {
-                double v[4];
+        if (pairs_tile_boxes<SIM, PREC, true>() && box_lo(SIM, PREC, d->fa)) {
+            const unsigned char* fl = Sjf + d->Sj_off / (PB * 3) + tri_index(R, 0);
+            // the written rows, 32 units at a time (the warps of a group agree)
+            for (int b = g; b <= R; b += 32 * COMB_GROUPS) {
+                const int R2 = b + COMB_GROUPS * lane;
+                unsigned m = __ballot_sync(0xffffffffu, R2 <= R && fl[min(R2, R)] != 0);
+                while (m) {
+                    double v[4];
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    v[u] = m ? (double)sj[(size_t)(b + COMB_GROUPS * (__ffs(m) - 1)) * ROW] : 0.0;
-                    m &= m - 1;
+                    for (int u = 0; u < 4; ++u) {
+                        v[u] = m ? (double)sj[(size_t)(b + COMB_GROUPS * (__ffs(m) - 1)) * ROW] : 0.0;
+                        m &= m - 1;
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) F += v[u];
                 }
-#pragma unroll
-                for (int u = 0; u < 4; ++u) F += v[u];
             }
+        } else {
+#pragma unroll 8
+            for (int R2 = g; R2 <= R; R2 += COMB_GROUPS) F += (double)sj[(size_t)R2 * ROW];
         }
         part[g][t] = F;
         __syncthreads();
