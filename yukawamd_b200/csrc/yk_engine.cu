@@ -80,24 +80,24 @@ __global__ void k_commit_state(const double* __restrict__ src, double* __restric
 // The same for positions, with the distance that they move (nearest image) in
 // units of 1/MOVED_UNIT of 1 / scale, at most MOVED_CAP of them, summed.
 constexpr int MOVED_UNIT = 1024, MOVED_CAP = 4;
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(64)
 k_commit_positions(const double* __restrict__ src, double* __restrict__ dst, int n, const unsigned* __restrict__ flag,
-                   double lx, double ly, double lz, double scale, unsigned long long* __restrict__ moved)
+                   float3 L, float3 iL, float scale, unsigned long long* __restrict__ moved)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     unsigned m = 0;
     if (i < n && *flag == 0) {
-        const double L[3] = {lx, ly, lz};
-        double r2 = 0.0;
+        const float Lc[3] = {L.x, L.y, L.z}, iLc[3] = {iL.x, iL.y, iL.z};
+        float r2 = 0.f;
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             const double x = src[3 * (size_t)i + c];
-            double d = x - dst[3 * (size_t)i + c];
-            d -= L[c] * rint(d / L[c]);
+            float d = (float)(x - dst[3 * (size_t)i + c]);
+            d -= Lc[c] * rintf(d * iLc[c]);
             r2 += d * d;
             dst[3 * (size_t)i + c] = x;
         }
-        m = (unsigned)(MOVED_UNIT * fmin(sqrt(r2) * scale, (double)MOVED_CAP));
+        m = (unsigned)(MOVED_UNIT * fminf(sqrtf(r2) * scale, (float)MOVED_CAP));
     }
     m = __reduce_add_sync(0xffffffffu, m);
     if ((threadIdx.x & 31) == 0 && m) atomicAdd(moved, (unsigned long long)m);
@@ -1882,9 +1882,11 @@ int yk_set_state(yk_ctx* c, const double* x, const double* v, const double* vold
     for (int q = 0; q < 4; ++q) {
         if (!src[q]) continue;
         if (q == 0)
-            k_commit_positions<<<(c->n + 255) / 256, 256, 0, c->stream>>>(
-                c->stage, c->x, c->n, c->nonfinite, c->p.xl[0], c->p.xl[1], c->p.xl[2],
-                std::cbrt(c->n / (c->p.xl[0] * c->p.xl[1] * c->p.xl[2])), moved);
+            k_commit_positions<<<(c->n + 63) / 64, 64, 0, c->stream>>>(
+                c->stage, c->x, c->n, c->nonfinite,
+                make_float3((float)c->p.xl[0], (float)c->p.xl[1], (float)c->p.xl[2]),
+                make_float3((float)(1.0 / c->p.xl[0]), (float)(1.0 / c->p.xl[1]), (float)(1.0 / c->p.xl[2])),
+                (float)std::cbrt(c->n / (c->p.xl[0] * c->p.xl[1] * c->p.xl[2])), moved);
         else
             k_commit_state<<<(int)((cnt + 255) / 256), 256, 0, c->stream>>>(c->stage + q * cnt, dst[q], cnt,
                                                                              c->nonfinite);
