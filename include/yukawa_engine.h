@@ -309,10 +309,12 @@ typedef struct yk_tuning {
     int pair_seg;         /* longest job of the half-pair kernels, in source
                              tiles (jobs shrink towards the end of the job
                              list); 0 = automatic (8 FP64, 4 mixed).  No
-                             effect on ion boxes that take the octet kernel
-                             (one target per thread; FP64, or mixed up to
-                             6,144 and from 24,576 particles), whose jobs are
-                             cut by cost on the device                      */
+                             effect on boxes that take an octet kernel
+                             (one target per thread; FP64 ions, mixed ions
+                             with r_c clear of L/2 and edges below 16,384 fm up
+                             to 6,144 and from 24,576 particles, nucleons up to
+                             4,096 in FP64 and 2,048 mixed; yk_force_kernel
+                             tells), whose jobs are cut on the device       */
     int sort_every;       /* steps between Hilbert re-orderings (-1 = never,
                              0 = automatic: 4)                              */
     int graph_steps;      /* steps per CUDA graph of yk_run: the graphs take
@@ -325,7 +327,7 @@ typedef struct yk_tuning {
                              so split x more CTAs (threads per target) work on
                              a small box: 1, 2 or 4 (jobs of one tile then);
                              0 = 1; ignored by kernels 1 and 3 and by the octet
-                             kernel (as pair_seg).  Batches: 0/1             */
+                             kernels (as pair_seg).  Batches: 0/1            */
     int targets_per_thread; /* targets each thread of the half-pair kernel
                              holds: 1, or 2 (blocks of 256 targets, every
                              source read and reaction reduction shared by two
@@ -347,10 +349,10 @@ YK_API int yk_set_tuning(yk_ctx* ctx, const yk_tuning* t);
 YK_API const char* yk_force_kernel(const yk_ctx* ctx, int automatic);
 
 /* The batch's tunables: pair_seg (most source tiles per work item; a small box
- * takes fewer, so that its longest row still makes 16 items), graph_steps (steps per CUDA graph of yk_batch_run) and sort_every (steps
- * between the boxes' Hilbert re-orderings, counted from the start of each
- * graph, which always re-sorts; 0 = automatic: 4).  force_kernel must be 0
- * or 2.  Changing pair_seg rebuilds the job table and its scratch. */
+ * takes fewer, so that its longest row still makes 16 items), graph_steps (steps
+ * per CUDA graph of yk_batch_run) and sort_every (steps between the boxes'
+ * Hilbert re-orderings, counted from the start of each graph, which always
+ * re-sorts; 0 = automatic: 4).  force_kernel must be 0 or 2.  Changing pair_seg rebuilds the job table and its scratch. */
 YK_API int yk_batch_get_tuning(yk_batch* b, yk_tuning* out);
 YK_API int yk_batch_set_tuning(yk_batch* b, const yk_tuning* t);
 

@@ -1,11 +1,13 @@
-// yk_octets.cuh -- the FP64 half-pair force kernel on octets of targets.
+// yk_octets.cuh -- the force kernels on octets of targets: half pairs
+// (k_force_octets, ions) and every pair from both sides (k_force_octets_all, small
+// boxes of ions or nucleons), their job table and combines, and the FP64 form of
+// the pairs (Form64; the mixed form is in yk_octets32.cuh).
 //
-// Units, jobs, scratch rows and the tile pipeline are those of yk_pairs.cuh
-// (target block R of 128 slots against source tiles C; a warp holds 32 of the
-// block's targets).  What differs is how a warp works through a tile.  Its 32
-// targets are four octets, 8 consecutive slots of the Hilbert order each, and
-// a lane is (a, b) = (lane & 7, lane >> 3): target a of the octet at hand and
-// every fourth source of the octet's own source list.
+// Units, scratch rows and the tile layout in slots are those of yk_pairs.cuh
+// (target block R of 128 slots against source tiles C).  What differs is how a
+// warp works through a tile: by octets, 8 consecutive slots of the Hilbert order
+// each, and a lane is (a, b) = (lane & 7, lane >> 3): target a of the octet at
+// hand and every fourth source of the octet's own source list.
 //
 //   list    per octet, the tile's sources within the screening radius of the
 //           octet's bounding box (FP32, widened as near_groups), one byte each
@@ -974,8 +976,9 @@ constexpr int OCT_COST_CTAS = 8;
 constexpr int OCT_JOBS = 3;                   // jobs per resident warp before the cuts get shorter
 
 // Cost of every window of row R (OCT_COST_CTAS CTAs, each summing its share of
-// the row): the number of (octet, source octet)
-// pairs within reach, plus 2 for a tile within reach.
+// the row): 0 in a tile out of the block's reach, else 1 and twice the number of
+// the block's octets within reach of the window's sources (so 16 a tile and twice
+// its (octet, source octet) pairs).
 static __global__ void __launch_bounds__(256)
 k_octet_cost(const float4* __restrict__ obox, const float4* __restrict__ tbox, int M, ForceArgs fa,
              unsigned char* __restrict__ cost, int* __restrict__ row_cost)
@@ -1233,14 +1236,15 @@ struct OctetAllSmem {
 
 constexpr int OCT_ALL_WARPS = 16;             // resident warps per SM
 
-// Source chunk length of k_force_octets_all for n particles, n0 at least: about
-// 48 chunks, a power of two up to a tile and then whole tiles (no tile in two
+// Source chunk length of k_force_octets_all for n particles: about 48 chunks, a
+// power of two from 16 up to a tile and then whole tiles (no tile in two
 // pieces).  Shorter chunks cost more in job overhead than they balance
 // (N = 2,000: 64 sources 34.6 us per force call, 32 38, 16 44), longer ones
-// leave the last jobs running alone (N = 12,345: 256 sources 115 us, 512 136).
-inline int octet_all_len(int n, int n0 = 16)
+// leave the last jobs running alone (seen at N = 12,345, beyond the sizes that
+// the kernel is given: 256 sources 115 us, 512 136).
+inline int octet_all_len(int n)
 {
-    int len = n0;
+    int len = 16;
     while (len < PB && 48 * len < n) len *= 2;
     if (len >= PB) len = std::max(len, (n / 48 + PB / 2) / PB * PB);
     return len;
