@@ -329,6 +329,7 @@ class SlotBatch(Batch):
         self._b = C.c_void_p()
         self.nrep = int(nslots)
         self.n = [0] * self.nrep
+        self.params = [proto]
         check_batch(self._lib.yk_batch_create_slots(C.byref(proto), self.nrep, int(max_particles),
                                                     int(max_pair_units), int(device), C.byref(self._b)))
 

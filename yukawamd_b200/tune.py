@@ -172,11 +172,14 @@ def tune(engine, candidates=None, steps=16, warmup=2, device=0, save=True):
 BATCH_SEGS = (8, 4, 16, 2, 32)
 
 
+def _batch_kind(batch, device):
+    p = batch.params[0]
+    return "r%d|%s|batch|sim%d|prec%d|nrep%d|" % (REVISION, gpu_name(device), p.sim_type, p.precision, batch.nrep)
+
+
 def batch_key(batch, device=0):
     import numpy as np
-    p = batch.params[0]
-    return "r%d|%s|batch|sim%d|prec%d|nrep%d|nb%d" % (REVISION, gpu_name(device), p.sim_type, p.precision, batch.nrep,
-                                                      bucket(int(np.sqrt(np.mean(np.square(batch.n))))))
+    return _batch_kind(batch, device) + "nb%d" % bucket(int(np.sqrt(np.mean(np.square(batch.n)))))
 
 
 def tune_batch(batch, segs=BATCH_SEGS, steps=50, device=0, save=True):
@@ -211,7 +214,15 @@ def tune_batch(batch, segs=BATCH_SEGS, steps=50, device=0, save=True):
 
 
 def apply_batch(batch, device=0):
-    ent = _load().get(batch_key(batch, device))
+    """Apply the cached choice for this batch; True if one existed.  A slot
+    batch that holds no box yet has no size: it takes the latest choice for its
+    kind and number of slots."""
+    doc = _load()
+    if any(batch.n):
+        ent = doc.get(batch_key(batch, device))
+    else:
+        kind = _batch_kind(batch, device)
+        ent = max((e for k, e in doc.items() if k.startswith(kind)), key=lambda e: e["when"], default=None)
     if not ent:
         return False
     batch.set_tuning(pair_seg=ent["pair_seg"], graph_steps=ent.get("graph_steps", 50))
